@@ -51,15 +51,18 @@ struct LikState {
     bool loaded = false;
     int64_t n = 0, n0 = 0, agents = 0;
     int epochs = 0, num_anchors = 0, words = 0, chunks = 0, ball_grid = 0, eval_grid[2] = {0, 0};
+    int wt_span = 1;           // epochs per weight table
     int64_t chunk_agents = 0;  // > 0: at most this many agents' balls per chunk (pg_tuning)
     DBuf<int64_t> epoch_nodes, fo, bo, coff, boff, bcnt, badj;
-    DBuf<int32_t> epoch_t, fc, bc, pub, anchors, cites, agent_epoch, bids;
+    DBuf<int32_t> epoch_t, fc, bc, pub, anchors, cites, agent_epoch, bids, order;
     DBuf<uint8_t> cflag;
     DBuf<float> fit;
     DBuf<float4> feat;
-    DBuf<double> theta, pp, zglob, gglob, gpart, zagent, out, res;
+    DBuf<double> theta, pp, zglob, gglob, gpart, zagent, out, res, spart;
     DBuf<uint32_t> err;
+    DBuf<float> wt;                          // weight table of a range of epochs (run_lik)
     std::vector<int64_t> hboff;              // ball offsets on the host
+    std::vector<int64_t> hnodes;             // epoch_nodes on the host
     std::vector<std::pair<int64_t, int64_t>> ball_chunks;  // agent ranges whose balls fit in bids
     bool balls_cached = false;               // one chunk: built at load, reused by every pass
     int64_t ball_elems = 0, adj_entries = 0, citations = 0;
@@ -404,15 +407,17 @@ void free_checkpoint(Checkpoint& k) {
 void free_lik(LikState& L) {
     DBuf<int64_t>* i64[] = {&L.epoch_nodes, &L.fo, &L.bo, &L.coff, &L.boff, &L.bcnt, &L.badj};
     for (auto* b : i64) dfree(*b);
-    DBuf<int32_t>* i32[] = {&L.epoch_t, &L.fc, &L.bc, &L.pub, &L.anchors, &L.cites, &L.agent_epoch, &L.bids};
+    DBuf<int32_t>* i32[] = {&L.epoch_t, &L.fc, &L.bc, &L.pub, &L.anchors, &L.cites, &L.agent_epoch, &L.bids, &L.order};
     for (auto* b : i32) dfree(*b);
-    DBuf<double>* f64[] = {&L.theta, &L.pp, &L.zglob, &L.gglob, &L.gpart, &L.zagent, &L.out, &L.res};
+    DBuf<double>* f64[] = {&L.theta, &L.pp, &L.zglob, &L.gglob, &L.gpart, &L.zagent, &L.out, &L.res, &L.spart};
     for (auto* b : f64) dfree(*b);
     dfree(L.cflag);
     dfree(L.fit);
     dfree(L.feat);
     dfree(L.err);
+    dfree(L.wt);
     L.hboff.clear();
+    L.hnodes.clear();
     L.ball_chunks.clear();
     L.balls_cached = false;
     L.loaded = false;
@@ -2431,6 +2436,9 @@ pg_status check_theta(pg_ctx* c, int32_t batch, const double* theta) {
     return PG_OK;
 }
 
+// Largest weight table of 64 points held at once, unless a single epoch needs more.
+constexpr int64_t kLikTableBytes = 1ll << 30;
+
 LikBalls make_balls(const LikState& L, int64_t a0) {
     LikBalls Bl{};
     Bl.boff = L.boff.p;
@@ -2439,7 +2447,31 @@ LikBalls make_balls(const LikState& L, int64_t a0) {
     Bl.cflag = L.cflag.p;
     Bl.cnt = L.bcnt.p;
     Bl.adj = L.badj.p;
+    Bl.order = L.balls_cached ? L.order.p : nullptr;
     return Bl;
+}
+
+// Epochs per weight table (LikBatch::wt) of rows of BE points, with the table allocated; 0: no table.
+// At 64 points a row costs its 256-byte write, about what five ball elements save (3 epochs of 200k
+// nodes, forward and adjoint, direct against table: 700 us / 883 us at 0.9 ball elements per row,
+// 762 / 965 at 1.9; at 172 per row 46.3 / 15.4 ms).  Up to 32 points the table was faster wherever
+// measured (8 points: 350 / 263 us at 0.15 elements per row, 456 / 300 at 1.9).
+int lik_table_epochs(pg_ctx* c, int BE) {
+    LikState& L = c->lik;
+    int64_t rows = 0;
+    for (int e = 0; e < L.epochs; ++e) rows += L.hnodes[(size_t)e];
+    if (BE > 32 ? L.ball_elems < 4 * rows : 8 * L.ball_elems < rows) return 0;
+    const int64_t need = L.wt_span * std::max<int64_t>(L.hnodes[(size_t)L.epochs - 1], 1) * BE;
+    if (L.wt.n < need) {
+        dfree(L.wt);
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || 4 * need > (int64_t)(free_b / 8) ||
+            dalloc(L.wt, need) != cudaSuccess) {
+            cudaGetLastError();  // no room: the direct walk
+            return 0;
+        }
+    }
+    return L.wt_span;
 }
 
 // One pass (forward or adjoint) over every group of <= 64 points; results[b * K + k].
@@ -2458,7 +2490,7 @@ pg_status run_lik(pg_ctx* c, int32_t batch, const double* theta, int adjoint, do
     const int K = adjoint ? 4 : 1;
     const int64_t zneed = (int64_t)groups * std::max<int64_t>(L.agents, 1) * kLikMaxB;
     if (L.theta.n < 4 * (int64_t)groups * kLikMaxB) PG_CUDA(c, dalloc(L.theta, 4 * (int64_t)groups * kLikMaxB));
-    if (L.pp.n < 8 * (int64_t)groups * kLikMaxB) PG_CUDA(c, dalloc(L.pp, 8 * (int64_t)groups * kLikMaxB));
+    if (L.pp.n < kLikPP * (int64_t)groups * kLikMaxB) PG_CUDA(c, dalloc(L.pp, kLikPP * (int64_t)groups * kLikMaxB));
     if (L.zagent.n < zneed) {
         if (adjoint) return fail(c, PG_ERR_STATE, "run pg_loglik_fwd first");
         PG_CUDA(c, dalloc(L.zagent, zneed));
@@ -2474,10 +2506,10 @@ pg_status run_lik(pg_ctx* c, int32_t batch, const double* theta, int adjoint, do
         PG_CUDA(c, dalloc(L.out, std::max<int64_t>(1, L.agents) * kLikMaxB * 4));
     if (L.res.n < kLikMaxB * 4) PG_CUDA(c, dalloc(L.res, kLikMaxB * 4));
     // per point: alpha, 1/tau, gamma, beta, log beta, 1/beta, 1/tau^2, tau
-    std::vector<double> pp((size_t)batch * 8);
+    std::vector<double> pp((size_t)batch * kLikPP);
     for (int b = 0; b < batch; ++b) {
         const double* t = theta + 4 * b;
-        double* q = pp.data() + 8 * b;
+        double* q = pp.data() + kLikPP * b;
         q[0] = t[0];
         q[1] = 1.0 / t[1];
         q[2] = t[2];
@@ -2486,10 +2518,21 @@ pg_status run_lik(pg_ctx* c, int32_t batch, const double* theta, int adjoint, do
         q[5] = 1.0 / t[3];
         q[6] = 1.0 / (t[1] * t[1]);
         q[7] = t[1];
+        const double al = q[0] * kLog2e, ga = q[2] * kLog2e, it = q[1] * kLog2e;
+        LikC k;
+        k.al2 = (float)al;
+        k.ga2 = (float)ga;
+        k.it2 = (float)it;
+        k.al2l = (float)(al - (double)k.al2);
+        k.ga2l = (float)(ga - (double)k.ga2);
+        k.it2l = (float)(it - (double)k.it2);
+        k.al2s = k.al2 * 0x1p-24f;
+        k.ga2s = k.ga2 * 0x1p-24f;
+        std::memcpy(q + 8, &k, sizeof(k));
     }
     PG_CUDA(c, cudaMemcpyAsync(L.theta.p, theta, sizeof(double) * 4 * (size_t)batch, cudaMemcpyHostToDevice, c->stream));
-    PG_CUDA(c, cudaMemcpyAsync(L.pp.p, pp.data(), sizeof(double) * 8 * (size_t)batch, cudaMemcpyHostToDevice, c->stream));
-    PG_CUDA(c, cudaMemsetAsync(L.err.p, 0, sizeof(uint32_t), c->stream));
+    PG_CUDA(c, cudaMemcpyAsync(L.pp.p, pp.data(), sizeof(double) * kLikPP * (size_t)batch, cudaMemcpyHostToDevice, c->stream));
+    PG_CUDA(c, cudaMemsetAsync(L.err.p, 0, 2 * sizeof(uint32_t), c->stream));
     const LikTrace T = make_trace(c);
     if (c->timing) record_event(c->lev[0], c->stream);
     std::vector<double> h((size_t)kLikMaxB * 4);
@@ -2502,19 +2545,32 @@ pg_status run_lik(pg_ctx* c, int32_t batch, const double* theta, int adjoint, do
         P.BW = std::min(P.BE, 32);
         P.exact_exp2 = adjoint ? L.fwd_exact_exp2 : L.exact_exp2;
         P.theta = L.theta.p + 4 * (int64_t)g * kLikMaxB;
-        P.pp = L.pp.p + 8 * (int64_t)g * kLikMaxB;
+        P.pp = L.pp.p + kLikPP * (int64_t)g * kLikMaxB;
         P.zglob = L.zglob.p + (int64_t)g * L.epochs * kLikMaxB;
         P.gglob = L.gglob.p;
         P.gpart = L.gpart.p;
         P.zagent = L.zagent.p + (int64_t)g * L.agents * kLikMaxB;
         P.out = L.out.p;
         P.res = L.res.p;
+        P.spart = L.spart.p;
         P.error = L.err.p;
-        launch_lik_global(T, P, adjoint, c->stream);
-        for (const auto& ch : L.ball_chunks) {
-            const LikBalls Bl = make_balls(L, ch.first);
-            if (!L.balls_cached) launch_lik_ball(T, Bl, 1, ch.first, ch.second, L.ball_grid, c->stream);
-            launch_lik_eval(T, P, Bl, adjoint, ch.first, ch.second, L.eval_grid[adjoint], c->stream);
+        const int step = lik_table_epochs(c, P.BE);
+        const int span = step > 0 ? step : L.epochs;
+        for (int e0 = 0; e0 < L.epochs; e0 += span) {
+            P.e0 = e0;
+            P.e1 = std::min(L.epochs, e0 + span);
+            P.wt = step > 0 ? L.wt.p : nullptr;
+            P.wt_n = L.hnodes[(size_t)P.e1 - 1];
+            launch_lik_global(T, P, adjoint, c->stream);
+            // the agents of these epochs, by the chunks their balls are kept in
+            const int64_t b0 = L.hnodes[(size_t)P.e0] - L.n0, b1 = L.hnodes[(size_t)P.e1] - L.n0;
+            for (const auto& ch : L.ball_chunks) {
+                const int64_t a0 = std::max(ch.first, b0), a1 = std::min(ch.second, b1);
+                if (a0 >= a1) continue;
+                const LikBalls Bl = make_balls(L, L.balls_cached ? ch.first : a0);
+                if (!L.balls_cached) launch_lik_ball(T, Bl, 1, a0, a1, L.ball_grid, c->stream);
+                launch_lik_eval(T, P, Bl, adjoint, a0, a1, L.eval_grid[adjoint], c->stream);
+            }
         }
         launch_lik_sum(T, P, adjoint, c->stream);
         PG_CUDA(c, cudaGetLastError());
@@ -2588,11 +2644,13 @@ pg_status pg_trace_load(pg_ctx* c, const pg_trace_desc* t) {
     L.agents = agents;
     L.epochs = E;
     L.num_anchors = t->num_anchors;
+    L.hnodes.assign(t->epoch_nodes, t->epoch_nodes + E + 1);
     int64_t nmax = 1;
     for (int e = 0; e < E; ++e) nmax = std::max(nmax, t->epoch_nodes[e]);
     L.words = (int)std::min<int64_t>((nmax + 31) / 32, kLikMaxWords);
     L.words = (L.words + 3) / 4 * 4;
     L.chunks = (int)((nmax + kLikChunk - 1) / kLikChunk);
+    L.wt_span = (int)std::min<int64_t>(E, std::max<int64_t>(1, kLikTableBytes / (4 * nmax * kLikMaxB)));
     pg_status s = PG_OK;
     if ((s = upload(c, L.epoch_nodes, t->epoch_nodes, (int64_t)E + 1)) != PG_OK) return s;
     if ((s = upload(c, L.epoch_t, t->epoch_t, (int64_t)E)) != PG_OK) return s;
@@ -2650,7 +2708,8 @@ pg_status pg_trace_load(pg_ctx* c, const pg_trace_desc* t) {
     if ((s = upload(c, L.anchors, t->anchors, 4 * std::max<int64_t>(agents, 1) * (agents > 0))) != PG_OK) return s;
     if ((s = upload(c, L.agent_epoch, aep.data(), agents)) != PG_OK) return s;
     PG_CUDA(c, dalloc(L.feat, (int64_t)E * n));
-    PG_CUDA(c, dalloc(L.err, 1));
+    PG_CUDA(c, dalloc(L.err, 2));
+    PG_CUDA(c, dalloc(L.spart, (int64_t)kLikSumCtas * kLikMaxB * 4));
     int ball_sm = 1, eval_sm[2] = {1, 1};
     PG_CUDA(c, init_lik_kernels(L.words, &ball_sm, eval_sm));
     L.ball_grid = c->num_sms * ball_sm;
@@ -2724,6 +2783,22 @@ pg_status pg_trace_load(pg_ctx* c, const pg_trace_desc* t) {
         chunk_max = std::max(chunk_max, L.hboff[(size_t)ch.second] - L.hboff[(size_t)ch.first]);
     PG_CUDA(c, dalloc(L.bids, chunk_max));
     L.balls_cached = L.ball_chunks.size() == 1;
+    if (L.balls_cached && agents > 0) {
+        // longest balls first (a counting sort by the ball size's bit length, stable, so that a class
+        // walks the epochs' tables once: finer classes were 4 % slower at 200k nodes and 10 epochs), over
+        // the epochs whose weight tables are held together
+        std::vector<int32_t> order((size_t)agents);
+        for (int e = 0; e < E; e += L.wt_span) {
+            const int64_t b0 = t->epoch_nodes[e] - n0, b1 = t->epoch_nodes[std::min(E, e + L.wt_span)] - n0;
+            int64_t at[66] = {};
+            auto key = [&](int64_t v) { return cnt[(size_t)v] > 0 ? __builtin_clzll((unsigned long long)cnt[(size_t)v]) : 64; };
+            for (int64_t v = b0; v < b1; ++v) ++at[key(v) + 1];
+            at[0] = b0;
+            for (int q = 1; q < 66; ++q) at[q] += at[q - 1];
+            for (int64_t v = b0; v < b1; ++v) order[(size_t)at[key(v)]++] = (int32_t)v;
+        }
+        if ((s = upload(c, L.order, order.data(), agents)) != PG_OK) return s;
+    }
     if (L.balls_cached) {
         LikBalls emit_balls = make_balls(L, 0);
         emit_balls.bmap = bmap.p;

@@ -17,8 +17,22 @@ namespace pg {
 constexpr int kLikMaxB = 64;         // parameter points per launch
 constexpr int kLikThreads = 256;
 constexpr int kLikList = 4096;       // ball ids staged in shared memory per window
-constexpr int kLikChunk = 4096;      // nodes per CTA in the per-epoch global sums
+constexpr int kLikSumCtas = 304;     // CTAs of the totals
+constexpr int kLikSumThreads = 1024;
+constexpr int kLikChunk = 1024;      // nodes per CTA in the per-epoch global sums
 constexpr int kLikMaxWords = 24576;  // ball bitmap words per pass (96 KiB, 786,432 ids)
+
+// Per-point constants of the weight exponent in base 2, each as an fp32 high part and the fp32
+// remainder of its FP64 value; al2s and ga2s scale the exact layout's packed low parts (stored
+// times 2^24) back.  Computed once per point on the host: per agent and point on the device, their
+// FP64 products and conversions were a tenth of the forward pass.
+struct LikC {
+    float al2, ga2, it2;     // alpha log2 e, gamma log2 e, log2 e / tau (high parts)
+    float al2l, ga2l, it2l;  // their remainders
+    float al2s, ga2s;        // al2 2^-24, ga2 2^-24 (exact)
+};
+constexpr int kLikPP = 12;  // doubles per point in LikBatch::pp
+static_assert(sizeof(LikC) == 32, "LikC fills the last four doubles of a point's row");
 
 struct LikTrace {
     int64_t n;                   // nodes at the end of the trace
@@ -48,14 +62,21 @@ struct LikBatch {
     int32_t BW;          // agent pass: points per warp, min(32, B) rounded up to a power of two
     int32_t exact_exp2;  // 1: weights from exp2_exact (fp32, ~2 ulp), 0: the special-function unit
     const double* theta; // [B][4] alpha, tau, gamma, beta
-    const double* pp;    // [B][8] alpha, 1/tau, gamma, beta, log beta, 1/beta, 1/tau^2, tau
+    const double* pp;    // [B][kLikPP] alpha, 1/tau, gamma, beta, log beta, 1/beta, 1/tau^2, tau, LikC
     double* zglob;       // [epochs][B]      sum_{j<n_e} w_j          (forward writes)
     double* gglob;       // [epochs][B][3]   sum_j w_j dlog w_j/dtheta (adjoint writes)
-    double* gpart;       // [epochs][chunks][B][4] partial sums of the global pass
+    double* gpart;       // [epochs][chunks][B][1|4] partial sums of the global pass
     double* zagent;      // [agents][B]      per-agent normaliser Z_a (forward writes, adjoint reads)
     double* out;         // [agents][B][1|4] per-agent log-likelihood or gradient
     double* res;         // [B][1|4]         totals
-    uint32_t* error;     // bit 2: a normaliser was not positive
+    double* spart;       // [kLikSumCtas][B * (1|4)] partial totals
+    uint32_t* error;     // [0] bit 2: a normaliser was not positive; [1] the totals' ticket (0 between launches)
+    // weight table of epochs [e0, e1): w_j at every point, row (e, j) at wt + ((e - e0) wt_n + j) BE;
+    // the global pass of the same launch writes it, the agent pass gathers from it.  Null: the agent
+    // pass evaluates every ball element's weight itself.
+    float* wt;
+    int64_t wt_n;
+    int32_t e0, e1;      // epochs of this global pass
 };
 
 // Agents' 2-hop balls, built once per trace when they fit in memory (else per chunk of agents and
@@ -71,6 +92,9 @@ struct LikBalls {
     // of walking the rows again (agent a's bitmap of pass i at bmap + a bmap_stride + i bitmap_words)
     uint32_t* bmap;
     int64_t bmap_stride;
+    // optional: each epoch's agents in descending ball size (by powers of two), the order the agent
+    // pass takes them in; null: as numbered
+    const int32_t* order;
 };
 
 size_t lik_ball_smem(int bitmap_words);

@@ -178,3 +178,47 @@ def test_ball_chunks_rebuilt_per_pass_give_identical_results(trace_mid):
         ga, gb = a.loglik_grad(pts), b.loglik_grad(pts)
     np.testing.assert_array_equal(la, lb)
     np.testing.assert_array_equal(ga, gb)
+
+
+def _check_against_oracle(trace, pts, exact=False):
+    """Log-likelihood to 1e-7, gradient to 1e-6: the bounds stated at the top of this file."""
+    with GrowthEngine(seed=1) as eng:
+        eng.set_lik_exact_exp2(exact)
+        eng.load_trace(trace)
+        ll, gr = eng.loglik(pts), eng.loglik_grad(pts)
+        balls = eng.stats()["lik_ball_elems"]
+    llo, gro = O.loglik(trace, pts)
+    assert (np.abs(ll - llo) / np.abs(llo)).max() <= 1e-7
+    assert (np.linalg.norm(gr - gro, axis=1) / np.linalg.norm(gro, axis=1)).max() <= 1e-6
+    return balls, int(trace.epoch_nodes[:-1].sum())
+
+
+@pytest.mark.parametrize("points", [1, 2, 3, 8, 9, 16, 17, 32, 33, 63, 64, 65])
+def test_weight_table_at_every_row_width(gpu, points):
+    """Balls summed from the weight table: every lane layout (points a power of two, one above, one
+    below), balls of all remainders (a 2-hop ball's size is arbitrary), agents of several epochs."""
+    g = W.plain_pa_seed(1500, 6, seed=21)
+    tr = W.grow_trace(g, W.calibration_params(), 3, seed=5)
+    balls, rows = _check_against_oracle(tr, W.theta_batch(points, seed=points), exact=points % 2 == 1)
+    assert balls >= 4 * rows  # the table is used at every batch size
+
+
+def test_weights_evaluated_in_place_for_few_balls(gpu):
+    """Few ball elements for the nodes there are: no table."""
+    g = W.plain_pa_seed(60_000, 3, seed=22)
+    prm = W.calibration_params()
+    prm.growth_rate, prm.fixed_new_nodes = 0.0, 40
+    tr = W.grow_trace(g, prm, 2, seed=6)
+    for points in (2, 40):
+        balls, rows = _check_against_oracle(tr, W.theta_batch(points, seed=points))
+        assert 8 * balls < rows
+
+
+def test_weight_table_in_several_parts(gpu):
+    """Four epochs of 1.1M nodes: the table holds three of them at a time (1 GiB at 64 points)."""
+    g = W.plain_pa_seed(1_100_000, 10, seed=23)
+    prm = W.calibration_params()
+    prm.growth_rate, prm.fixed_new_nodes = 0.0, 2500
+    tr = W.grow_trace(g, prm, 4, seed=7)
+    balls, rows = _check_against_oracle(tr, W.theta_batch(3, seed=9))
+    assert 8 * balls >= rows
