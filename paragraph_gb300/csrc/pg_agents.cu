@@ -415,40 +415,18 @@ __device__ __forceinline__ void d_agent_setup(const Arena& A, int64_t agents, in
     }
     A.indeg[slot] = 0;
     int heavy = 0;
-    if (rc && k >= 2) {
-        // a generator with many row entries, or a few long ones, makes a long 2-hop stream: such
-        // agents are listed for the CTA-wide pass (k_rc_big), mark = list slot + 1
+    if (rc) {
         double w3[3], alpha;
         int32_t gen;
         rc_agent_params(A.seed, (uint32_t)(r + A.rep_base), ep, (uint32_t)al, rp.n, rp.rc_w, rp.rc_alpha, w3,
                         &alpha, &gen);
-        const int64_t* fo = A.fwd_off + rp.obase;
-        const BRow* br = A.brow + rp.nbase;
-        int64_t gb0, gb1;
-        bspan(br, gen, gb0, gb1);
-        const int64_t gd = (fo[gen + 1] - fo[gen]) + (gb1 - gb0);
-        bool big = gd >= kRcBigGd;
-        if (!big) {
-            const int32_t* fc = A.fwd_col + rp.ebase;
-            const int32_t* bc = A.bcol + rp.bbase;
-            int64_t len = 0;
-            for (int64_t e = fo[gen]; e < fo[gen + 1]; ++e) {
-                const int32_t y = fc[e];
-                len += (fo[y + 1] - fo[y]) + blen(br, y);
-            }
-            for (int64_t e = gb0; e < gb1; ++e) {
-                const int32_t y = bc[e];
-                len += (fo[y + 1] - fo[y]) + blen(br, y);
-            }
-            big = len >= kRcBigStream;
-        }
-        if (big) {
-            const unsigned long long q = atomicAdd(&A.st->rc_big_count, 1ull);
-            if (q < (unsigned long long)kRcBigCap) {
-                A.heavy_list[q] = (int32_t)a;
-                heavy = (int)q + 1;
-            }
-        }
+        double* o = A.rc_agent + a * 6;  // the agent kernels read them back (and pg_rc_copy_agents)
+        o[0] = w3[0];
+        o[1] = w3[1];
+        o[2] = w3[2];
+        o[3] = alpha;
+        o[4] = (double)gen;
+        o[5] = (double)k;
     }
     if (!rc && A.sampler == kSamplerThinning && rp.p_global < 1.0) {
         // the anchors (the same draw the agent kernel makes): flag the hubs among them, whose
@@ -486,6 +464,54 @@ __device__ __forceinline__ void d_agent_setup(const Arena& A, int64_t agents, in
 }
 
 __global__ void __launch_bounds__(256) k_agent_setup(Arena A, int64_t agents) { d_agent_setup(A, agents, blockIdx.x); }
+
+// Refcompat, after the setup: a generator with many row entries, or a few long ones, makes a long
+// 2-hop stream; such agents are listed for the CTA-wide pass (k_rc_big), mark = list slot + 1.  One
+// warp per agent, a lane per generator row entry: the row lengths of a generator are loads that
+// depend on its row, and one thread taking them in turn was latency all through.  Setup and route of an
+// epoch of 7,000 agents: 75 us in one thread per agent, now 8 + 10 us.
+__global__ void __launch_bounds__(256) k_rc_route(Arena A, int64_t agents) {
+    if (A.st->error) return;
+    const int lane = lane_id();
+    const int64_t a = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (a >= agents || A.kk[a] < 2) return;
+    const int r = replica_of_agent(A.rep, A.R, a);
+    const Replica& rp = A.rep[r];
+    const int32_t gen = (int32_t)A.rc_agent[a * 6 + 4];
+    const int64_t* fo = A.fwd_off + rp.obase;
+    const BRow* br = A.brow + rp.nbase;
+    int64_t gb0, gb1;
+    bspan(br, gen, gb0, gb1);
+    const int64_t f0 = fo[gen], lf = fo[gen + 1] - f0, gd = lf + (gb1 - gb0);
+    int64_t len = 0;
+    for (int64_t q = lane; q < gd; q += 32) {
+        const int32_t y = q < lf ? A.fwd_col[rp.ebase + f0 + q] : A.bcol[rp.bbase + gb0 + (q - lf)];
+        len += (fo[y + 1] - fo[y]) + blen(br, y);
+    }
+    len = warp_sum(len);
+    if (lane == 0 && (gd >= kRcBigGd || len >= kRcBigStream)) {
+        const unsigned long long q = atomicAdd(&A.st->rc_big_count, 1ull);
+        if (q < (unsigned long long)kRcBigCap) {
+            A.heavy_list[q] = (int32_t)a;
+            A.heavy_mark[a] = (int)q + 1;
+            // a stream of several parts takes an item more for each; without room it stays one
+            int parts = len >= 64ll * kRcPart ? 64 : (int)((len + kRcPart - 1) / kRcPart);
+            int first = 0;
+            if (parts > 1) {
+                const unsigned long long i = atomicAdd(&A.st->rc_part_count, (unsigned long long)(parts - 1));
+                if (i + (unsigned long long)(parts - 1) <= (unsigned long long)kRcParts) {
+                    first = (int)i;
+                    for (int p = 1; p < parts; ++p) A.rc_item[i + p - 1] = make_int2((int)q, p);
+                } else {
+                    for (unsigned long long j = i; j < (unsigned long long)kRcParts && j < i + parts - 1; ++j)
+                        A.rc_item[j] = make_int2(-1, 0);  // reserved, not used
+                    parts = 1;
+                }
+            }
+            A.rc_part[q] = make_int2(parts < 1 ? 1 : parts, first);
+        }
+    }
+}
 
 // After the edge-offset scan: totals and capacity checks.
 __device__ __forceinline__ void d_edges_check(const Arena& A, int64_t agents) {
@@ -601,79 +627,59 @@ __global__ void __launch_bounds__(kAgentWarps * 32, 4) k_agents(Arena A, int64_t
     d_agents<KCAP, BIG, THIN, HS>(A, agents, agent_dsm, stride);
 }
 
-__global__ void __launch_bounds__(kAgentWarps * 32) k_agents_rc(Arena A, int64_t agents) {
+// LISTED: the agents whose 2-hop lists k_rc_big has made; else all others, which do not wait for it.
+template <bool LISTED>
+__global__ void __launch_bounds__(kAgentWarps * 32, 6) k_agents_rc(Arena A, int64_t agents) {
     __shared__ RcSmem smem[kAgentWarps];
+    __shared__ int32_t arr[kAgentWarps][kKMax];  // citations in arrival order
+    __shared__ __align__(16) int32_t set[kAgentWarps][1 << kRcSetBits];
     if (A.st->error) return;
     RcSmem& S = smem[threadIdx.x >> 5];
     const int lane = lane_id();
+    const unsigned long long listed = A.st->rc_big_count;
+    const int64_t limit = LISTED ? (int64_t)(listed < (unsigned long long)kRcBigCap ? listed : kRcBigCap) : agents;
     while (true) {
         long long q = 0;
-        if (lane == 0) q = (long long)atomicAdd(&A.st->queue_small, 1ull);
+        if (lane == 0) q = (long long)atomicAdd(LISTED ? &A.st->queue_big : &A.st->queue_small, 1ull);
         q = __shfl_sync(kFull, q, 0);
-        if (q >= agents) break;
-        process_agent_rc(A, q, A.kk[q], S);
+        if (q >= limit) break;
+        const int64_t a = LISTED ? A.heavy_list[q] : q;
+        if (!LISTED && A.heavy_mark[a] > 0) continue;
+        process_agent_rc(A, a, A.kk[a], S, arr[threadIdx.x >> 5], set[threadIdx.x >> 5]);
     }
 }
 
-// The 2-hop streams of the refcompat agents the setup listed (long streams), one CTA per
-// agent: the warps take the 32-entry chunks of every group's stream in turn, each keeping its own top
-// min(k, kKMax) of its part of the stream with the keys, validity and duplicate rule of the
-// one-warp path; the lists are merged pairwise (dropping entries that two warps both reached; the
-// k smallest distinct (key, id) pairs do not depend on the merge order) and warp 0 stores
-// the sorted ids and the stream's counters for k_agents_rc.
+// The 2-hop streams of the refcompat agents that k_rc_route listed (long streams), a CTA per work item: a
+// stream, or a part of one that is longer than kRcPart entries (the longest, alone on a CTA, was the
+// launch's tail).  Each warp keeps the top of its share; the lists are merged pairwise (dropping entries
+// that two warps both reached; the smallest distinct (key, id) pairs do not depend on the merge
+// order), an agent's last item merges its items' lists, and the sorted ids and the stream's counters
+// are stored for k_agents_rc<true>.  Bound by issue (about 165 instructions per 32 elements, half of them
+// Philox) and by instruction fetch.  200k papers, 10 epochs of 3 %: 0.60 ms an epoch in the last with
+// FP64 keys, 0.09 now.
 constexpr int kRcBigWarps = 8;
+constexpr int kRcBigSetBits = 12;  // the generator's 1-hop set: 4,096 slots
 
-__global__ void __launch_bounds__(kRcBigWarps * 32) k_rc_big(Arena A) {
+__global__ void __launch_bounds__(kRcBigWarps * 32, 3) k_rc_big(Arena A) {
     __shared__ RcSmem sm[kRcBigWarps];
+    __shared__ __align__(16) int32_t set[1 << kRcBigSetBits];
     __shared__ int s_nb[kRcBigWarps];
     __shared__ long long s_cnt[2];
     __shared__ long long s_item;
+    // the warps' smallest full-list threshold (float bits); an odd score was met; the agent's last item
+    __shared__ int s_thr, s_odd, s_last;
     if (cta_error(A)) return;
     const int warp = threadIdx.x >> 5, lane = lane_id();
     RcSmem& S = sm[warp];
     const long long listed = (long long)A.st->rc_big_count;
-    const long long total = listed < kRcBigCap ? listed : kRcBigCap;
-    while (true) {
-        if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.st->rc_big_queue, 1ull);
-        if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
+    const long long agents = listed < kRcBigCap ? listed : kRcBigCap;
+    const long long asked = (long long)A.st->rc_part_count;
+    const long long more = asked < kRcParts ? asked : kRcParts;
+    // one pairwise merge of the warps' lists, log2(warps) rounds: warp w takes warp w + h's list when
+    // w % 2h == 0; the result is warp 0's
+    auto merge = [&](int cap, int nb) {
+        if (lane == 0) s_nb[warp] = nb;
         __syncthreads();
-        const long long it = s_item;
-        if (it >= total) break;
-        const int64_t a = A.heavy_list[it];
-        const int r = replica_of_agent(A.rep, A.R, a);
-        const Replica& rp = A.rep[r];
-        const int64_t al = a - rp.abase;
-        RcCtx X;
-        X.fo = A.fwd_off + rp.obase;
-        X.fc = A.fwd_col + rp.ebase;
-        X.br = A.brow + rp.nbase;
-        X.bc = A.bcol + rp.bbase;
-        X.pa = A.rc_pa + rp.nbase;
-        X.rec = A.rc_rec + rp.nbase;
-        X.fit = A.rc_fit + rp.nbase;
-        X.seed = A.seed;
-        X.rep = (uint32_t)(r + A.rep_base);
-        X.ep = (uint32_t)A.st->epoch;
-        X.unit = (uint32_t)al;
-        double alpha;
-        rc_agent_params(A.seed, X.rep, X.ep, X.unit, rp.n, rp.rc_w, rp.rc_alpha, X.w3, &alpha, &X.gen);
-        X.gf0 = X.fo[X.gen];
-        X.glf = X.fo[X.gen + 1] - X.gf0;
-        int64_t gb1;
-        bspan(X.br, X.gen, X.gb0, gb1);
-        X.gd = X.glf + (gb1 - X.gb0);
-        const int k = A.kk[a];
-        const int kcap = k < kKMax ? k : kKMax;
-        int nb = 0;
-        long long rows = 0, elems = 0;
-        rc_2hop_slice(X, 32 * warp, 32 * kRcBigWarps, warp == 0, kcap, nb, rows, elems, S);
-        if (lane == 0) {
-            s_nb[warp] = nb;
-            atomicAdd((unsigned long long*)&s_cnt[0], (unsigned long long)rows);
-            atomicAdd((unsigned long long*)&s_cnt[1], (unsigned long long)elems);
-        }
-        __syncthreads();
-        // pairwise merges, log2(warps) rounds: warp w takes warp w + h's list when w % 2h == 0
         for (int h = 1; h < kRcBigWarps; h <<= 1) {
             if ((warp & (2 * h - 1)) == 0) {
                 const int w = warp + h;
@@ -681,28 +687,120 @@ __global__ void __launch_bounds__(kRcBigWarps * 32) k_rc_big(Arena A) {
                 for (int q0 = 0; q0 < nw; q0 += 32) {
                     const int q = q0 + lane;
                     const bool v = q < nw;
-                    rc_topk_offer(v, v ? sm[w].bk[q] : 0.0f, v ? sm[w].bi[q] : 0, kcap, nb, S);
+                    nb = rc_offer(v, v ? sm[w].bk[q] : 0.0f, v ? sm[w].bi[q] : 0, cap, nb, &S);
                 }
                 if (lane == 0) s_nb[warp] = nb;
             }
             __syncthreads();
         }
+        return nb;
+    };
+    // the whole stream's part `part` of `parts` into the warps' merged list
+    auto walk = [&](const RcCtx& X, const int32_t* H, int part, int parts, bool exact, int cap) {
+        if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
+        if (threadIdx.x == 0) {
+            s_thr = 0x7f800000;
+            s_odd = 0;
+        }
+        __syncthreads();
+        RcTop T = rc_top(cap, &s_thr);
+        long long rows = 0, elems = 0;
+        const bool odd = rc_2hop_slice(X, warp, kRcBigWarps, part, parts, exact, T, rows, elems, S, H, kRcBigSetBits);
+        if (lane == 0) {
+            atomicAdd((unsigned long long*)&s_cnt[0], (unsigned long long)rows);
+            atomicAdd((unsigned long long*)&s_cnt[1], (unsigned long long)elems);
+            if (odd) s_odd = 1;
+        }
+        return merge(cap, T.nb);
+    };
+    while (true) {
+        // the items of many-part streams first (they are the long ones), then every agent's first part
+        if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.st->rc_big_queue, 1ull);
+        __syncthreads();
+        const long long q = s_item;
+        __syncthreads();
+        if (q >= agents + more) break;
+        const int2 own = q < more ? A.rc_item[q] : make_int2((int)(q - more), 0);
+        const int slot = own.x, part = own.y;
+        if (slot < 0) continue;
+        const int2 pf = A.rc_part[slot];
+        const int64_t a = A.heavy_list[slot];
+        RcCtx X;
+        rc_ctx(A, a, X);
+        const int k = A.kk[a];
+        const int kcap = k < kKMax ? k : kKMax;
+        const int32_t* H = rc_set(X, set, kRcBigSetBits, (int)threadIdx.x, kRcBigWarps * 32, true) ? set : nullptr;
+        int nb = walk(X, H, part, pf.x, false, kcap + kRcSlack);
+        long long rows = s_cnt[0], elems = s_cnt[1];
+        bool odd = s_odd != 0;
+        if (pf.x > 1) {
+            // the item's list and counters to memory; the agent's last item merges them all
+            const int64_t it = part == 0 ? slot : kRcBigCap + pf.y + part - 1;
+            if (warp == 0) {
+                int2* l = A.rc_item_list + it * kRcItemList;
+                for (int i = lane; i < nb; i += 32) __stcg(l + i, make_int2(__float_as_int(S.bk[i]), S.bi[i]));
+                if (lane == 0) {
+                    long long* m = A.rc_item_meta + it * 4;
+                    __stcg(m + 0, (long long)nb);
+                    __stcg(m + 1, rows);
+                    __stcg(m + 2, elems);
+                    __stcg(m + 3, (long long)odd);
+                }
+                __threadfence();
+                __syncwarp();
+                if (lane == 0) s_last = atomicAdd(&A.rc_ticket[slot], 1u) == (unsigned)pf.x - 1u;
+            }
+            __syncthreads();
+            const bool last = s_last != 0;
+            __syncthreads();
+            if (!last) continue;
+            __threadfence();
+            if (threadIdx.x == 0) A.rc_ticket[slot] = 0u;
+            nb = 0;
+            rows = elems = 0;
+            odd = false;
+            for (int p = 0; p < pf.x; ++p) {
+                const int64_t ip = p == 0 ? slot : kRcBigCap + pf.y + p - 1;
+                const long long* m = A.rc_item_meta + ip * 4;
+                rows += __ldcg(m + 1);
+                elems += __ldcg(m + 2);
+                odd |= __ldcg(m + 3) != 0;
+                if (p % kRcBigWarps != warp) continue;
+                const int np = (int)__ldcg(m);
+                const int2* l = A.rc_item_list + ip * kRcItemList;
+                for (int i0 = 0; i0 < np; i0 += 32) {
+                    const bool v = i0 + lane < np;
+                    const int2 e = v ? __ldcg(l + i0 + lane) : make_int2(0, 0);
+                    nb = rc_offer(v, __int_as_float(e.x), e.y, kcap + kRcSlack, nb, &S);
+                }
+            }
+            nb = merge(kcap + kRcSlack, nb);
+        }
+        // the approximate keys first; the exact ones for the whole stream when those cannot decide
         if (warp == 0) {
-            int32_t* ids = A.rc_big_id + it * kKMax;
-            for (int q = lane; q < nb; q += 32) ids[q] = S.bi[q];
+            const bool done = !odd && rc_refine(X, kcap, nb, S);
+            if (lane == 0) s_last = done ? 1 : 0;
+        }
+        __syncthreads();
+        const bool done = s_last != 0;
+        __syncthreads();
+        if (!done) {
+            nb = walk(X, H, 0, 1, true, kcap);
+            rows = s_cnt[0];
+            elems = s_cnt[1];
+        }
+        if (warp == 0) {
+            int32_t* ids = A.rc_big_id + (int64_t)slot * kKMax;
+            for (int i = lane; i < nb; i += 32) ids[i] = S.bi[i];
             if (lane == 0) {
-                long long* meta = A.rc_big_meta + it * 3;
+                long long* meta = A.rc_big_meta + (int64_t)slot * 3;
                 meta[0] = nb;
-                meta[1] = s_cnt[0];
-                meta[2] = s_cnt[1];
+                meta[1] = rows;
+                meta[2] = elems;
             }
         }
-        __syncthreads();  // the lists and counters are reused by the next agent
+        __syncthreads();  // the lists and counters are reused by the next item
     }
-}
-
-void launch_rc_big(const Arena& A, int num_sms, cudaStream_t s) {
-    k_rc_big<<<(unsigned)num_sms * 2, kRcBigWarps * 32, 0, s>>>(A);
 }
 
 static int g_blocks_rc = 0;
@@ -710,17 +808,25 @@ static int g_blocks_rc = 0;
 cudaError_t init_rc_kernels() {
     if (g_blocks_rc) return cudaSuccess;
     const cudaError_t e =
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_rc, k_agents_rc, kAgentWarps * 32, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_rc, k_agents_rc<false>, kAgentWarps * 32, 0);
     if (g_blocks_rc < 1) g_blocks_rc = 1;
     return e;
 }
 
-void launch_rc_agents(const Arena& A, int64_t agents, int num_sms, cudaStream_t s) {
+void launch_rc_agents(const Arena& A, int64_t agents, int num_sms, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
+                      cudaEvent_t join) {
     if (agents <= 0) return;
     int64_t grid = (int64_t)num_sms * (g_blocks_rc ? g_blocks_rc : 1);
     const int64_t need = (agents + kAgentWarps - 1) / kAgentWarps;
     if (grid > need) grid = need;
-    k_agents_rc<<<(unsigned)grid, kAgentWarps * 32, 0, s>>>(A, agents);
+    // the long streams beside the other agents; then the agents that read their lists
+    cudaEventRecord(fork, s);
+    cudaStreamWaitEvent(side, fork, 0);
+    k_rc_big<<<(unsigned)num_sms * 2, kRcBigWarps * 32, 0, side>>>(A);
+    cudaEventRecord(join, side);
+    k_agents_rc<false><<<(unsigned)grid, kAgentWarps * 32, 0, s>>>(A, agents);
+    cudaStreamWaitEvent(s, join, 0);
+    k_agents_rc<true><<<(unsigned)grid, kAgentWarps * 32, 0, s>>>(A, agents);
 }
 
 static int g_blocks[2][2] = {{0, 0}, {0, 0}};  // [thin][big]
@@ -729,6 +835,9 @@ static int g_blocks_hs[2] = {0, 0};             // thinning, k <= 64, by shape (
 void launch_agent_setup(const Arena& A, int64_t agents, cudaStream_t s) {
     if (agents <= 0) return;
     k_agent_setup<<<(unsigned)((agents + 255) / 256), 256, 0, s>>>(A, agents);
+    if (A.weight_model == 1) {
+        k_rc_route<<<(unsigned)((agents + 7) / 8), 256, 0, s>>>(A, agents);
+    }
     launch_scan_i32_to_i64(A.kk, A.eoff, agents, A.blocksum, s);
     k_edges_check<<<1, 256, 0, s>>>(A, agents);
 }

@@ -123,8 +123,11 @@ struct pg_ctx {
     DBuf<int32_t> src_tmp;  // sources of an edge range being copied out
     // refcompat functor
     DBuf<double> rc_pa, rc_rec, rc_fit, rc_rtab, rc_agent;
+    DBuf<float4> rc_s32;
     DBuf<int32_t> rc_big_id;
-    DBuf<long long> rc_big_meta;
+    DBuf<long long> rc_big_meta, rc_item_meta;
+    DBuf<int2> rc_part, rc_item, rc_item_list;
+    DBuf<uint32_t> rc_ticket;
     DBuf<int32_t> rc_lag, rc_dur, rc_cnt;
     DBuf<uint64_t> rc_ftab;
     DBuf<unsigned long long> rc_acc;
@@ -322,6 +325,7 @@ Arena make_arena(pg_ctx* c) {
     A.first_wait_polls = c->first_wait_polls;
     A.weight_model = c->cfg.weight_model;
     A.rc_pa = c->rc_pa.p;
+    A.rc_s32 = c->rc_s32.p;
     A.rc_rec = c->rc_rec.p;
     A.rc_fit = c->rc_fit.p;
     A.rc_lag = c->rc_lag.p;
@@ -333,6 +337,11 @@ Arena make_arena(pg_ctx* c) {
     A.rc_agent = c->rc_agent.p;
     A.rc_big_id = c->rc_big_id.p;
     A.rc_big_meta = c->rc_big_meta.p;
+    A.rc_part = c->rc_part.p;
+    A.rc_item = c->rc_item.p;
+    A.rc_item_list = c->rc_item_list.p;
+    A.rc_item_meta = c->rc_item_meta.p;
+    A.rc_ticket = c->rc_ticket.p;
     return A;
 }
 
@@ -611,9 +620,16 @@ pg_status upload_arena(pg_ctx* c, std::vector<HostRep>& reps, const std::vector<
     PG_CUDA(c, dalloc(c->hub_cand, (int64_t)R * kHeavyMax));
     if (c->cfg.weight_model == PG_WEIGHTS_REFCOMPAT) {
         PG_CUDA(c, dalloc(c->rc_pa, S));
+        PG_CUDA(c, dalloc(c->rc_s32, S));
         if (!c->rc_big_id.p) {
             PG_CUDA(c, dalloc(c->rc_big_id, (int64_t)kRcBigCap * kKMax));
             PG_CUDA(c, dalloc(c->rc_big_meta, (int64_t)kRcBigCap * 3));
+            PG_CUDA(c, dalloc(c->rc_part, kRcBigCap));
+            PG_CUDA(c, dalloc(c->rc_item, kRcParts));
+            PG_CUDA(c, dalloc(c->rc_item_list, (int64_t)(kRcBigCap + kRcParts) * kRcItemList));
+            PG_CUDA(c, dalloc(c->rc_item_meta, (int64_t)(kRcBigCap + kRcParts) * 4));
+            PG_CUDA(c, dalloc(c->rc_ticket, kRcBigCap));
+            PG_CUDA(c, cudaMemsetAsync(c->rc_ticket.p, 0, 4 * (size_t)kRcBigCap, c->stream));
         }
         PG_CUDA(c, dalloc(c->rc_rec, S));
         PG_CUDA(c, dalloc(c->rc_fit, S));
@@ -977,14 +993,13 @@ pg_status enqueue_pa_epoch(pg_ctx* c, int64_t epoch, int64_t agents, cudaEvent_t
         launch_agent_setup(A, agents, s);
         PG_STAGE("agent setup");
         if (events) record_event(ev[2], s);
-        launch_rc_big(A, c->num_sms, s);
-        launch_rc_agents(A, agents, c->num_sms, s);
+        launch_rc_agents(A, agents, c->num_sms, s, c->side, c->fork, c->join);
         PG_STAGE("refcompat agents");
         if (events) record_event(ev[3], s);
         launch_bwd_append(A, agents, c->num_sms, s, c->side, c->fork, c->join);
         PG_STAGE("backward append");
         if (events) record_event(ev[4], s);
-        c->launches += kPaEpochKernels - 4 - 2 + kRcScoreKernels + 2 + (c->out_src ? 1 : 0);
+        c->launches += kPaEpochKernels - 4 - 2 + kRcScoreKernels + 4 + (c->out_src ? 1 : 0);
         return PG_OK;
     }
     // the hub index reads only the CSR and the weights and guide table only node attributes: the
@@ -1231,12 +1246,18 @@ void pg_destroy(pg_ctx* c) {
     dfree(c->cdf);
     dfree(c->guide);
     dfree(c->rc_pa);
+    dfree(c->rc_s32);
     dfree(c->rc_rec);
     dfree(c->rc_fit);
     dfree(c->rc_rtab);
     dfree(c->rc_agent);
     dfree(c->rc_big_id);
     dfree(c->rc_big_meta);
+    dfree(c->rc_part);
+    dfree(c->rc_item);
+    dfree(c->rc_item_list);
+    dfree(c->rc_item_meta);
+    dfree(c->rc_ticket);
     dfree(c->rc_lag);
     dfree(c->rc_dur);
     dfree(c->rc_cnt);

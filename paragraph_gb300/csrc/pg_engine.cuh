@@ -29,9 +29,16 @@ constexpr int kErChunk = 65536;      // ids per ER Philox stream
 constexpr int kSortMid = 256;        // appended segments up to this length sort in one warp's registers
 constexpr int kBitmapWords = 40960;  // 160 KiB of shared bitmap in the large-segment sort
 #define PG_MAX_ANCHORS_DEV 4
-constexpr int kRcBigGd = 32;         // refcompat generators with this many row entries: a CTA per 2-hop stream
-constexpr int kRcBigStream = 1024;  // ... or a 2-hop stream (the rows of the generator's rows) this long
+// Refcompat 2-hop streams taken by CTAs (k_rc_big): generators with this many row entries, or whose
+// rows' rows hold this many entries; and the entries of a CTA's part.  Ten epochs of a 200k-paper seed
+// at 32/1024/16384, 64/2048/8192, 96/3072/4096: 4.49, 4.03, 4.28 ms (beside k_agents_rc; shorter streams
+// cost a CTA more in merges than its warps save, longer ones leave single warps as the tail).
+constexpr int kRcBigGd = 64;
+constexpr int kRcBigStream = 2048;
 constexpr int kRcBigCap = 16384;     // such agents per epoch (the rest keep the one-warp path)
+constexpr int kRcPart = 8192;
+constexpr int kRcParts = 8192;       // items beyond one per agent that an epoch can hold
+constexpr int kRcItemList = 264;     // entries of an item's list (kKMax + kRcSlack)
 constexpr int kGBits = 13;           // per-warp global hash for anchor rows too large for shared memory
 constexpr int kZCap = 1024;          // 1-hop frontier entries kept in shared memory per warp
 constexpr int kRelocChunk = 4096;    // backward entries per copy task of a moved row
@@ -141,7 +148,8 @@ struct EpochState {
     unsigned long long queue_big;
     unsigned long long big_count;
     unsigned long long heavy_count;  // agents the small thinning kernel takes first
-    unsigned long long rc_big_count, rc_big_queue;  // refcompat agents with a CTA-wide 2-hop pass
+    // refcompat agents with a CTA-wide 2-hop pass: listed, work items beyond the first of each, queue
+    unsigned long long rc_big_count, rc_part_count, rc_big_queue;
     unsigned long long sort_small_count;
     unsigned long long sort_large_count;
     unsigned long long sort_scratch;
@@ -204,6 +212,11 @@ struct Arena {
     int32_t* zbig;             // [agent-kernel warp slots][1 << kGBits] rows of anchors too large for H
     int32_t* rc_big_id;        // [kRcBigCap][kKMax] sorted top of each listed refcompat agent's 2-hop stream
     long long* rc_big_meta;    // [kRcBigCap][3] entries, rows, elements of that stream
+    int2* rc_part;             // [kRcBigCap] parts of the stream, item number of its second part
+    int2* rc_item;             // [kRcParts] list slot and part of each item beyond the first of an agent
+    int2* rc_item_list;        // [kRcBigCap + kRcParts][kRcItemList] key bits and id: an item's list
+    long long* rc_item_meta;   // [kRcBigCap + kRcParts][4] entries, rows, elements, odd
+    unsigned int* rc_ticket;   // [kRcBigCap] items of the agent that are done (0 between epochs)
     longlong2* reloc;          // [reloc_cap] moved-row copy tasks: (source, destination << 16 | length)
     int64_t reloc_cap;
     int64_t* new_start;        // [slots] where a row's new entries of the epoch start
@@ -222,6 +235,7 @@ struct Arena {
     int32_t* hub_add;          // [R][kHeavyMax] node taking bit b this epoch, or -1
     int32_t* hub_cand;         // [R][kHeavyMax] nodes that become hubs this epoch
     // refcompat functor (null unless the context uses PG_WEIGHTS_REFCOMPAT)
+    float4* rc_s32;            // [slots] the score components in fp32 (pa, rec, fit), for the key filter
     double* rc_pa;             // [slots] score components of the epoch
     double* rc_rec;
     double* rc_fit;
@@ -439,8 +453,8 @@ void launch_bwd_append(const Arena& A, int64_t agents, int num_sms, cudaStream_t
 // refcompat functor: score components of the epoch (4 kernels) and the agent kernel
 constexpr int kRcScoreKernels = 4;
 void launch_rc_scores(const Arena& A, cudaStream_t s);
-void launch_rc_big(const Arena& A, int num_sms, cudaStream_t s);
-void launch_rc_agents(const Arena& A, int64_t agents, int num_sms, cudaStream_t s);
+void launch_rc_agents(const Arena& A, int64_t agents, int num_sms, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
+                      cudaEvent_t join);
 cudaError_t init_rc_kernels();
 // ER epoch plan: tasks are (new node, 2^16-id chunk) pairs over n existing nodes; each task owns
 // s_full slots (s_last for the last chunk), laid out per_node apart

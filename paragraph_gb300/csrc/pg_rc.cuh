@@ -111,11 +111,18 @@ PG_HD float rc_key(uint64_t seed, uint32_t rep, uint32_t ep, uint32_t unit, int3
     return (float)(E / score);
 }
 
-// Peak fitness of a new paper: inversion of the 1000-entry CDF table.
+// Peak fitness of a new paper: inversion of the 1000-entry CDF table (ascending), by bisection -- one
+// thread's scan reached hundreds of entries in most warps, 50 us of an epoch's setup.
 PG_HD int32_t rc_peak_draw(const uint64_t* table, uint64_t u) {
-    for (int i = 0; i < kRcFitMax; ++i)
-        if (u < table[i]) return i + 1;
-    return kRcFitMax;
+    int lo = 0, hi = kRcFitMax - 1;  // the first entry above u, or the last
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (u < table[mid])
+            hi = mid;
+        else
+            lo = mid + 1;
+    }
+    return lo + 1;
 }
 
 // ---- host tables

@@ -13,11 +13,16 @@
 // concatenated and split evenly over the lanes.  Keys are functions of (agent, node), so the stream
 // is never deduplicated and its order does not matter.
 
+constexpr int kRcSlack = 8;          // list entries beyond k while keys are approximate
+constexpr int kRcList = kKMax + 32;  // list capacity: kKMax + kRcSlack in whole warps
+constexpr int kRcSetBits = 8;        // a warp's set of its generator's 1-hop ids: 256 slots
+
 struct RcSmem {
-    float bk[kKMax];    // top-k keys, ascending
-    int32_t bi[kKMax];  // their ids
-    int32_t arr[kKMax]; // citations in arrival order
-    int32_t out[kKMax]; // sorted row (emit)
+    float bk[kRcList];    // top-k keys, ascending
+    int32_t bi[kRcList];  // their ids
+    int32_t out[kRcList]; // scratch
+    float qk[64];         // elements below the list's threshold, not yet offered (rc_queue)
+    int32_t qi[64];
 };
 
 __device__ __forceinline__ bool rc_in_rows(const int64_t* fo, const int32_t* fc, const BRow* br,
@@ -79,10 +84,10 @@ __device__ __forceinline__ void rc_topk_offer(bool valid, float key, int id, int
     if (!nk) return;
     const int rank = __popc(km & ((1u << lane) - 1u));
     if (keep) S.out[rank] = below;
-    float tk[kKMax / 32];
-    int ti[kKMax / 32];
+    float tk[kRcList / 32];
+    int ti[kRcList / 32];
 #pragma unroll
-    for (int j = 0; j < kKMax / 32; ++j) {
+    for (int j = 0; j < kRcList / 32; ++j) {
         const int i = lane + 32 * j;
         tk[j] = 0.0f;
         ti[j] = 0;
@@ -93,7 +98,7 @@ __device__ __forceinline__ void rc_topk_offer(bool valid, float key, int id, int
     }
     __syncwarp();  // every read of the old list (and the scratch writes) done
 #pragma unroll
-    for (int j = 0; j < kKMax / 32; ++j) {
+    for (int j = 0; j < kRcList / 32; ++j) {
         const int i = lane + 32 * j;
         if (i < nb) {
             int lo = 0, hi = nk;  // kept candidates ahead of entry i: those with below <= i
@@ -119,7 +124,53 @@ __device__ __forceinline__ void rc_topk_offer(bool valid, float key, int id, int
     nb = nb + nk < k ? nb + nk : k;
 }
 
-// What the 2-hop stream of one refcompat agent needs.
+// The same out of line, returning the new list length: the streams call it only for chunks with an
+// element below their threshold, and one copy of it keeps their loops short.
+__device__ __noinline__ int rc_offer(bool valid, float key, int id, int k, int nb, RcSmem* S) {
+    rc_topk_offer(valid, key, id, k, nb, *S);
+    return nb;
+}
+
+// A warp's list in the making: candidates below the threshold wait in a queue and are offered 32 at a
+// time, since an offer costs some 300 instructions however few of its lanes carry one.
+struct RcTop {
+    int cap, nb, nq;   // list capacity, its length, queued
+    float thr;         // nothing above it can matter
+    int* shared_thr;   // the smallest full-list threshold of the CTA's warps (float bits), or null
+};
+__device__ __forceinline__ RcTop rc_top(int cap, int* shared_thr) {
+    return RcTop{cap, 0, 0, __int_as_float(0x7f800000), shared_thr};
+}
+// offers the last min(nq, 32) queued
+__device__ __forceinline__ void rc_flush(RcTop& T, RcSmem& S) {
+    const int lane = lane_id(), n = T.nq < 32 ? T.nq : 32;
+    __syncwarp();
+    T.nq -= n;
+    const bool v = lane < n;
+    T.nb = rc_offer(v, v ? S.qk[T.nq + lane] : 0.0f, v ? S.qi[T.nq + lane] : 0, T.cap, T.nb, &S);
+    if (T.nb == T.cap) {
+        T.thr = fminf(T.thr, S.bk[T.cap - 1]);
+        if (T.shared_thr) {
+            if (lane == 0) atomicMin(T.shared_thr, __float_as_int(T.thr));
+            T.thr = fminf(T.thr, __int_as_float(*(volatile int*)T.shared_thr));
+        }
+    }
+    __syncwarp();
+}
+__device__ __forceinline__ void rc_queue(RcTop& T, bool valid, float key, int id, RcSmem& S) {
+    const bool can = valid && key <= T.thr;
+    const unsigned m = __ballot_sync(kFull, can);
+    if (!m) return;
+    if (can) {
+        const int at = T.nq + __popc(m & ((1u << lane_id()) - 1u));
+        S.qk[at] = key;
+        S.qi[at] = id;
+    }
+    T.nq += __popc(m);
+    if (T.nq >= 32) rc_flush(T, S);
+}
+
+// What the streams of one refcompat agent need.
 struct RcCtx {
     const int64_t* fo;
     const int32_t* fc;
@@ -128,22 +179,198 @@ struct RcCtx {
     const double* pa;
     const double* rec;
     const double* fit;
+    const float4* s32;
     double w3[3];
+    float w32[3];
     uint64_t seed;
     uint32_t rep, ep, unit;
     int32_t gen;
     int64_t gf0, glf, gb0, gd;  // the generator's forward row start and length, backward start, degree
 };
 
-// The 2-hop stream (N2 without N1 and g) of the generator's 1-hop groups (32 entries of N1 each):
-// every group's rows are concatenated, and the 32-entry chunks t0 = cfirst, cfirst + cstep, ... of
-// that concatenation are split over the lanes, each valid entry keyed and offered to the warp's
-// top-k list of capacity kcap.  One warp takes every chunk (cfirst 0, cstep 32); the warps of a
-// CTA take every cstep-th.  rows (when count_rows) and elems count the byte model.
-__device__ __forceinline__ void rc_2hop_slice(const RcCtx& X, int64_t cfirst, int64_t cstep, bool count_rows, int kcap,
-                                              int& nb, long long& rows, long long& elems, RcSmem& S) {
+__device__ __forceinline__ void rc_ctx(const Arena& A, int64_t a, RcCtx& X) {
+    const int r = replica_of_agent(A.rep, A.R, a);
+    const Replica& rp = A.rep[r];
+    X.fo = A.fwd_off + rp.obase;
+    X.fc = A.fwd_col + rp.ebase;
+    X.br = A.brow + rp.nbase;
+    X.bc = A.bcol + rp.bbase;
+    X.pa = A.rc_pa + rp.nbase;
+    X.rec = A.rc_rec + rp.nbase;
+    X.fit = A.rc_fit + rp.nbase;
+    X.s32 = A.rc_s32 + rp.nbase;
+    X.seed = A.seed;
+    X.rep = (uint32_t)(r + A.rep_base);
+    X.ep = (uint32_t)A.st->epoch;
+    X.unit = (uint32_t)(a - rp.abase);
+    const double* o = A.rc_agent + a * 6;  // drawn by the setup
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        X.w3[i] = o[i];
+        X.w32[i] = (float)o[i];
+    }
+    X.gen = (int32_t)o[4];
+    X.gf0 = X.fo[X.gen];
+    X.glf = X.fo[X.gen + 1] - X.gf0;
+    int64_t gb1;
+    bspan(X.br, X.gen, X.gb0, gb1);
+    X.gd = X.glf + (gb1 - X.gb0);
+}
+
+__device__ __forceinline__ double rc_score(const RcCtx& X, int32_t j) {
+    return X.w3[0] * X.pa[j] + X.w3[1] * X.rec[j] + X.w3[2] * X.fit[j];
+}
+
+// the exact key, out of line: rare, and its FP64 log is long
+__device__ __noinline__ float rc_key_exact(const RcCtx& X, int32_t j) {
+    return rc_key(X.seed, X.rep, X.ep, X.unit, j, rc_score(X, j));
+}
+
+__device__ __forceinline__ float rc_score32(const RcCtx& X, const float4 s) {
+    return __fmaf_rn(X.w32[2], s.z, __fmaf_rn(X.w32[1], s.y, X.w32[0] * s.x));
+}
+
+// ---- approximate keys.  An exact key takes an FP64 log, division and score, some hundred FP64
+// operations, and GB300 does two per clock and SM: the FP64 pipe was what the streams waited for.  Only
+// the order of the k smallest keys of a stream matters, so the stream is ranked by an fp32
+// approximation of the key whose relative error is below kRcEps, and exact keys are taken only where
+// approximations come within twice the error of one another (rc_refine).
+//
+// The error: u = ((x >> 11) + 1) 2^-53 and d = 1 - u come from the integer exactly up to their one
+// fp32 rounding (2^-23 relative with the two-part conversion).  E = -log u is d (1 + d/2 + ... + d^5/6)
+// for d < 1/16 (truncation d^6/7 < 1e-8) and -ln2 lg2.approx(u) else, where E >= 0.064: the unit's
+// absolute error 2^-22 in lg2 (relative 2^-22 below u = 1/2) is at most 4e-6 of E.  The score is a sum of three nonnegative
+// products of values rounded once (4e-7), the division adds 2 ulp.  Together below 5e-6; kRcEps is
+// 2^-16 = 1.5e-5.  Scores below 2^-100 in fp32 (a score of zero among them) are reported as odd.
+constexpr float kRcEps = 0x1p-16f;
+
+__device__ __forceinline__ float rc_key_approx(const RcCtx& X, int32_t j, float score) {
+    const u32x4 r = draw(X.seed, kStreamRcKey, X.rep, X.ep, X.unit, (uint32_t)j);
+    const uint32_t lo = r.x[0] & ~0x7FFu, nlo = ~r.x[0] & ~0x7FFu;
+    const float u = __fmaf_rn((float)r.x[1], 0x1p-32f, (float)lo * 0x1p-64f + 0x1p-53f);
+    const float d = __fmaf_rn((float)~r.x[1], 0x1p-32f, (float)nlo * 0x1p-64f);
+    float l;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(u));
+    float p = 1.0f / 6.0f;
+    p = __fmaf_rn(p, d, 1.0f / 5.0f);
+    p = __fmaf_rn(p, d, 1.0f / 4.0f);
+    p = __fmaf_rn(p, d, 1.0f / 3.0f);
+    p = __fmaf_rn(p, d, 1.0f / 2.0f);
+    p = __fmaf_rn(p, d, 1.0f);
+    const float E = d < 0.0625f ? d * p : -0x1.62e430p-1f * l;
+    return __fdividef(E, score);
+}
+
+// The generator's 1-hop set in shared memory (2^bits slots, hash_insert's table), built by `threads`
+// threads of which this is number t (a warp, or with cta = true a CTA).  False, and no set, when the
+// rows would fill more than three quarters of it: membership is then a search of the rows.  (Searching the
+// rows for the elements that a bit signature let through was what most chunks waited for: the
+// bisection's dependent loads, four chunks in turn.)
+__device__ __forceinline__ bool rc_set(const RcCtx& X, int32_t* H, int bits, int t, int threads, bool cta) {
+    if (X.gd > (3ll << bits) / 4) return false;
+    for (int q = t; q < 1 << bits; q += threads) H[q] = -1;
+    if (cta)
+        __syncthreads();
+    else
+        __syncwarp();
+    for (int64_t q = t; q < X.gd; q += threads) hash_insert(H, bits, q < X.glf ? X.fc[X.gf0 + q] : X.bc[X.gb0 + (q - X.glf)]);
+    if (cta)
+        __syncthreads();
+    else
+        __syncwarp();
+    return true;
+}
+
+// One group's share of the stream (rc_2hop_slice), positions in I (int when the group's rows hold
+// fewer than 2^30 entries).  base: this lane's row, both directions as one run;
+// ys: its start in the concatenation; this warp takes every nw-th 32-entry chunk from number `warp`.
+// Four chunks are taken together, so that their row entries, then their scores, are in flight at
+// once.  Elements of the 1-hop set H (null: search the rows) are not valid.
+template <typename I>
+__device__ __forceinline__ bool rc_group(const RcCtx& X, int warp, int nw, const int32_t* base, I ys, I tot, bool exact,
+                                         RcTop& T, long long& elems, RcSmem& S, const int32_t* H, int bits) {
+    constexpr int U = 4;
     const int lane = lane_id();
-    for (int64_t q0 = 0; q0 < X.gd; q0 += 32) {
+    bool odd = false;
+    const int32_t* rel = base - ys;
+    for (I t0 = (I)32 * warp; t0 < tot; t0 += (I)32 * nw * U) {
+        int32_t z[U];
+        bool in[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const I t = t0 + (I)32 * nw * u + lane;
+            in[u] = t < tot;
+            const I tt = in[u] ? t : tot - 1;
+            int o = 0;  // owner: the last lane whose row starts at or before tt
+#pragma unroll
+            for (int b = 16; b >= 1; b >>= 1)
+                if (__shfl_sync(kFull, ys, o + b) <= tt) o += b;
+            const int32_t* p = (const int32_t*)__shfl_sync(kFull, (unsigned long long)rel, o);
+            z[u] = p[tt];
+        }
+        float4 sc[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) sc[u] = __ldg(X.s32 + z[u]);
+        if (T.shared_thr) T.thr = fminf(T.thr, __int_as_float(*(volatile int*)T.shared_thr));
+        // one copy of the key and list code, the chunks' values moving through the first: four copies
+        // made the instruction fetch the wait that led
+#pragma unroll 1
+        for (int u = 0; u < U; ++u) {
+            bool valid = in[0] && z[0] != X.gen;
+            if (H) {
+                if (hash_contains(H, bits, z[0])) valid = false;
+            } else if (valid) {
+                valid = !rc_in_rows(X.fo, X.fc, X.br, X.bc, X.gen, z[0]);
+            }
+            float key = 0.0f;
+            if (!exact) {
+                const float s = rc_score32(X, sc[0]);
+                key = rc_key_approx(X, z[0], s);
+                odd |= in[0] && !(s > 0x1p-100f);
+            } else if (valid) {
+                key = rc_key_exact(X, z[0]);
+            }
+            elems += __popc(__ballot_sync(kFull, valid));
+            rc_queue(T, valid, key, z[0], S);
+#pragma unroll
+            for (int v = 0; v + 1 < U; ++v) {
+                z[v] = z[v + 1];
+                in[v] = in[v + 1];
+                sc[v] = sc[v + 1];
+            }
+        }
+    }
+    return odd;
+}
+
+// the same out of line with 64-bit positions: a group of 2^30 row entries or more
+__device__ __noinline__ bool rc_group_long(const RcCtx& X, int warp, int nw, const int32_t* base, int64_t ys, int64_t tot,
+                                           bool exact, RcTop* Tp, long long* elems_p, RcSmem* S, const int32_t* H,
+                                           int bits) {
+    RcTop T = *Tp;
+    long long elems = *elems_p;
+    const bool odd = rc_group<int64_t>(X, warp, nw, base, ys, tot, exact, T, elems, *S, H, bits);
+    *Tp = T;
+    *elems_p = elems;
+    return odd;
+}
+
+// The 2-hop stream (N2 without N1 and g) of the generator's 1-hop groups (32 entries of N1 each):
+// every group's rows are concatenated and split into 32-entry chunks, each valid entry keyed (approximately, or exactly) and offered to the warp's list of
+// capacity T.cap.  The stream is shared by `parts` CTAs of nw warps (or is one warp's): part and warp
+// number this one.  A stream of at least as many groups as parts is dealt out by groups, whose chunks
+// the part's warps take in turn; else all the parts' warps take the chunks in turn.  rows and elems
+// count the byte model (every row and element once over all parts and warps).  Returns whether some
+// score was too small for the approximation.
+__device__ __forceinline__ bool rc_2hop_slice(const RcCtx& X, int warp, int nw, int part, int parts, bool exact, RcTop& T,
+                                              long long& rows, long long& elems, RcSmem& S, const int32_t* H,
+                                              int bits) {
+    const bool by_group = X.gd > 32ll * (parts - 1);
+    const int w = by_group ? warp : part * nw + warp, n = by_group ? nw : parts * nw;
+    int turn = 0;  // chunks of the groups so far, modulo n
+    const int lane = lane_id();
+    bool odd = false;
+    for (int64_t q0 = by_group ? 32ll * part : 0; q0 < X.gd; q0 += by_group ? 32ll * parts : 32) {
         const int64_t q = q0 + lane;
         int32_t y = -1;
         if (q < X.gd) {
@@ -151,74 +378,99 @@ __device__ __forceinline__ void rc_2hop_slice(const RcCtx& X, int64_t cfirst, in
             if (y == X.gen) y = -1;
         }
         const int nrow = __popc(__ballot_sync(kFull, y >= 0));
-        if (count_rows) rows += nrow;
-        int64_t yf0 = 0, ylf = 0, yb0 = 0, yd = 0;
+        if (w == 0) rows += nrow;
+        // a cited paper's forward row has a copy right before its backward entries: one run; a paper
+        // never cited is its forward row
+        int64_t yd = 0;
+        const int32_t* base = X.fc;
         if (y >= 0) {
-            yf0 = X.fo[y];
-            ylf = X.fo[y + 1] - yf0;
-            int64_t yb1;
-            bspan(X.br, y, yb0, yb1);
-            yd = ylf + (yb1 - yb0);
+            const int64_t f0 = X.fo[y], lf = X.fo[y + 1] - f0;
+            int64_t b0, b1;
+            bspan(X.br, y, b0, b1);
+            yd = lf + (b1 - b0);
+            base = b1 > b0 ? X.bc + (b0 - lf) : X.fc + f0;
         }
         const int64_t incl = warp_incl_scan(yd);
-        const int64_t tot = __shfl_sync(kFull, incl, 31);
-        const int64_t ys = incl - yd;
-        for (int64_t t0 = cfirst; t0 < tot; t0 += cstep) {
-            const int64_t t = t0 + lane;
-            const int64_t tt = t < tot ? t : tot - 1;
-            int lo = 0, hi = 31;  // owner: the last lane whose rows start at or before tt
-#pragma unroll
-            for (int it = 0; it < 5; ++it) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (__shfl_sync(kFull, ys, mid) <= tt)
-                    lo = mid;
-                else
-                    hi = mid - 1;
-            }
-            const int64_t of0 = __shfl_sync(kFull, yf0, lo), olf = __shfl_sync(kFull, ylf, lo);
-            const int64_t ob0 = __shfl_sync(kFull, yb0, lo), oys = __shfl_sync(kFull, ys, lo);
-            bool valid = false;
-            int32_t z = 0;
-            float key = 0.0f;
-            if (t < tot) {
-                const int64_t x = t - oys;
-                z = x < olf ? X.fc[of0 + x] : X.bc[ob0 + (x - olf)];
-                valid = z != X.gen && !rc_in_rows(X.fo, X.fc, X.br, X.bc, X.gen, z);
-                if (valid)
-                    key = rc_key(X.seed, X.rep, X.ep, X.unit, z,
-                                 X.w3[0] * X.pa[z] + X.w3[1] * X.rec[z] + X.w3[2] * X.fit[z]);
-            }
-            elems += __popc(__ballot_sync(kFull, valid));
-            topk_offer(valid, key, z, kcap, nb, S);
+        const int64_t tot = __shfl_sync(kFull, incl, 31), ys = incl - yd;
+        const int mine = w >= turn ? w - turn : w - turn + n;
+        turn = (int)((turn + (tot + 31) / 32) % n);
+        if (tot < (1ll << 30)) {
+            odd |= rc_group<int>(X, mine, n, base, (int)ys, (int)tot, exact, T, elems, S, H, bits);
+        } else {
+            RcTop t = T;
+            long long el = elems;
+            odd |= rc_group_long(X, mine, n, base, ys, tot, exact, &t, &el, &S, H, bits);
+            T = t;
+            elems = el;
         }
     }
+    if (T.nq) rc_flush(T, S);
+    return __any_sync(kFull, odd);
 }
 
-__device__ void process_agent_rc(const Arena& A, int64_t a, int k, RcSmem& S) {
+// The exact keys of the list's n leading elements by approximate key, and the k smallest of them as the
+// new list (ascending, ties by id); returns its length.
+__device__ __noinline__ int rc_exact_list(const RcCtx& X, int k, int n, RcSmem* Sp) {
+    RcSmem& S = *Sp;
+    const int lane = lane_id();
+    for (int q = lane; q < n; q += 32) S.bk[q] = rc_key_exact(X, S.bi[q]);
+    __syncwarp();
+    // the list's arrays are reused by the offers: its entries wait in registers
+    float key[kRcList / 32];
+    int32_t id[kRcList / 32];
+#pragma unroll
+    for (int j = 0; j < kRcList / 32; ++j) {
+        const int q = lane + 32 * j;
+        key[j] = q < n ? S.bk[q] : 0.0f;
+        id[j] = q < n ? S.bi[q] : 0;
+    }
+    __syncwarp();
+    int nb = 0;
+#pragma unroll
+    for (int j = 0; j < kRcList / 32; ++j)
+        if (32 * j < n) nb = rc_offer(lane + 32 * j < n, key[j], id[j], k, nb, Sp);
+    __syncwarp();
+    return nb;
+}
+
+// The list of a stream's nb <= k + kRcSlack leading elements by approximate key becomes the list of its
+// k smallest exact keys, ascending (ties by id).  Only the order is used, so no exact key is needed while
+// neighbours up to the k-th and the one after are more than twice the error apart (all but a few in
+// a thousand lists of 15); else the whole list's are taken.  False: elements outside the list could
+// belong to it.
+__device__ __forceinline__ bool rc_refine(const RcCtx& X, int k, int& nb, RcSmem& S) {
+    const int lane = lane_id();
+    auto apart = [&](int i, int j) { return S.bk[j] * (1.0f - 2.0f * kRcEps) > S.bk[i] * (1.0f + kRcEps); };
+    bool close = false;
+    for (int i = lane; i < k && i + 1 < nb; i += 32) close |= !apart(i, i + 1);
+    if (!__any_sync(kFull, close)) {
+        nb = nb < k ? nb : k;
+        return true;
+    }
+    // with room left the list holds the whole stream; else what it lacks is at or above its last entry
+    if (nb == k + kRcSlack && !apart(k - 1, nb - 1)) return false;
+    nb = rc_exact_list(X, k, nb, &S);
+    return true;
+}
+
+__device__ void process_agent_rc(const Arena& A, int64_t a, int k, RcSmem& S, int32_t* arr, int32_t* set) {
     const int lane = lane_id();
     const unsigned below = (1u << lane) - 1u;
     const int r = replica_of_agent(A.rep, A.R, a);
     const Replica& rp = A.rep[r];
     const int64_t n = rp.n, al = a - rp.abase;
     const uint32_t ep = (uint32_t)A.st->epoch, unit = (uint32_t)al, rep = (uint32_t)(r + A.rep_base);
-    const int64_t* fo = A.fwd_off + rp.obase;
-    const int32_t* fc = A.fwd_col + rp.ebase;
-    const BRow* br = A.brow + rp.nbase;
-    const int32_t* bc = A.bcol + rp.bbase;
-    const double* pa = A.rc_pa + rp.nbase;
-    const double* rec = A.rc_rec + rp.nbase;
-    const double* fit = A.rc_fit + rp.nbase;
-    double w3[3], alpha;
-    int32_t gen;
-    rc_agent_params(A.seed, rep, ep, unit, n, rp.rc_w, rp.rc_alpha, w3, &alpha, &gen);
-    auto score = [&](int32_t j) { return w3[0] * pa[j] + w3[1] * rec[j] + w3[2] * fit[j]; };
+    RcCtx X;
+    rc_ctx(A, a, X);
+    const double alpha = A.rc_agent[a * 6 + 3];
+    const int32_t gen = X.gen;
 
     int c = 1;
-    if (lane == 0) S.arr[0] = gen;
+    if (lane == 0) arr[0] = gen;
     int32_t tgt = 0;
     const int sy = k >= 2 ? rc_same_year(A.seed, rep, ep, al, rp.delta, rp.rc_sy, n, &tgt) : 0;
     if (sy) {
-        if (lane == 0) S.arr[c] = tgt;
+        if (lane == 0) arr[c] = tgt;
         ++c;
     }
     const int rsv = (int)floor(rp.rc_frc * (double)k);
@@ -226,31 +478,40 @@ __device__ void process_agent_rc(const Arena& A, int64_t a, int k, RcSmem& S) {
     int in_t = rem1 > 0 ? (int)ceil((double)rem1 * alpha) : 0;
     if (in_t > rem1) in_t = rem1 > 0 ? rem1 : 0;
     long long rows = 1, elems = 0, draws = 0;
-    const int64_t gf0 = fo[gen], glf = fo[gen + 1] - gf0;
-    int64_t gb0, gb1;
-    bspan(br, gen, gb0, gb1);
-    const int64_t gd = glf + (gb1 - gb0);
-
     // ---- the 1-hop set
     int in = 0;
     if (in_t > 0) {
         int nb = 0;
-        for (int64_t q0 = 0; q0 < gd; q0 += 32) {
-            const int64_t q = q0 + lane;
-            bool valid = false;
-            int32_t y = 0;
-            float key = 0.0f;
-            if (q < gd) {
-                y = q < glf ? fc[gf0 + q] : bc[gb0 + (q - glf)];
-                valid = y != gen;
-                if (valid) key = rc_key(A.seed, rep, ep, unit, y, score(y));
+        long long e1 = 0;
+        for (int exact = 0; exact < 2; ++exact) {  // as the 2-hop streams: approximate keys, exact ones if they cannot decide
+            nb = 0;
+            e1 = 0;
+            bool odd = false;
+            for (int64_t q0 = 0; q0 < X.gd; q0 += 32) {
+                const int64_t q = q0 + lane;
+                bool valid = false;
+                int32_t y = 0;
+                float key = 0.0f;
+                if (q < X.gd) {
+                    y = q < X.glf ? X.fc[X.gf0 + q] : X.bc[X.gb0 + (q - X.glf)];
+                    valid = y != gen;
+                    if (exact) {
+                        if (valid) key = rc_key_exact(X, y);
+                    } else {
+                        const float sc = rc_score32(X, __ldg(X.s32 + y));
+                        key = rc_key_approx(X, y, sc);
+                        odd |= !(sc > 0x1p-100f);
+                    }
+                }
+                e1 += __popc(__ballot_sync(kFull, valid));
+                nb = rc_offer(valid, key, y, exact ? in_t : in_t + kRcSlack, nb, &S);
             }
-            elems += __popc(__ballot_sync(kFull, valid));
-            topk_offer(valid, key, y, in_t, nb, S);
+            if (exact || (!__any_sync(kFull, odd) && rc_refine(X, in_t, nb, S))) break;
         }
+        elems += e1;
         in = nb;
         __syncwarp();
-        for (int q = lane; q < in; q += 32) S.arr[c + q] = S.bi[q];
+        for (int q = lane; q < in; q += 32) arr[c + q] = S.bi[q];
         __syncwarp();
         c += in;
     }
@@ -260,26 +521,6 @@ __device__ void process_agent_rc(const Arena& A, int64_t a, int k, RcSmem& S) {
     int out = 0;
     if (rem2 > 0) {
         int nb = 0;
-        RcCtx X;
-        X.fo = fo;
-        X.fc = fc;
-        X.br = br;
-        X.bc = bc;
-        X.pa = pa;
-        X.rec = rec;
-        X.fit = fit;
-        X.w3[0] = w3[0];
-        X.w3[1] = w3[1];
-        X.w3[2] = w3[2];
-        X.seed = A.seed;
-        X.rep = rep;
-        X.ep = ep;
-        X.unit = unit;
-        X.gen = gen;
-        X.gf0 = gf0;
-        X.glf = glf;
-        X.gb0 = gb0;
-        X.gd = gd;
         const int big = A.heavy_mark[a];
         if (big > 0) {
             // listed by the setup: k_rc_big has walked the stream with a whole CTA; its sorted
@@ -292,11 +533,21 @@ __device__ void process_agent_rc(const Arena& A, int64_t a, int k, RcSmem& S) {
             elems += meta[2];
             __syncwarp();
         } else {
-            rc_2hop_slice(X, 0, 32, true, rem2, nb, rows, elems, S);
+            const int32_t* H = rc_set(X, set, kRcSetBits, lane, 32, false) ? set : nullptr;
+            long long r2 = 0, e2 = 0;
+            for (int exact = 0; exact < 2; ++exact) {  // exact keys when the approximate ones cannot decide
+                RcTop T = rc_top(exact ? rem2 : rem2 + kRcSlack, nullptr);
+                r2 = e2 = 0;
+                const bool odd = rc_2hop_slice(X, 0, 1, 0, 1, exact != 0, T, r2, e2, S, H, kRcSetBits);
+                nb = T.nb;
+                if (exact || (!odd && rc_refine(X, rem2, nb, S))) break;
+            }
+            rows += r2;
+            elems += e2;
         }
         out = nb;
         __syncwarp();
-        for (int q = lane; q < out; q += 32) S.arr[c + q] = S.bi[q];
+        for (int q = lane; q < out; q += 32) arr[c + q] = S.bi[q];
         __syncwarp();
         c += out;
     }
@@ -315,7 +566,7 @@ __device__ void process_agent_rc(const Arena& A, int64_t a, int k, RcSmem& S) {
         const uint32_t xr = (my & 3u) == 0 ? x.x[0] : ((my & 3u) == 1 ? x.x[1] : ((my & 3u) == 2 ? x.x[2] : x.x[3]));
         const int32_t v = (int32_t)bounded32(xr, (uint32_t)(n - 1));
         bool pre = false;
-        for (int q = 0; q < c; ++q) pre |= S.arr[q] == v;
+        for (int q = 0; q < c; ++q) pre |= arr[q] == v;
         const unsigned grp = __match_any_sync(kFull, v);
         const unsigned gc = grp & __ballot_sync(kFull, !pre);
         const int first = gc ? __ffs(gc) - 1 : 32;
@@ -330,21 +581,12 @@ __device__ void process_agent_rc(const Arena& A, int64_t a, int k, RcSmem& S) {
         draws += __popc(consumed);
         const unsigned took = am & consumed;
         __syncwarp();
-        if ((took >> lane) & 1u) S.arr[c + __popc(took & below)] = v;
+        if ((took >> lane) & 1u) arr[c + __popc(took & below)] = v;
         __syncwarp();
         c += __popc(took);
         rnd -= __popc(took);
         cidx += 32;
     }
     if (c != k && lane == 0) atomicOr(&A.st->error, kErrArg);
-    if (lane == 0 && A.rc_agent) {
-        double* o = A.rc_agent + a * 6;
-        o[0] = w3[0];
-        o[1] = w3[1];
-        o[2] = w3[2];
-        o[3] = alpha;
-        o[4] = (double)gen;
-        o[5] = (double)k;
-    }
-    emit_row<kKMax>(A, rp, a, al, n, S.arr, c < k ? c : k, rows, elems, draws);
+    emit_row<kKMax>(A, rp, a, al, n, arr, c < k ? c : k, rows, elems, draws);
 }

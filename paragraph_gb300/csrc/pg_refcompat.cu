@@ -123,12 +123,15 @@ __global__ void __launch_bounds__(kTileThreads) k_rc_scores(Arena A) {
         const int64_t v = v0 + threadIdx.x + i * kTileThreads;
         if (v >= rp.n) continue;
         const int64_t slot = rp.nbase + v;
-        A.rc_pa[slot] = A.rc_pa[slot] / rp.rc_dpa;
-        A.rc_fit[slot] = A.rc_fit[slot] / rp.rc_dfit;
+        const double pa = A.rc_pa[slot] / rp.rc_dpa, fit = A.rc_fit[slot] / rp.rc_dfit;
         const int64_t age = ep - A.pub[slot];
-        A.rc_rec[slot] = (age >= 0 && age < rp.rc_rec_len && rp.rc_U > 0.0)
-                             ? P[age] / ((double)cnt[age] * rp.rc_U)
-                             : 0.0;
+        const double rec = (age >= 0 && age < rp.rc_rec_len && rp.rc_U > 0.0)
+                               ? P[age] / ((double)cnt[age] * rp.rc_U)
+                               : 0.0;
+        A.rc_pa[slot] = pa;
+        A.rc_fit[slot] = fit;
+        A.rc_rec[slot] = rec;
+        A.rc_s32[slot] = make_float4((float)pa, (float)rec, (float)fit, 0.0f);
         ++act;
     }
     act = __reduce_add_sync(0xffffffffu, act);

@@ -32,6 +32,7 @@ __device__ __forceinline__ void d_epoch_begin(const Arena& A, int64_t epoch, int
         st->big_count = 0;
         st->heavy_count = 0;
         st->rc_big_count = 0;
+        st->rc_part_count = 0;
         st->rc_big_queue = 0;
         st->sort_small_count = 0;
         st->sort_large_count = 0;

@@ -157,3 +157,36 @@ def test_refcompat_needs_configuration(gpu):
             eng.grow_epoch()
         with pytest.raises(PGError):
             eng.rc_configure(RCParams(gamma=7), [10, 12], [1.0])
+
+
+@pytest.mark.parametrize("case", [
+    # 40 papers that 4,500 others cite: their own generators' rows overflow the shared set and are dealt
+    # out by groups; everyone else's stream is long rows dealt out by chunks
+    dict(hubs=40, citers=4500, w=(-1, -1, -1), bag=(2, 9, 17), rec_len=40),
+    # lists up to the largest out-degree, longer than a stream now and then
+    dict(hubs=3, citers=900, w=(0.2, 0.3, 0.5), bag=(120, 248, 250, 300), rec_len=40),
+    # scores of exactly zero (papers older than the recency table): exact keys for the whole stream
+    dict(hubs=6, citers=3000, w=(0.0, 1.0, 0.0), bag=(3, 12, 30), rec_len=3),
+])
+def test_refcompat_stream_splits_and_fallbacks_bit_exact(gpu, case):
+    n = 6000
+    base = W.rc_seed(n, 4, seed=11)
+    rng = np.random.default_rng(12)
+    hubs = rng.choice(n, case["hubs"], replace=False)
+    src = [base.src] + [rng.choice(n, case["citers"], replace=False).astype(np.int32) for _ in hubs]
+    dst = [base.dst] + [np.full(case["citers"], h, np.int32) for h in hubs]
+    g = W.SeedGraph(base.pub, base.fitness, np.concatenate(src), np.concatenate(dst))
+    rec = 0.8 ** np.arange(case["rec_len"], dtype=np.float64)
+    rc = RCParams(pa_weight=case["w"][0], rec_weight=case["w"][1], fit_weight=case["w"][2], growth_rate=0.1,
+                  same_year=0.1)
+    eng, og = _run_both(g, rc, np.array(case["bag"], np.int32), rec / rec.sum(), 2)
+    with eng:
+        for _ in range(2):
+            eng.grow_epoch()
+            og.rc_epoch()
+            np.testing.assert_array_equal(eng.arrivals(), og.arrivals())
+            np.testing.assert_array_equal(eng.rc_agents(), og.rc_agents())
+            st, so = eng.stats(), og.stats()
+            for k in ("rows_expanded", "elems_streamed", "draws"):
+                assert st[k] == so[k], k
+        _compare(eng, og)
