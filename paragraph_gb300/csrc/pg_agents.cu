@@ -1,7 +1,8 @@
 // pg_agents.cu -- per-agent citation sampling of the preferential-attachment epoch.
 //
 // Replaces kernelCallStage1/_warped/2/3/4 and the fused ABMKernel (src/kernel.cu:17-402,436-573;
-// device bodies src/abm.cu:376-565,577-994).  One warp owns one agent (new paper) and does:
+// device bodies src/abm.cu:376-565,577-994).  One warp (thinning) or one CTA (enumeration,
+// refcompat streams) owns one agent (new paper).  The enumeration sampler does:
 //   1. global race: k draws without replacement from the replica's quantised CDF.  Draw i picks the
 //      smallest j with cdf[j] - C(j) > y, where C(j) sums the weights already chosen at ids <= j;
 //      the warp searches 32-ary (32 probes per round, ballot), which gives the same j as any other
@@ -19,8 +20,6 @@
 //      cited node's in-degree counter returns the edge's rank for the backward append.
 // No per-agent O(n) state exists (the reference clears O(n) bitmaps per agent,
 // includes/abm.cuh:178-184, src/abm.cu:722-726).
-#include <type_traits>
-
 #include "pg_engine.cuh"
 #include "pg_rc.cuh"
 #include "pg_scan.cuh"
@@ -34,17 +33,6 @@ constexpr unsigned kFull = 0xffffffffu;
 __device__ __forceinline__ bool key_less(float ka, int ia, float kb, int ib) {
     return ka < kb || (ka == kb && ia < ib);
 }
-
-template <int KCAP>
-struct AgentSmem {
-    double g_t[KCAP];
-    uint64_t c_cq[KCAP];
-    int32_t g_id[KCAP];
-    int32_t c_id[KCAP];
-    float bk[KCAP];
-    int32_t bi[KCAP];
-    int32_t out[KCAP];
-};
 
 // Offer one candidate per lane to the warp's sorted top-k list (bk, bi)[0..nb) of S.
 template <typename SM>
@@ -91,32 +79,6 @@ __device__ __forceinline__ void topk_offer(bool valid, float key, int id, int k,
         }
         pass = pass && lane != leader && (nb < k || key_less(key, id, S.bk[k - 1], S.bi[k - 1]));
         mask = __ballot_sync(kFull, pass);
-    }
-}
-
-struct AgentCtx {
-    const uint64_t* cdf;
-    const float* w;
-    const int64_t* fwd_off;
-    const int32_t* fwd_col;
-    const BRow* bwd_row;
-    const int32_t* bwd_col;
-    uint64_t seed;
-    uint32_t rep, ep, unit;
-    double beta_m1;
-};
-
-__device__ __forceinline__ void boost_key(const AgentCtx& C, bool valid, int z, float& key,
-                                          bool& ok) {
-    ok = false;
-    key = 0.0f;
-    if (valid) {
-        const float wz = C.w[z];
-        if (wz > 0.0f) {
-            const u32x4 x = draw(C.seed, kStreamBoost, C.rep, C.ep, C.unit, (uint32_t)z);
-            key = -logf_pg(u01f(x.x[0])) / wz;
-            ok = true;
-        }
     }
 }
 
@@ -170,209 +132,366 @@ __device__ void emit_row(const Arena& A, const Replica& rp, int64_t a, int64_t a
     __syncwarp();
 }
 
-template <int KCAP>
-__device__ void process_agent(const Arena& A, int64_t a, int k, AgentSmem<KCAP>& S) {
+#include "pg_thin.cuh"
+#include "pg_rc_agent.cuh"
+
+// ---------------------------------------------------------------- the enumeration sampler
+// What the enumeration sampler's stream needs.
+struct EnCtx {
+    const float* w;
+    const int64_t* fo;
+    const int32_t* fc;
+    const BRow* br;
+    const int32_t* bc;
+    uint64_t seed;
+    uint32_t rep, ep, unit;
+};
+
+// E_z / w_z, E_z exponential from the Philox stream of (agent, z); valid for a positive weight
+__device__ __forceinline__ float en_key(const EnCtx& C, int32_t z, float wz) {
+    const u32x4 x = draw(C.seed, kStreamBoost, C.rep, C.ep, C.unit, (uint32_t)z);
+    return -logf_pg(u01f(x.x[0])) / wz;
+}
+
+// As rc_queue, with the keys left to the flush: an element joins the queue (with its weight) unless an
+// estimate of its key is clear of the threshold.  The estimate's E is -ln 2 lg2.approx(u), within
+// 2^-22 absolute of the logarithm for u in (1/2, 1] and 2^-22 relative below (PTX), logf_pg is within two ulp:
+// 4e-7 + 1e-5 E covers both and the threshold's product.  The logarithm and the division of
+// en_key are 50 of a chunk's 165 instructions, and few elements of a ball pass.
+__device__ __forceinline__ void en_flush(const EnCtx& C, RcTop& T, RcSmem& S) {
+    const int lane = lane_id(), at = (T.nq < 32 ? 0 : T.nq - 32) + lane;
+    __syncwarp();
+    if (at < T.nq) S.qk[at] = en_key(C, S.qi[at], S.qk[at]);
+    rc_flush(T, S);
+}
+__device__ __forceinline__ void en_queue(const EnCtx& C, RcTop& T, bool valid, int32_t z, float wz, RcSmem& S) {
+    const u32x4 x = draw(C.seed, kStreamBoost, C.rep, C.ep, C.unit, (uint32_t)z);
+    float l;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(u01f(x.x[0])));
+    const float E = -0x1.62e430p-1f * l;
+    const bool can = valid && E * (1.0f - 1e-5f) - 4e-7f <= T.thr * wz;
+    const unsigned m = __ballot_sync(kFull, can);
+    if (!m) return;
+    if (can) {
+        const int at = T.nq + __popc(m & ((1u << lane_id()) - 1u));
+        S.qk[at] = wz;
+        S.qi[at] = z;
+    }
+    T.nq += __popc(m);
+    if (T.nq >= 32) en_flush(C, T, S);
+}
+
+// The rows of up to 32 papers (this lane's: base, its entries from ys on in their concatenation of tot
+// entries), of which this warp takes every nw-th 32-entry chunk from number `warp`.  As in rc_group, four
+// chunks' entries and then weights are in flight at once, and one copy of the key code takes them in
+// turn.
+template <typename I>
+__device__ __forceinline__ void en_group(const EnCtx& C, int warp, int nw, const int32_t* base, I ys, I tot, RcTop& T,
+                                         RcSmem& S) {
+    constexpr int U = 4;
     const int lane = lane_id();
-    const int r = replica_of_agent(A.rep, A.R, a);
-    const Replica& rp = A.rep[r];
+    const int32_t* rel = base - ys;
+    for (I t0 = (I)32 * warp; t0 < tot; t0 += (I)32 * nw * U) {
+        int32_t z[U];
+        bool in[U];
+        float w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const I t = t0 + (I)32 * nw * u + lane;
+            in[u] = t < tot;
+            const I tt = in[u] ? t : tot - 1;
+            int o = 0;  // owner: the last lane whose row starts at or before tt
+#pragma unroll
+            for (int b = 16; b >= 1; b >>= 1)
+                if (__shfl_sync(kFull, ys, o + b) <= tt) o += b;
+            const int32_t* p = (const int32_t*)__shfl_sync(kFull, (unsigned long long)rel, o);
+            z[u] = p[tt];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) w[u] = C.w[z[u]];
+        T.thr = fminf(T.thr, __int_as_float(*(volatile int*)T.shared_thr));
+#pragma unroll 1
+        for (int u = 0; u < U; ++u) {
+            en_queue(C, T, in[0] && w[0] > 0.0f, z[0], w[0], S);
+#pragma unroll
+            for (int v = 0; v + 1 < U; ++v) {
+                z[v] = z[v + 1];
+                in[v] = in[v + 1];
+                w[v] = w[v + 1];
+            }
+        }
+    }
+}
+// the same with 64-bit positions, out of line: 2^30 entries or more
+__device__ __noinline__ void en_group_long(const EnCtx& C, int warp, int nw, const int32_t* base, int64_t ys, int64_t tot,
+                                           RcTop* Tp, RcSmem* S) {
+    RcTop T = *Tp;
+    en_group<int64_t>(C, warp, nw, base, ys, tot, T, *S);
+    *Tp = T;
+}
+
+// Shared memory of one agent: the warps' lists, and the global race.
+struct EnSmem {
+    RcSmem top[kAgentWarps];
+    double g_t[kKMax];
+    uint64_t c_cq[kKMax];   // chosen so far, by id: their cumulative weight
+    uint64_t c_cdf[kKMax];  // and their CDF entries
+    int32_t g_id[kKMax];
+    int32_t out[kKMax];
+    int nb[kAgentWarps];
+    int thr;
+    long long item;
+};
+
+// The global race, one warp: k draws without replacement from the quantised CDF (g_id, g_t); their number.
+// The draws depend on one another only through the integer weights left (R): the exponentials are
+// taken 32 at a time, one per lane, before the searches and divided by their R after them, so no FP64
+// operation but the k additions of t is in the chain (GB300 does two FP64 operations per clock and SM;
+// a log and a division per draw, in turn, were two thirds of an agent).
+__device__ __forceinline__ int en_race(const Arena& A, const Replica& rp, const EnCtx& C, int k, EnSmem& S) {
+    const int lane = lane_id();
     const int64_t n = rp.n;
-    const int64_t al = a - rp.abase;
-    AgentCtx C;
-    C.cdf = A.cdf + rp.nbase;
-    C.w = A.w + rp.nbase;
-    C.fwd_off = A.fwd_off + rp.obase;
-    C.fwd_col = A.fwd_col + rp.ebase;
-    C.bwd_row = A.brow + rp.nbase;
-    C.bwd_col = A.bcol + rp.bbase;
-    C.seed = A.seed;
-    C.rep = (uint32_t)(r + A.rep_base);
-    C.ep = (uint32_t)A.st->epoch;
-    C.unit = (uint32_t)al;
-    C.beta_m1 = rp.beta_m1;
+    const uint64_t* cdf = A.cdf + rp.nbase;
     const int s = cdf_shift(bitsf(rp.wmax_bits), n);
     const double scale = bitsd((uint64_t)(1023 - s) << 52);
-
-    // ---------------------------------------------------------------- 1. global race
     uint64_t R = rp.wq_total;
     double t = 0.0;
     int nc = 0;
+    uint64_t own_r = 0;  // R before this lane's draw
+    double own_e = 0.0;
+    uint64_t own_u = 0;
+    // the first round of every search probes the same 32 places
+    int64_t p0 = n > 32 ? (int64_t)(lane + 1) * ((n + 31) / 32) - 1 : lane;
+    if (p0 > n - 1) p0 = n - 1;
+    const uint64_t cdf0 = cdf[p0];
+    // the times of draws i0 .. i0 + cnt - 1
+    auto times = [&](int i0, int cnt) {
+        const double dt = own_e / ((double)own_r * scale);
+        for (int q = 0; q < cnt; ++q) {
+            t = t + __shfl_sync(kFull, dt, q);
+            if (lane == q) S.g_t[i0 + q] = t;
+        }
+    };
     for (int i = 0; i < k; ++i) {
         if (R == 0) break;
-        const u32x4 x = draw(C.seed, kStreamGlobal, C.rep, C.ep, C.unit, (uint32_t)i);
-        const double E = -log_pg(u01d(x.x[0], x.x[1]));
-        t = t + E / ((double)R * scale);
-        const uint64_t y = mulhi64(u64of(x.x[2], x.x[3]), R);
-        // 32-ary search for the smallest j in [0, n) with F(j) = cdf[j] - C(j) > y
+        if ((i & 31) == 0) {
+            if (i) times(i - 32, 32);
+            const u32x4 x = draw(C.seed, kStreamGlobal, C.rep, C.ep, C.unit, (uint32_t)(i + lane));
+            own_e = -log_pg(u01d(x.x[0], x.x[1]));
+            own_u = u64of(x.x[2], x.x[3]);
+        }
+        if (lane == (i & 31)) own_r = R;
+        const uint64_t y = mulhi64(__shfl_sync(kFull, own_u, i & 31), R);
+        // The answer is the smallest j with cdf[j] - C(j) > y, C(j) the weight chosen at ids <= j.  A chosen
+        // c leaves an empty interval at cdf[c] - C(c); those at or below y are the chosen ids below j, and
+        // y plus their weight is a place of the plain CDF.
+        int m = 0;
+        for (int q0 = 0; q0 < nc; q0 += 32) {
+            const int q = q0 + lane;
+            m += __popc(__ballot_sync(kFull, q < nc && S.c_cdf[q] - S.c_cq[q] <= y));
+        }
+        const uint64_t chosen = m ? S.c_cq[m - 1] : 0, at = y + chosen;
+        // 32-ary search of the CDF
         int64_t lo = 0, hi = n;
         while (true) {
             const int64_t span = hi - lo;
             const int64_t step = span > 32 ? (span + 31) / 32 : 1;
             int64_t p = lo + (int64_t)(lane + 1) * step - 1;
             if (p > hi - 1) p = hi - 1;
-            // C(p): chosen weight at ids <= p
-            int cl = 0, ch = nc;
-            while (cl < ch) {
-                const int mid = (cl + ch) >> 1;
-                if (S.c_id[mid] <= p)
-                    cl = mid + 1;
-                else
-                    ch = mid;
-            }
-            const uint64_t cp = cl ? S.c_cq[cl - 1] : 0;
-            const bool pred = (C.cdf[p] - cp) > y;
-            const unsigned m = __ballot_sync(kFull, pred);
-            if (m == 0) {  // F(hi-1) > y is an invariant; report instead of probing out of range
+            const unsigned b = __ballot_sync(kFull, (lo == 0 && hi == n ? cdf0 : cdf[p]) > at);
+            if (b == 0) {  // cdf[hi-1] > at is an invariant; report instead of probing out of range
                 if (lane == 0) atomicOr(&A.st->error, kErrArg);
                 lo = 0;
                 break;
             }
-            const int L = __ffs(m) - 1;  // lane probing hi-1 is always true
-            const int64_t pL = __shfl_sync(kFull, p, L);
-            const int64_t pL1 = __shfl_sync(kFull, p, L > 0 ? L - 1 : 0);
+            const int L = __ffs(b) - 1;  // the first lane at or past the answer
+            const int64_t pL = lo + (int64_t)(L + 1) * step - 1 < hi ? lo + (int64_t)(L + 1) * step - 1 : hi - 1;
             if (span <= 32) {
                 lo = pL;
                 break;
             }
             hi = pL + 1;
-            lo = L > 0 ? pL1 + 1 : lo;
+            if (L > 0) lo += (int64_t)L * step;
         }
         const int j = (int)lo;
-        const uint64_t qj = C.cdf[j] - (j > 0 ? C.cdf[j - 1] : 0);
-        // insert j into the sorted chosen list
-        int below = 0;
-        for (int q = lane; q < nc; q += 32) below += S.c_id[q] < j ? 1 : 0;
-        const int pos = __reduce_add_sync(kFull, below);
-        for (int top = nc; top > pos; top -= 32) {
+        const uint64_t cj = cdf[j], qj = cj - (j > 0 ? cdf[j - 1] : 0);
+        // j into the sorted chosen list, at m
+        for (int top = nc; top > m; top -= 32) {
             const int q = top - 1 - lane;
-            const bool act = q >= pos;
-            int tid = 0;
-            uint64_t tq = 0;
+            const bool act = q >= m;
+            uint64_t tc = 0, tq = 0;
             if (act) {
-                tid = S.c_id[q];
+                tc = S.c_cdf[q];
                 tq = S.c_cq[q];
             }
             __syncwarp();
             if (act) {
-                S.c_id[q + 1] = tid;
+                S.c_cdf[q + 1] = tc;
                 S.c_cq[q + 1] = tq + qj;
             }
             __syncwarp();
         }
         if (lane == 0) {
-            S.c_id[pos] = j;
-            S.c_cq[pos] = (pos > 0 ? S.c_cq[pos - 1] : 0) + qj;
+            S.c_cdf[m] = cj;
+            S.c_cq[m] = chosen + qj;
             S.g_id[i] = j;
-            S.g_t[i] = t;
         }
         __syncwarp();
         ++nc;
         R -= qj;
     }
-    const int ng = nc;
-
-    // ---------------------------------------------------------------- 2. neighbourhood race
-    int nb = 0;
-    long long rows = 0, elems = 0;
-    if (C.beta_m1 > 0.0) {
-        const int na = rp.anchors;
-        const u32x4 xa = draw(C.seed, kStreamAnchor, C.rep, C.ep, C.unit, 0);
-        uint32_t xr = xa.x[0];
-        if (lane == 1) xr = xa.x[1];
-        if (lane == 2) xr = xa.x[2];
-        if (lane == 3) xr = xa.x[3];
-        const int anchor = (int)bounded32(xr, (uint32_t)n);
-        {
-            float key;
-            bool ok;
-            boost_key(C, lane < na, anchor, key, ok);
-            topk_offer(ok, key, anchor, k, nb, S);
-        }
-        rows += na;
-        elems += na;
-        for (int ai = 0; ai < na; ++ai) {
-            const int x = __shfl_sync(kFull, anchor, ai);
-            const int64_t fb = C.fwd_off[x], fe = C.fwd_off[x + 1];
-            int64_t bb, be;
-            bspan(C.bwd_row, x, bb, be);
-            const int64_t lf = fe - fb;
-            const int64_t deg1 = lf + (be - bb);
-            rows += deg1;
-            elems += deg1;
-            for (int64_t base = 0; base < deg1; base += 32) {
-                const int64_t idx = base + lane;
-                const bool valid = idx < deg1;
-                int y = 0;
-                if (valid) y = idx < lf ? C.fwd_col[fb + idx] : C.bwd_col[bb + idx - lf];
-                {
-                    float key;
-                    bool ok;
-                    boost_key(C, valid, y, key, ok);
-                    topk_offer(ok, key, y, k, nb, S);
-                }
-                int64_t yf = 0, yb = 0, ylf = 0, ylen = 0;
-                if (valid) {
-                    yf = C.fwd_off[y];
-                    ylf = C.fwd_off[y + 1] - yf;
-                    int64_t ye;
-                    bspan(C.bwd_row, y, yb, ye);
-                    ylen = ylf + (ye - yb);
-                }
-                const int64_t incl = warp_incl_scan<int64_t>(ylen);
-                const int64_t total = __shfl_sync(kFull, incl, 31);
-                elems += total;
-                for (int64_t pb = 0; pb < total; pb += 32) {
-                    const int64_t p = pb + lane;
-                    const bool v2 = p < total;
-                    int o = 0;
-#pragma unroll
-                    for (int b = 16; b >= 1; b >>= 1) {
-                        const int64_t iv = __shfl_sync(kFull, incl, o + b - 1);
-                        if (iv <= p) o += b;
-                    }
-                    const int64_t ex_o = __shfl_sync(kFull, incl - ylen, o);
-                    const int64_t yf_o = __shfl_sync(kFull, yf, o);
-                    const int64_t ylf_o = __shfl_sync(kFull, ylf, o);
-                    const int64_t yb_o = __shfl_sync(kFull, yb, o);
-                    int z = 0;
-                    if (v2) {
-                        const int64_t within = p - ex_o;
-                        z = within < ylf_o ? C.fwd_col[yf_o + within]
-                                           : C.bwd_col[yb_o + within - ylf_o];
-                    }
-                    float key;
-                    bool ok;
-                    boost_key(C, v2, z, key, ok);
-                    topk_offer(ok, key, z, k, nb, S);
-                }
-            }
-        }
-    }
-
-    // ---------------------------------------------------------------- 3. merge and emit
-    int taken = 0, gi = 0, bj = 0;
-    while (taken < k && (gi < ng || bj < nb)) {
-        const double tb = bj < nb ? (double)S.bk[bj] / C.beta_m1 : 0.0;
-        const bool take_g =
-            bj >= nb || (gi < ng && (S.g_t[gi] < tb || (S.g_t[gi] == tb && S.g_id[gi] <= S.bi[bj])));
-        const int id = take_g ? S.g_id[gi] : S.bi[bj];
-        if (take_g)
-            ++gi;
-        else
-            ++bj;
-        bool dup = false;
-        for (int q = lane; q < taken; q += 32) dup |= (S.out[q] == id);
-        if (!__any_sync(kFull, dup)) {
-            if (lane == 0) S.out[taken] = id;
-            __syncwarp();
-            ++taken;
-        }
-    }
-    if (taken != k && lane == 0) atomicOr(&A.st->error, kErrArg);
-    emit_row<KCAP>(A, rp, a, al, n, S.out, taken, rows, elems, ng);
+    if (nc) times((nc - 1) & ~31, ((nc - 1) & 31) + 1);
+    __syncwarp();
+    return nc;
 }
 
-#include "pg_thin.cuh"
-#include "pg_rc_agent.cuh"
+// One CTA per agent: warp 0 draws the global race, the other warps stream the 2-hop ball, each keeping
+// the k smallest keys of its chunks; the lists are merged and warp 0 merges the two races and emits.
+// What bounds it is latency: the race is k dependent searches, and a ball's elements are two dependent
+// loads, a Philox block and a logarithm each.  One warp per agent took both in turn and balls differ a
+// hundredfold: 30k nodes, 1,500 agents an epoch, 383 us an epoch; now 150 (4, 5, 8 CTAs per SM: 200,
+// 161, 164).
+__global__ void __launch_bounds__(kAgentWarps * 32, 6) k_agents_enum(Arena A, int64_t agents) {
+    __shared__ EnSmem S;
+    if (cta_error(A)) return;
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    while (true) {
+        if (threadIdx.x == 0) {
+            S.item = (long long)atomicAdd(&A.st->queue_small, 1ull);
+            S.thr = 0x7f800000;
+        }
+        __syncthreads();
+        const int64_t a = S.item;
+        if (a >= agents) break;
+        const int k = A.kk[a];
+        const int r = replica_of_agent(A.rep, A.R, a);
+        const Replica& rp = A.rep[r];
+        const int64_t n = rp.n, al = a - rp.abase;
+        EnCtx C;
+        C.w = A.w + rp.nbase;
+        C.fo = A.fwd_off + rp.obase;
+        C.fc = A.fwd_col + rp.ebase;
+        C.br = A.brow + rp.nbase;
+        C.bc = A.bcol + rp.bbase;
+        C.seed = A.seed;
+        C.rep = (uint32_t)(r + A.rep_base);
+        C.ep = (uint32_t)A.st->epoch;
+        C.unit = (uint32_t)al;
+        RcTop T = rc_top(k, &S.thr);
+        RcSmem& L = S.top[warp];
+        long long rows = 0, elems = 0;
+        int ng = 0;
+        if (warp == 0) {
+            ng = en_race(A, rp, C, k, S);
+        }
+        if (rp.beta_m1 > 0.0) {
+            const int na = rp.anchors;
+            const u32x4 xa = draw(C.seed, kStreamAnchor, C.rep, C.ep, C.unit, 0);
+            const uint32_t xr = lane == 0 ? xa.x[0] : (lane == 1 ? xa.x[1] : (lane == 2 ? xa.x[2] : xa.x[3]));
+            const int anchor = (int)bounded32(xr, (uint32_t)n);
+            rows += na;
+            elems += na;
+            // the chunks of all groups are dealt to the streaming warps in turn (warp 0 only counts)
+            constexpr int kS = kAgentWarps - 1;
+            const int me = warp - 1;
+            int turn = 0;
+            auto my_turn = [&]() { return me >= 0 && turn == me; };
+            if (my_turn()) {
+                const float wz = lane < na ? C.w[anchor] : 0.0f;
+                en_queue(C, T, wz > 0.0f, anchor, wz, L);
+            }
+            turn = (turn + 1) % kS;
+            for (int ai = 0; ai < na; ++ai) {
+                const int x = __shfl_sync(kFull, anchor, ai);
+                const int64_t fb = C.fo[x], lf = C.fo[x + 1] - fb;
+                int64_t bb, be;
+                bspan(C.br, x, bb, be);
+                const int64_t deg1 = lf + (be - bb);
+                rows += deg1;
+                elems += deg1;
+                for (int64_t g0 = 0; g0 < deg1; g0 += 32) {
+                    const int64_t idx = g0 + lane;
+                    const bool valid = idx < deg1;
+                    const int y = valid ? (idx < lf ? C.fc[fb + idx] : C.bc[bb + idx - lf]) : 0;
+                    if (my_turn()) {
+                        const float wy = valid ? C.w[y] : 0.0f;
+                        en_queue(C, T, wy > 0.0f, y, wy, L);
+                    }
+                    turn = (turn + 1) % kS;
+                    // a cited paper's forward row has a copy right before its backward entries: one run
+                    int64_t yd = 0;
+                    const int32_t* base = C.fc;
+                    if (valid) {
+                        const int64_t yf = C.fo[y], ylf = C.fo[y + 1] - yf;
+                        int64_t yb, ye;
+                        bspan(C.br, y, yb, ye);
+                        yd = ylf + (ye - yb);
+                        base = ye > yb ? C.bc + (yb - ylf) : C.fc + yf;
+                    }
+                    const int64_t incl = warp_incl_scan<int64_t>(yd);
+                    const int64_t tot = __shfl_sync(kFull, incl, 31);
+                    elems += tot;
+                    if (me >= 0) {
+                        const int mine = me >= turn ? me - turn : me - turn + kS;
+                        if (tot < (1ll << 30)) {
+                            en_group<int>(C, mine, kS, base, (int)(incl - yd), (int)tot, T, L);
+                        } else {
+                            RcTop t = T;
+                            en_group_long(C, mine, kS, base, incl - yd, tot, &t, &L);
+                            T = t;
+                        }
+                    }
+                    turn = (int)((turn + (tot + 31) / 32) % kS);
+                }
+            }
+            if (T.nq) en_flush(C, T, L);
+        }
+        if (lane == 0) S.nb[warp] = T.nb;
+        __syncthreads();
+        // warp 0's list is empty: it takes warp 1's part of the merges
+        for (int h = 1; h < kAgentWarps; h <<= 1) {
+            if ((warp & (2 * h - 1)) == 0) {
+                const int w = warp + h, nw = S.nb[w];
+                for (int q0 = 0; q0 < nw; q0 += 32) {
+                    const int q = q0 + lane;
+                    const bool v = q < nw;
+                    T.nb = rc_offer(v, v ? S.top[w].bk[q] : 0.0f, v ? S.top[w].bi[q] : 0, k, T.nb, &L);
+                }
+                if (lane == 0) S.nb[warp] = T.nb;
+            }
+            __syncthreads();
+        }
+        if (warp == 0) {
+            // the first k distinct nodes of the two races by (time, id)
+            int taken = 0, gi = 0, bj = 0;
+            const int nb = T.nb;
+            double* b_t = reinterpret_cast<double*>(S.c_cq);  // the race is done with its list
+            for (int q = lane; q < nb; q += 32) b_t[q] = (double)L.bk[q] / rp.beta_m1;
+            __syncwarp();
+            while (taken < k && (gi < ng || bj < nb)) {
+                const double tb = bj < nb ? b_t[bj] : 0.0;
+                const bool take_g =
+                    bj >= nb || (gi < ng && (S.g_t[gi] < tb || (S.g_t[gi] == tb && S.g_id[gi] <= L.bi[bj])));
+                const int id = take_g ? S.g_id[gi] : L.bi[bj];
+                if (take_g)
+                    ++gi;
+                else
+                    ++bj;
+                bool dup = false;
+                for (int q = lane; q < taken; q += 32) dup |= (S.out[q] == id);
+                if (!__any_sync(kFull, dup)) {
+                    if (lane == 0) S.out[taken] = id;
+                    __syncwarp();
+                    ++taken;
+                }
+            }
+            if (taken != k && lane == 0) atomicOr(&A.st->error, kErrArg);
+            emit_row<kKMax>(A, rp, a, al, n, S.out, taken, rows, elems, ng);
+        }
+        __syncthreads();  // the shared memory is the next agent's
+    }
+}
+
 
 // ---------------------------------------------------------------- setup: out-degree + new nodes
 __device__ __forceinline__ void d_agent_setup(const Arena& A, int64_t agents, int vb) {
@@ -549,39 +668,27 @@ __host__ __device__ constexpr size_t thin_smem_bytes() {
     return sizeof(ThinSmem<KCAP, ThinHash<KCAP, HS>::value, ThinStage<KCAP, HS>::value>) * kAgentWarps;
 }
 
-// The agent loop of one warp.  Thinning variants: the warp's shared memory is dsm + warp * stride
-// (the calling kernel's dynamic shared memory; stride >= sizeof of this variant's ThinSmem); the
-// enumeration variants use static shared memory.
-template <int KCAP, bool BIG, bool THIN, int HS = 0>
+// The agent loop of one warp of the thinning sampler.  The warp's shared memory is dsm + warp * stride
+// (the calling kernel's dynamic shared memory; stride >= sizeof of this variant's ThinSmem).
+template <int KCAP, bool BIG, int HS = 0>
 __device__ __forceinline__ void d_agents(const Arena& A, int64_t agents, unsigned char* dsm, size_t stride) {
     constexpr int HCAP = ThinHash<KCAP, HS>::value;
     constexpr int STAGE = ThinStage<KCAP, HS>::value;
-    using Smem = typename std::conditional<THIN, ThinSmem<KCAP, HCAP, STAGE>, AgentSmem<KCAP>>::type;
-    Smem* sp;
-    if constexpr (THIN) {
-        sp = reinterpret_cast<Smem*>(dsm + (threadIdx.x >> 5) * stride);
-    } else {
-        __shared__ Smem agent_ssm[kAgentWarps];
-        sp = &agent_ssm[threadIdx.x >> 5];
-        (void)dsm;
-        (void)stride;
-    }
+    using Smem = ThinSmem<KCAP, HCAP, STAGE>;
+    Smem& S = *reinterpret_cast<Smem*>(dsm + (threadIdx.x >> 5) * stride);
     if (A.st->error) return;
-    Smem& S = *sp;
     const int lane = lane_id();
     // the small thinning kernel walks the heavy list, then every agent not on it
-    constexpr bool kHeavyFirst = THIN && !BIG;
+    constexpr bool kHeavyFirst = !BIG;
     const int64_t hc = kHeavyFirst ? (int64_t)A.st->heavy_count : 0;
     const int64_t limit = BIG ? (int64_t)A.st->big_count : agents + hc;
     uint32_t phase = 0;
-    if constexpr (THIN) {
-        if (lane == 0) {
-            mbar_init(&S.bar[0], 1);
-            mbar_init(&S.bar[1], 1);
-        }
-        fence_proxy_async();
-        __syncwarp();
+    if (lane == 0) {
+        mbar_init(&S.bar[0], 1);
+        mbar_init(&S.bar[1], 1);
     }
+    fence_proxy_async();
+    __syncwarp();
     while (true) {
         long long q = 0;
         if (lane == 0)
@@ -601,30 +708,25 @@ __device__ __forceinline__ void d_agents(const Arena& A, int64_t agents, unsigne
         }
         const int k = A.kk[a];
         if (!BIG && k > KCAP) continue;
-        if constexpr (THIN) {
-            const bool ok = general ? process_agent_thin<KCAP, HCAP, STAGE, true>(A, a, k, S, phase)
-                                    : process_agent_thin<KCAP, HCAP, STAGE, false>(A, a, k, S, phase);
-            if (!ok) break;
-        } else
-            process_agent<KCAP>(A, a, k, S);
+        const bool ok = general ? process_agent_thin<KCAP, HCAP, STAGE, true>(A, a, k, S, phase)
+                                : process_agent_thin<KCAP, HCAP, STAGE, false>(A, a, k, S, phase);
+        if (!ok) break;
     }
-    if constexpr (THIN) {
-        // every copy this warp issued has been waited for: the barriers' memory can be reused
-        __syncwarp();
-        if (lane == 0) {
-            mbar_inval(&S.bar[0]);
-            mbar_inval(&S.bar[1]);
-        }
-        __syncwarp();
+    // every copy this warp issued has been waited for: the barriers' memory can be reused
+    __syncwarp();
+    if (lane == 0) {
+        mbar_inval(&S.bar[0]);
+        mbar_inval(&S.bar[1]);
     }
+    __syncwarp();
 }
 
-template <int KCAP, bool BIG, bool THIN, int HS = 0>
+template <int KCAP, bool BIG, int HS = 0>
 __global__ void __launch_bounds__(kAgentWarps * 32, 4) k_agents(Arena A, int64_t agents) {
-    // the thinning variants hold two stage buffers per warp and go past 48 KiB: dynamic
+    // two stage buffers per warp go past 48 KiB: dynamic
     extern __shared__ __align__(16) unsigned char agent_dsm[];
     constexpr size_t stride = thin_smem_bytes<KCAP, HS>() / kAgentWarps;
-    d_agents<KCAP, BIG, THIN, HS>(A, agents, agent_dsm, stride);
+    d_agents<KCAP, BIG, HS>(A, agents, agent_dsm, stride);
 }
 
 // LISTED: the agents whose 2-hop lists k_rc_big has made; else all others, which do not wait for it.
@@ -829,7 +931,7 @@ void launch_rc_agents(const Arena& A, int64_t agents, int num_sms, cudaStream_t 
     k_agents_rc<true><<<(unsigned)grid, kAgentWarps * 32, 0, s>>>(A, agents);
 }
 
-static int g_blocks[2][2] = {{0, 0}, {0, 0}};  // [thin][big]
+static int g_blocks_enum = 0, g_blocks_big = 0;  // enumeration; thinning, k > 64
 static int g_blocks_hs[2] = {0, 0};             // thinning, k <= 64, by shape (small_hash)
 
 void launch_agent_setup(const Arena& A, int64_t agents, cudaStream_t s) {
@@ -844,41 +946,37 @@ void launch_agent_setup(const Arena& A, int64_t agents, cudaStream_t s) {
 
 // Occupancy of the persistent agent kernels; called once per process before any capture.
 cudaError_t init_agent_kernels() {
-    if (g_blocks[0][0]) return cudaSuccess;
+    if (g_blocks_enum) return cudaSuccess;
     cudaError_t e = cudaSuccess;
     const int th = kAgentWarps * 32;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks[0][0], k_agents<kKSmall, false, false>, th, 0);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks[0][1], k_agents<kKMax, true, false>, th, 0);
+    int en = 0;
     constexpr size_t d0 = thin_smem_bytes<kKSmall, 0>(), d1 = thin_smem_bytes<kKSmall, 1>(),
                      db = thin_smem_bytes<kKMax, 0>();
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_agents<kKSmall, false, true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d0);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_agents<kKSmall, false, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_agents<kKMax, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)db);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_hs[0], k_agents<kKSmall, false, true, 0>, th, d0);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_hs[1], k_agents<kKSmall, false, true, 1>, th, d1);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks[1][1], k_agents<kKMax, true, true>, th, db);
-    g_blocks[1][0] = g_blocks_hs[0];
-    for (auto& row : g_blocks)
-        for (int& b : row)
-            if (b < 1) b = 1;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_agents<kKSmall, false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d0);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_agents<kKSmall, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_agents<kKMax, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)db);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_hs[0], k_agents<kKSmall, false, 0>, th, d0);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_hs[1], k_agents<kKSmall, false, 1>, th, d1);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_big, k_agents<kKMax, true>, th, db);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&en, k_agents_enum, th, 0);
+    if (g_blocks_big < 1) g_blocks_big = 1;
     for (int& b : g_blocks_hs)
         if (b < 1) b = 1;
+    g_blocks_enum = en < 1 ? 1 : en;
     return e;
 }
 
-// Warps of the agent kernels that can be resident at once (the rows of the global anchor table).
+// Warps of the thinning kernels that can be resident at once (the rows of the global anchor table).
 int64_t agent_warp_slots(int num_sms) {
-    int mb = 1;
+    int mb = g_blocks_big;
     for (int b : g_blocks_hs) mb = b > mb ? b : mb;
-    for (auto& row : g_blocks)
-        for (int b : row) mb = b > mb ? b : mb;
     const int64_t sep = (int64_t)num_sms * mb * kAgentWarps;
     const int64_t per = (int64_t)(2 * num_sms) * 8;  // the epoch kernel: 2 CTAs of 8 warps per SM at most
     return sep > per ? sep : per;
 }
 
 int agent_occupancy(int thin, int small_hash) {
-    if (!thin) return g_blocks[0][0];
+    if (!thin) return g_blocks_enum;
     return g_blocks_hs[small_hash == 1 ? 1 : 0];
 }
 
@@ -888,21 +986,19 @@ void launch_agents(const Arena& A, int64_t agents, int num_sms, cudaStream_t s) 
     const int hs = t && A.tune_small_hash == 1 ? 1 : 0;
     int per_sm = agent_occupancy(t, hs);
     if (A.tune_agent_ctas > 0 && A.tune_agent_ctas < per_sm) per_sm = A.tune_agent_ctas;
-    int64_t need = (agents + kAgentWarps - 1) / kAgentWarps;
+    const int64_t need = t ? (agents + kAgentWarps - 1) / kAgentWarps : agents;
     int64_t grid = (int64_t)num_sms * per_sm;
     if (grid > need) grid = need;
-    const unsigned gbig = (unsigned)num_sms * g_blocks[t][1];
     const int th = kAgentWarps * 32;
-    if (t) {
-        if (hs == 1)
-            k_agents<kKSmall, false, true, 1><<<(unsigned)grid, th, thin_smem_bytes<kKSmall, 1>(), s>>>(A, agents);
-        else
-            k_agents<kKSmall, false, true, 0><<<(unsigned)grid, th, thin_smem_bytes<kKSmall, 0>(), s>>>(A, agents);
-        k_agents<kKMax, true, true><<<gbig, th, thin_smem_bytes<kKMax, 0>(), s>>>(A, agents);
-    } else {
-        k_agents<kKSmall, false, false><<<(unsigned)grid, th, 0, s>>>(A, agents);
-        k_agents<kKMax, true, false><<<gbig, th, 0, s>>>(A, agents);
+    if (!t) {
+        k_agents_enum<<<(unsigned)grid, th, 0, s>>>(A, agents);
+        return;
     }
+    if (hs == 1)
+        k_agents<kKSmall, false, 1><<<(unsigned)grid, th, thin_smem_bytes<kKSmall, 1>(), s>>>(A, agents);
+    else
+        k_agents<kKSmall, false, 0><<<(unsigned)grid, th, thin_smem_bytes<kKSmall, 0>(), s>>>(A, agents);
+    k_agents<kKMax, true><<<(unsigned)(num_sms * g_blocks_big), th, thin_smem_bytes<kKMax, 0>(), s>>>(A, agents);
 }
 
 
@@ -1016,8 +1112,8 @@ __global__ void __launch_bounds__(kEpochThreads, 2) k_epoch(Arena A, int64_t epo
     }
     grid_sync(A);
     // the agents: k <= 256 queue, then the k <= 64 queue (heavy list first)
-    d_agents<kKMax, true, true>(A, agents, ep_dsm, kEpochWarpSmem);
-    d_agents<kKSmall, false, true, 1>(A, agents, ep_dsm, kEpochWarpSmem);
+    d_agents<kKMax, true>(A, agents, ep_dsm, kEpochWarpSmem);
+    d_agents<kKSmall, false, 1>(A, agents, ep_dsm, kEpochWarpSmem);
     grid_sync(A);
     // backward append: the cited rows' new lengths, new spans for the rows that outgrew theirs
     d_bwd_grow(A, agents);

@@ -1036,7 +1036,7 @@ pg_status enqueue_pa_epoch(pg_ctx* c, int64_t epoch, int64_t agents, cudaEvent_t
     PG_STAGE("backward append");
     if (events) record_event(ev[4], s);
 #undef PG_STAGE
-    c->launches += kPaEpochKernels + (c->out_src ? 1 : 0);
+    c->launches += kPaEpochKernels - (thin ? 0 : 1) + (c->out_src ? 1 : 0);
     return PG_OK;
 }
 

@@ -582,3 +582,28 @@ def test_run_er_epochs_matches_single_epochs(gpu, p):
     for x, y in zip(last1, last2):
         np.testing.assert_array_equal(x, y)
     np.testing.assert_array_equal(ind1, ind2)
+
+
+@pytest.mark.parametrize("n0,delta,lam,beta,anchors,alpha", [
+    (3001, 37, 31.0, 4.0, 4, 1.0),    # out-degrees on both sides of 32 and 64
+    (5003, 21, 190.0, 2.5, 1, 1.0),   # lists of up to 256, one anchor
+    (2000, 40, 100.0, 500.0, 3, 0.0),  # the ball's race leads everywhere
+    (257, 300, 200.0, 1.5, 3, 2.0),   # nearly every node is taken: the race without replacement to its end
+])
+def test_enumeration_lists_and_race_bit_exact(gpu, n0, delta, lam, beta, anchors, alpha):
+    """The enumeration sampler over list lengths from one warp's width to the largest, on a graph whose
+    popular nodes put rows of hundreds of entries into the balls."""
+    g = _popular_seed(n0, 12, 100, 240, seed=5)
+    prm = PAParams(alpha=alpha, tau=5.0, gamma=1.0, beta=beta, mean_out_degree=lam, growth_rate=0.0,
+                   fixed_new_nodes=delta, num_anchors=anchors)
+    with GrowthEngine(seed=99, record_trace=True, sampler=PG_SAMPLER_ENUMERATE) as eng:
+        eng.load_graph(g.pub, g.fitness, g.src, g.dst, prm, planned_epochs=2)
+        og = _oracle_for(g, prm, 99, sampler=PG_SAMPLER_ENUMERATE)
+        for _ in range(2):
+            eng.grow_epoch()
+            og.pa_epoch()
+            np.testing.assert_array_equal(eng.arrivals(), og.arrivals())
+            st, so = eng.stats(), og.stats()
+            for k in ("rows_expanded", "elems_streamed", "draws"):
+                assert st[k] == so[k], k
+            _compare_state(eng, og)
