@@ -940,7 +940,7 @@ void launch_agent_setup(const Arena& A, int64_t agents, cudaStream_t s) {
     if (A.weight_model == 1) {
         k_rc_route<<<(unsigned)((agents + 7) / 8), 256, 0, s>>>(A, agents);
     }
-    launch_scan_i32_to_i64(A.kk, A.eoff, agents, A.blocksum, s);
+    scan_impl<int32_t>(A.kk, A.eoff, agents, A.blocksum, s, false);
     k_edges_check<<<1, 256, 0, s>>>(A, agents);
 }
 
@@ -1049,7 +1049,7 @@ constexpr size_t kEpochSmem = kEpochWarps * kEpochWarpSmem;
 __global__ void __launch_bounds__(kEpochThreads, 2) k_epoch(Arena A, int64_t epoch, int64_t agents, int G) {
     extern __shared__ __align__(16) unsigned char ep_dsm[];
     const int T = A.ntiles;
-    const int hub_items = A.R * kHeavyMax * G;
+    const int hub_items = A.R * G;
     // epoch start: new-node counts and agent offsets
     if (blockIdx.x == 0) d_epoch_begin(A, epoch, -1);
     grid_sync(A);
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(kEpochThreads, 2) k_epoch(Arena A, int64_t epo
     }
     grid_sync(A);
     // hub threshold; tile-local CDF scans
-    if (blockIdx.x == 0) d_hub_pick(A);
+    for (int r = blockIdx.x; r < A.R; r += gridDim.x) d_hub_pick(A, r);
     for (int t = blockIdx.x; t < T; t += gridDim.x) {
         d_cdf_tiles(A, t);
         __syncthreads();
@@ -1073,7 +1073,7 @@ __global__ void __launch_bounds__(kEpochThreads, 2) k_epoch(Arena A, int64_t epo
     if (blockIdx.x == gridDim.x - 1) d_tile_scan(A);
     grid_sync(A);
     // hub bits; CDF offsets and guide marks
-    if (blockIdx.x == 0) d_hub_assign(A);
+    d_hub_assign(A);
     for (int t = blockIdx.x; t < T; t += gridDim.x) {
         d_cdf_add(A, t);
         __syncthreads();
@@ -1156,7 +1156,7 @@ int epoch_kernel_ctas() { return g_epoch_ctas > 0 ? g_epoch_ctas : 0; }
 cudaError_t launch_epoch_kernel(const Arena& A, int64_t epoch, int64_t agents, cudaStream_t s) {
     if (g_epoch_ctas <= 0) return cudaErrorNotSupported;
     Arena a = A;
-    int G = A.R >= 64 ? 1 : 64 / A.R;
+    int G = hub_ctas(A.R, g_epoch_ctas / 2);
     void* args[] = {&a, &epoch, &agents, &G};
     return cudaLaunchCooperativeKernel((const void*)k_epoch, dim3((unsigned)g_epoch_ctas), dim3(kEpochThreads), args,
                                        kEpochSmem, s);

@@ -1025,7 +1025,7 @@ pg_status enqueue_pa_epoch(pg_ctx* c, int64_t epoch, int64_t agents, cudaEvent_t
     launch_agent_setup(A, agents, s);
     PG_STAGE("agent setup");
     if (c->cfg.sampler == PG_SAMPLER_THINNING) {
-        launch_hub_pairs(A, s);  // for the hubs the setup found among the anchors
+        launch_hub_pairs(A, c->num_sms, s);  // for the hubs the setup found among the anchors
         PG_STAGE("hub pairs");
     }
     if (events) record_event(ev[2], s);

@@ -437,7 +437,7 @@ void launch_epoch_begin(const Arena& A, int64_t epoch, int pa_mode, cudaStream_t
 void launch_epoch_begin_delta(const Arena& A, int64_t epoch, int64_t delta, cudaStream_t s);
 void launch_weights(const Arena& A, cudaStream_t s);
 void launch_hubs(const Arena& A, int num_sms, cudaStream_t s);
-void launch_hub_pairs(const Arena& A, cudaStream_t s);
+void launch_hub_pairs(const Arena& A, int num_sms, cudaStream_t s);
 void launch_guide(const Arena& A, cudaStream_t s);
 void launch_agent_setup(const Arena& A, int64_t agents, cudaStream_t s);
 void launch_agents(const Arena& A, int64_t agents, int num_sms, cudaStream_t s);

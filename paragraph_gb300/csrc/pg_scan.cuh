@@ -2,7 +2,9 @@
 // pg_agents.cu).
 //
 // Reduce-then-scan in three steps (tile sums, one CTA scans the sums, tiles rescan with their
-// offset), as three launches or as three phases of the persistent epoch kernel.  Integer sums are
+// offset), as three launches or as three phases of the persistent epoch kernel; up to kScanDirect
+// tiles the middle step goes, each tile adding up the sums before its own (a few loads per thread
+// against a launch of its own, 3 us), and a single tile needs no sums at all.  Integer sums are
 // exact, so the result does not depend on the tile decomposition.
 #pragma once
 #include "pg_engine.cuh"
@@ -12,6 +14,7 @@ namespace pg {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 4;
 constexpr int kScanBlock = kScanThreads * kScanItems;
+constexpr int kScanDirect = 1024;  // tiles, four sums per thread
 
 int scan_blocks_needed(int64_t n) { return (int)((n + kScanBlock - 1) / kScanBlock); }
 
@@ -99,14 +102,51 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const TIn* __restri
     d_scan_apply<TIn>(in, n, blocksum, nb, out, blockIdx.x);
 }
 
+// The apply step from the tiles' own sums.
 template <typename TIn>
-static void scan_impl(const TIn* in, int64_t* out, int64_t n, int64_t* blocksum, cudaStream_t s) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_direct(const TIn* __restrict__ in, int64_t n,
+                                                              const int64_t* __restrict__ sums, int nb,
+                                                              int64_t* __restrict__ out) {
+    __shared__ int64_t sw[33];
+    const int vb = blockIdx.x;
+    int64_t before = 0;
+    for (int i = threadIdx.x; i < vb; i += kScanThreads) before += sums[i];
+    int64_t prefix;
+    block_excl_scan<int64_t>(before, sw, &prefix);
+    __syncthreads();
+    const int64_t base = (int64_t)vb * kScanBlock + (int64_t)threadIdx.x * kScanItems;
+    int64_t v[kScanItems];
+    int64_t s = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+        const int64_t idx = base + i;
+        v[i] = idx < n ? (int64_t)in[idx] : 0;
+        s += v[i];
+    }
+    int64_t tot;
+    int64_t ex = block_excl_scan<int64_t>(s, sw, &tot) + prefix;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+        const int64_t idx = base + i;
+        if (idx < n) out[idx] = ex;
+        ex += v[i];
+    }
+    if (vb == nb - 1 && threadIdx.x == 0) out[n] = prefix + tot;
+}
+
+template <typename TIn>
+static void scan_impl(const TIn* in, int64_t* out, int64_t n, int64_t* blocksum, cudaStream_t s, bool direct = true) {
     if (n <= 0) {
         cudaMemsetAsync(out, 0, sizeof(int64_t), s);
         return;
     }
     const int nb = scan_blocks_needed(n);
-    k_scan_reduce<TIn><<<nb, kScanThreads, 0, s>>>(in, n, blocksum);
+    direct = direct && nb <= kScanDirect;
+    if (nb > 1 || !direct) k_scan_reduce<TIn><<<nb, kScanThreads, 0, s>>>(in, n, blocksum);
+    if (direct) {
+        k_scan_direct<TIn><<<nb, kScanThreads, 0, s>>>(in, n, blocksum, nb, out);
+        return;
+    }
     k_scan_blocksums<<<1, 1024, 0, s>>>(blocksum, nb);
     k_scan_apply<TIn><<<nb, kScanThreads, 0, s>>>(in, n, blocksum, nb, out);
 }

@@ -380,9 +380,11 @@ __device__ __forceinline__ void d_hub_hist(const Arena& A, int vb) {
 
 __global__ void __launch_bounds__(kTileThreads) k_hub_hist(Arena A) { d_hub_hist(A, blockIdx.x); }
 
-__device__ __forceinline__ void d_hub_pick(const Arena& A) {
+// Threshold and cleared lists of replica r (one CTA of kHeavyMax threads or more).
+__device__ __forceinline__ void d_hub_pick(const Arena& A, int r) {
     if (cta_error(A)) return;
-    for (int r = threadIdx.x; r < A.R; r += blockDim.x) {
+    __shared__ int full;
+    if (threadIdx.x == 0) {
         Replica& rp = A.rep[r];
         int thr = 0x7fffffff, cum = 0;
         for (int b = kHeavyBins - 1; b >= 0; --b) {
@@ -392,22 +394,26 @@ __device__ __forceinline__ void d_hub_pick(const Arena& A) {
         }
         rp.heavy_thr = thr;
         rp.hub_nadd = 0;
-        rp.hub_full = !rp.hub_valid;
+        full = !rp.hub_valid;
+        rp.hub_full = full;
         rp.hub_valid = 1;
     }
     __syncthreads();
-    for (int64_t i = threadIdx.x; i < (int64_t)A.R * kHeavyMax; i += blockDim.x) {
+    const int64_t i = (int64_t)r * kHeavyMax + threadIdx.x;
+    if (threadIdx.x < kHeavyMax) {
         A.hub_rem[i] = -1;
         A.hub_add[i] = -1;
-        if (A.rep[i / kHeavyMax].hub_full) A.hlist[i] = -1;
+        if (full) A.hlist[i] = -1;
+        // hub-pair masks are OR-accumulated by k_hub_pairs, for the hubs the agent setup flags
+#pragma unroll
+        for (int w = 0; w < kMaskWords; ++w) A.hub2[i * kMaskWords + w] = 0;
+        if (threadIdx.x < kHeavyMax / 32) A.hub_need[(int64_t)r * (kHeavyMax / 32) + threadIdx.x] = 0u;
     }
-    // hub-pair masks are OR-accumulated by k_hub_pairs, for the hubs the agent setup flags
-    const int64_t words = (int64_t)A.R * kHeavyMax * kMaskWords;
-    for (int64_t i = threadIdx.x; i < words; i += blockDim.x) A.hub2[i] = 0;
-    for (int64_t i = threadIdx.x; i < (int64_t)A.R * (kHeavyMax / 32); i += blockDim.x) A.hub_need[i] = 0u;
+    __syncthreads();  // `full` is rewritten for the CTA's next replica
 }
 
-__global__ void k_hub_pick(Arena A) { d_hub_pick(A); }
+// one CTA per replica: one for all of them took 98 us for the 256 of an ensemble
+__global__ void __launch_bounds__(kHeavyMax) k_hub_pick(Arena A) { d_hub_pick(A, blockIdx.x); }
 
 // Nodes leaving the hub set give up their bit (hub_rem), nodes joining it are listed (hub_cand).
 __device__ __forceinline__ void d_hub_collect(const Arena& A, int vb) {
@@ -450,7 +456,7 @@ __global__ void __launch_bounds__(kTileThreads) k_hub_collect(Arena A) { d_hub_c
 __device__ __forceinline__ void d_hub_assign(const Arena& A) {
     if (A.st->error) return;
     const int lane = lane_id();
-    for (int r = threadIdx.x >> 5; r < A.R; r += blockDim.x >> 5) {
+    for (int r = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < A.R; r += (int)((gridDim.x * blockDim.x) >> 5)) {
         Replica& rp = A.rep[r];
         int32_t* hl = A.hlist + (int64_t)r * kHeavyMax;
         const int32_t* rem = A.hub_rem + (int64_t)r * kHeavyMax;
@@ -498,107 +504,130 @@ __device__ __forceinline__ void d_hub_assign(const Arena& A) {
 
 __global__ void __launch_bounds__(256) k_hub_assign(Arena A) { d_hub_assign(A); }
 
-// G CTAs per (replica, hub bit) split a hub's neighbours.  SET = false: the node that left bit b
-// clears it on its neighbours; SET = true: the node that took bit b sets it (the clears of an epoch
-// all finish before its sets, so a bit freed and taken again in one epoch ends up right).
+// The replica's bits that `want` names, listed in shared memory by a CTA of at least kHeavyMax threads;
+// their number.
+template <typename F>
+__device__ __forceinline__ int hub_list(int* list, int* count, F want) {
+    if (threadIdx.x == 0) *count = 0;
+    __syncthreads();
+    if (threadIdx.x < kHeavyMax && want((int)threadIdx.x)) list[atomicAdd(count, 1)] = (int)threadIdx.x;
+    __syncthreads();
+    return *count;
+}
+
+// The G CTAs of replica r (this is number g) split the neighbours of the hubs that changed.
+// SET = false: the node that left bit b clears it on its neighbours; SET = true: the node that took bit
+// b sets it (the clears of an epoch all finish before its sets, so a bit freed and taken again in one
+// epoch ends up right).  Most epochs change a few hubs or none: a CTA per hub and part, launched to
+// find nothing, was 10 us.
 template <bool SET>
 __device__ __forceinline__ void d_hub_mask(const Arena& A, int G, int vb) {
-    if (A.st->error) return;
-    const int item = vb / G, g = vb % G;
-    const int r = item / kHeavyMax, b = item % kHeavyMax;
-    if (r >= A.R) return;
+    __shared__ int list[kHeavyMax], count;
+    if (cta_error(A)) return;
+    const int r = vb / G, g = vb % G;
+    const int32_t* changed = (SET ? A.hub_add : A.hub_rem) + (int64_t)r * kHeavyMax;
+    const int cnt = hub_list(list, &count, [&](int b) { return changed[b] >= 0; });
     const Replica& rp = A.rep[r];
-    const int64_t h = (SET ? A.hub_add : A.hub_rem)[(int64_t)r * kHeavyMax + b];
-    if (h < 0) return;
-    const unsigned long long bit = 1ull << (b & 63);
     const int64_t stride = (int64_t)G * blockDim.x;
-    for (int dir = 0; dir < 2; ++dir) {
-        int64_t p0, p1;
-        const int32_t* col;
-        if (dir) {
-            bspan(A.brow + rp.nbase, h, p0, p1);
-            col = A.bcol + rp.bbase;
-        } else {
-            p0 = A.fwd_off[rp.obase + h];
-            p1 = A.fwd_off[rp.obase + h + 1];
-            col = A.fwd_col + rp.ebase;
-        }
-        for (int64_t p = p0 + (int64_t)g * blockDim.x + threadIdx.x; p < p1; p += stride) {
-            unsigned long long* w = (unsigned long long*)&A.hmask[(rp.nbase + col[p]) * kMaskWords + (b >> 6)];
-            if (SET)
-                atomicOr(w, bit);
-            else
-                atomicAnd(w, ~bit);
+    for (int i = 0; i < cnt; ++i) {
+        const int b = list[i];
+        const int64_t h = changed[b];
+        const unsigned long long bit = 1ull << (b & 63);
+        const int64_t at = (int64_t)((g + b) % G) * blockDim.x + threadIdx.x;  // short rows start on different CTAs
+        for (int dir = 0; dir < 2; ++dir) {
+            int64_t p0, p1;
+            const int32_t* col;
+            if (dir) {
+                bspan(A.brow + rp.nbase, h, p0, p1);
+                col = A.bcol + rp.bbase;
+            } else {
+                p0 = A.fwd_off[rp.obase + h];
+                p1 = A.fwd_off[rp.obase + h + 1];
+                col = A.fwd_col + rp.ebase;
+            }
+            for (int64_t p = p0 + at; p < p1; p += stride) {
+                unsigned long long* w = (unsigned long long*)&A.hmask[(rp.nbase + col[p]) * kMaskWords + (b >> 6)];
+                if (SET)
+                    atomicOr(w, bit);
+                else
+                    atomicAnd(w, ~bit);
+            }
         }
     }
+    __syncthreads();  // the list is the next replica's
 }
 
 template <bool SET>
-__global__ void __launch_bounds__(256) k_hub_mask(Arena A, int G) { d_hub_mask<SET>(A, G, blockIdx.x); }
+__global__ void __launch_bounds__(kHeavyMax) k_hub_mask(Arena A, int G) { d_hub_mask<SET>(A, G, blockIdx.x); }
 
-// hub2[b] = OR of hmask over the hub's neighbours: the hubs sharing a neighbour with hub b.
+// hub2[b] = OR of hmask over the hub's neighbours: the hubs sharing a neighbour with hub b; only for
+// the hubs that are some agent's anchor (no other row is read).  CTAs as in d_hub_mask.
 __device__ __forceinline__ void d_hub_pairs(const Arena& A, int G, int vb) {
-    __shared__ unsigned long long acc[kMaskWords];
+    __shared__ int list[kHeavyMax], count;
     if (cta_error(A)) return;
-    const int item = vb / G, g = vb % G;
-    const int r = item / kHeavyMax, b = item % kHeavyMax;
-    if (r >= A.R) return;
+    const int r = vb / G, g = vb % G;
+    const int32_t* hl = A.hlist + (int64_t)r * kHeavyMax;
+    const uint32_t* need = A.hub_need + (int64_t)r * (kHeavyMax / 32);
+    const int cnt = hub_list(list, &count, [&](int b) { return ((need[b >> 5] >> (b & 31)) & 1u) && hl[b] >= 0; });
     const Replica& rp = A.rep[r];
-    const int64_t h = A.hlist[(int64_t)r * kHeavyMax + b];
-    if (h < 0) return;
-    // only an agent whose anchor is hub b reads its row
-    if (!((A.hub_need[(int64_t)r * (kHeavyMax / 32) + (b >> 5)] >> (b & 31)) & 1u)) return;
-    if (threadIdx.x < kMaskWords) acc[threadIdx.x] = 0;
-    __syncthreads();
     const int64_t stride = (int64_t)G * blockDim.x;
-    unsigned long long m[kMaskWords];
+    for (int i = 0; i < cnt; ++i) {
+        const int b = list[i];
+        const int64_t h = hl[b];
+        const int64_t at = (int64_t)((g + b) % G) * blockDim.x + threadIdx.x;
+        unsigned long long m[kMaskWords];
 #pragma unroll
-    for (int w = 0; w < kMaskWords; ++w) m[w] = 0;
-    for (int dir = 0; dir < 2; ++dir) {
-        int64_t p0, p1;
-        const int32_t* col;
-        if (dir) {
-            bspan(A.brow + rp.nbase, h, p0, p1);
-            col = A.bcol + rp.bbase;
-        } else {
-            p0 = A.fwd_off[rp.obase + h];
-            p1 = A.fwd_off[rp.obase + h + 1];
-            col = A.fwd_col + rp.ebase;
+        for (int w = 0; w < kMaskWords; ++w) m[w] = 0;
+        for (int dir = 0; dir < 2; ++dir) {
+            int64_t p0, p1;
+            const int32_t* col;
+            if (dir) {
+                bspan(A.brow + rp.nbase, h, p0, p1);
+                col = A.bcol + rp.bbase;
+            } else {
+                p0 = A.fwd_off[rp.obase + h];
+                p1 = A.fwd_off[rp.obase + h + 1];
+                col = A.fwd_col + rp.ebase;
+            }
+            for (int64_t p = p0 + at; p < p1; p += stride) {
+                const uint64_t* hm = A.hmask + (rp.nbase + col[p]) * kMaskWords;
+#pragma unroll
+                for (int w = 0; w < kMaskWords; ++w) m[w] |= hm[w];
+            }
         }
-        for (int64_t p = p0 + (int64_t)g * blockDim.x + threadIdx.x; p < p1; p += stride) {
-            const uint64_t* hm = A.hmask + (rp.nbase + col[p]) * kMaskWords;
 #pragma unroll
-            for (int w = 0; w < kMaskWords; ++w) m[w] |= hm[w];
+        for (int w = 0; w < kMaskWords; ++w) {
+            unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)m[w]);
+            unsigned hi = __reduce_or_sync(0xffffffffu, (unsigned)(m[w] >> 32));
+            if (lane_id() == 0 && (lo | hi))
+                atomicOr((unsigned long long*)&A.hub2[((int64_t)r * kHeavyMax + b) * kMaskWords + w],
+                         ((unsigned long long)hi << 32) | lo);
         }
-    }
-#pragma unroll
-    for (int w = 0; w < kMaskWords; ++w) {
-        unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)m[w]);
-        unsigned hi = __reduce_or_sync(0xffffffffu, (unsigned)(m[w] >> 32));
-        if (lane_id() == 0 && (lo | hi)) atomicOr(&acc[w], ((unsigned long long)hi << 32) | lo);
     }
     __syncthreads();
-    if (threadIdx.x < kMaskWords && acc[threadIdx.x])
-        atomicOr((unsigned long long*)&A.hub2[((int64_t)r * kHeavyMax + b) * kMaskWords + threadIdx.x],
-                 acc[threadIdx.x]);
 }
 
-__global__ void __launch_bounds__(256) k_hub_pairs(Arena A, int G) { d_hub_pairs(A, G, blockIdx.x); }
+__global__ void __launch_bounds__(kHeavyMax) k_hub_pairs(Arena A, int G) { d_hub_pairs(A, G, blockIdx.x); }
+
+// CTAs per replica of the hub kernels that walk rows: two per SM over all replicas, at least eight
+int hub_ctas(int R, int num_sms) {
+    const int g = 2 * num_sms / R;
+    return g < 8 ? 8 : g;
+}
 
 void launch_hubs(const Arena& A, int num_sms, cudaStream_t s) {
-    (void)num_sms;
-    const int G = A.R >= 64 ? 1 : 64 / A.R;  // CTAs per hub
+    const int G = hub_ctas(A.R, num_sms);
     k_hub_hist<<<A.ntiles, kTileThreads, 0, s>>>(A);
-    k_hub_pick<<<1, 256, 0, s>>>(A);
+    k_hub_pick<<<A.R, kHeavyMax, 0, s>>>(A);
     k_hub_collect<<<A.ntiles, kTileThreads, 0, s>>>(A);
-    k_hub_assign<<<1, 256, 0, s>>>(A);
-    k_hub_mask<false><<<(unsigned)(A.R * kHeavyMax * G), 256, 0, s>>>(A, G);
-    k_hub_mask<true><<<(unsigned)(A.R * kHeavyMax * G), 256, 0, s>>>(A, G);
+    k_hub_assign<<<(unsigned)((A.R + 7) / 8), 256, 0, s>>>(A);  // a warp per replica (one CTA for 256: 190 us)
+    k_hub_mask<false><<<(unsigned)(A.R * G), kHeavyMax, 0, s>>>(A, G);
+    k_hub_mask<true><<<(unsigned)(A.R * G), kHeavyMax, 0, s>>>(A, G);
 }
 
-void launch_hub_pairs(const Arena& A, cudaStream_t s) {
-    const int G = A.R >= 64 ? 1 : 64 / A.R;
-    k_hub_pairs<<<(unsigned)(A.R * kHeavyMax * G), 256, 0, s>>>(A, G);
+void launch_hub_pairs(const Arena& A, int num_sms, cudaStream_t s) {
+    const int G = hub_ctas(A.R, num_sms);
+    k_hub_pairs<<<(unsigned)(A.R * G), kHeavyMax, 0, s>>>(A, G);
 }
 
 void launch_epoch_begin(const Arena& A, int64_t epoch, int pa_mode, cudaStream_t s) {
