@@ -82,6 +82,9 @@ struct Checkpoint {
     DBuf<int64_t> fwd_off;
     DBuf<BRow> brow;
     DBuf<Replica> rep;
+    DBuf<CopySeg> segs;  // what a restore copies
+    int num_segs = 0;
+    int64_t chunks = 0;
 };
 
 }  // namespace
@@ -408,6 +411,7 @@ void free_checkpoint(Checkpoint& k) {
     dfree(k.brow);
     dfree(k.bcap);
     dfree(k.rep);
+    dfree(k.segs);
     dfree(k.rc_lag);
     dfree(k.rc_dur);
     k.valid = false;
@@ -1980,12 +1984,41 @@ pg_status pg_checkpoint(pg_ctx* c) {
     PG_CUDA(c, cudaMemcpyAsync(k.brow.p, c->brow.p, sizeof(BRow) * (size_t)c->S, d2d, s));
     PG_CUDA(c, cudaMemcpyAsync(k.bcap.p, c->bcap.p, sizeof(int32_t) * (size_t)c->S, d2d, s));
     PG_CUDA(c, cudaMemcpyAsync(k.rep.p, c->rep.p, sizeof(Replica) * (size_t)c->R, d2d, s));
+    // the hub index is not part of the checkpoint: the epoch after a restore rebuilds it
+    PG_CUDA(c, cudaMemset2DAsync(reinterpret_cast<char*>(k.rep.p) + offsetof(Replica, hub_valid), sizeof(Replica), 0,
+                                 sizeof(int32_t), (size_t)c->R, s));
+    std::vector<CopySeg> segs;
+    k.chunks = 0;
+    auto put_back = [&](void* dst, const void* src, size_t bytes) {
+        if (!bytes) return;
+        segs.push_back(CopySeg{static_cast<const char*>(src), static_cast<char*>(dst), (int64_t)bytes, k.chunks});
+        k.chunks += ((int64_t)bytes + kCopyChunk - 1) / kCopyChunk;
+    };
+    const size_t S = (size_t)c->S;
+    static_assert(sizeof(Replica) % 4 == 0 && sizeof(BRow) % 4 == 0, "whole words");
+    if (c->cfg.weight_model == PG_WEIGHTS_REFCOMPAT) {
+        put_back(c->rc_lag.p, k.rc_lag.p, 4 * S);
+        put_back(c->rc_dur.p, k.rc_dur.p, 4 * S);
+    }
+    put_back(c->pub.p, k.pub.p, 4 * S);
+    put_back(c->indeg.p, k.indeg.p, 4 * S);
+    put_back(c->fit.p, k.fit.p, 4 * S);
+    put_back(c->fwd_off.p, k.fwd_off.p, 8 * (S + (size_t)c->R));
+    put_back(c->brow.p, k.brow.p, sizeof(BRow) * S);
+    put_back(c->bcap.p, k.bcap.p, sizeof(int32_t) * S);
+    put_back(c->rep.p, k.rep.p, sizeof(Replica) * (size_t)c->R);
+    put_back(c->inc.p, nullptr, 4 * S);
     for (int r = 0; r < c->R; ++r) {
         const HostRep& h = c->hrep[(size_t)r];
         if (h.m) PG_CUDA(c, cudaMemcpyAsync(k.fwd_col.p + h.ebase, c->fwd_col.p + h.ebase, 4 * (size_t)h.m, d2d, s));
         const int64_t top = k.b_top[(size_t)r];
         if (top) PG_CUDA(c, cudaMemcpyAsync(k.bcol.p + h.bbase, c->bcol.p + h.bbase, 4 * (size_t)top, d2d, s));
+        put_back(c->fwd_col.p + h.ebase, k.fwd_col.p + h.ebase, 4 * (size_t)h.m);
+        put_back(c->bcol.p + h.bbase, k.bcol.p + h.bbase, 4 * (size_t)top);
     }
+    k.num_segs = (int)segs.size();
+    if (k.segs.n < (int64_t)segs.size()) PG_CUDA(c, dalloc(k.segs, (int64_t)segs.size()));
+    PG_CUDA(c, cudaMemcpyAsync(k.segs.p, segs.data(), sizeof(CopySeg) * segs.size(), cudaMemcpyHostToDevice, s));
     PG_CUDA(c, cudaStreamSynchronize(s));
     k.epoch = c->epoch;
     k.hrep = c->hrep;
@@ -1998,33 +2031,13 @@ pg_status pg_restore(pg_ctx* c) {
     Checkpoint& k = c->ckpt;
     if (!k.valid || k.pub.n != c->S || k.fwd_col.n != c->M || k.bcol.n != c->B)
         return fail(c, PG_ERR_STATE, "no checkpoint matches the current arena");
-    cudaStream_t s = c->stream;
-    const cudaMemcpyKind d2d = cudaMemcpyDeviceToDevice;
-    if (c->cfg.weight_model == PG_WEIGHTS_REFCOMPAT && k.rc_lag.n == c->S) {
-        PG_CUDA(c, cudaMemcpyAsync(c->rc_lag.p, k.rc_lag.p, 4 * (size_t)c->S, d2d, s));
-        PG_CUDA(c, cudaMemcpyAsync(c->rc_dur.p, k.rc_dur.p, 4 * (size_t)c->S, d2d, s));
-    }
-    PG_CUDA(c, cudaMemcpyAsync(c->pub.p, k.pub.p, 4 * (size_t)c->S, d2d, s));
-    PG_CUDA(c, cudaMemcpyAsync(c->indeg.p, k.indeg.p, 4 * (size_t)c->S, d2d, s));
-    PG_CUDA(c, cudaMemcpyAsync(c->fit.p, k.fit.p, 4 * (size_t)c->S, d2d, s));
-    PG_CUDA(c, cudaMemcpyAsync(c->fwd_off.p, k.fwd_off.p, 8 * (size_t)(c->S + c->R), d2d, s));
-    PG_CUDA(c, cudaMemcpyAsync(c->brow.p, k.brow.p, sizeof(BRow) * (size_t)c->S, d2d, s));
-    PG_CUDA(c, cudaMemcpyAsync(c->bcap.p, k.bcap.p, sizeof(int32_t) * (size_t)c->S, d2d, s));
-    PG_CUDA(c, cudaMemcpyAsync(c->rep.p, k.rep.p, sizeof(Replica) * (size_t)c->R, d2d, s));
-    // the hub index is not part of the checkpoint: the next epoch rebuilds it
-    PG_CUDA(c, cudaMemset2DAsync(reinterpret_cast<char*>(c->rep.p) + offsetof(Replica, hub_valid), sizeof(Replica), 0,
-                                 sizeof(int32_t), (size_t)c->R, s));
-    for (size_t r = 0; r < k.hrep.size(); ++r) {
-        const HostRep& h = k.hrep[r];
-        if (h.m) PG_CUDA(c, cudaMemcpyAsync(c->fwd_col.p + h.ebase, k.fwd_col.p + h.ebase, 4 * (size_t)h.m, d2d, s));
-        const int64_t top = k.b_top[r];
-        if (top) PG_CUDA(c, cudaMemcpyAsync(c->bcol.p + h.bbase, k.bcol.p + h.bbase, 4 * (size_t)top, d2d, s));
-    }
-    PG_CUDA(c, cudaMemsetAsync(c->inc.p, 0, 4 * (size_t)c->S, s));
-    // the saved state is consistent: clear the error word a failed epoch left set
-    PG_CUDA(c, cudaMemsetAsync(reinterpret_cast<char*>(c->st.p) + offsetof(EpochState, error), 0,
-                               sizeof(uint32_t), s));
-    PG_CUDA(c, cudaStreamSynchronize(s));
+    PG_CUDA(c, cudaSetDevice(c->device));
+    // the arrays put back in one launch, which also clears the error word a failed epoch left set: the
+    // saved state is consistent
+    cudaGetLastError();
+    launch_copy_segments(k.segs.p, k.num_segs, k.chunks, c->st.p, c->num_sms, c->stream);
+    PG_CUDA(c, cudaGetLastError());
+    PG_CUDA(c, cudaStreamSynchronize(c->stream));
     c->epoch = k.epoch;
     c->hrep = k.hrep;
     c->poisoned = false;

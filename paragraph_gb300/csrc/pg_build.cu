@@ -581,4 +581,51 @@ void launch_build_all(int32_t* src, int32_t* dst, int64_t m, const int64_t* raw_
     k_rep_totals<<<1, 256, 0, s>>>(go, gbeg, R, rep, u, laid);
 }
 
+// A restore is the arrays of the arena (and, of every replica, the used parts of the edge regions), some
+// ten ranges for one replica and 520 for the 256 of an ensemble: a copy call each was 3.4 ms of the
+// device's time and as much of the host's for 1.6 GB.  CTAs take 32 KB chunks in turn, eight 16-byte
+// loads in flight per thread.
+__global__ void __launch_bounds__(256) k_copy_segments(const CopySeg* __restrict__ segs, int num, int64_t chunks,
+                                                       EpochState* st) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->error = 0u;
+    for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+        int lo = 0, hi = num - 1;  // the last segment whose first chunk is at or before c
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (segs[mid].first <= c)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        const CopySeg g = segs[lo];
+        const int64_t off = (c - g.first) * kCopyChunk;
+        const int bytes = (int)(g.bytes - off < kCopyChunk ? g.bytes - off : kCopyChunk);
+        const int nv = bytes >> 4;
+        constexpr int kU = kCopyChunk / 16 / 256;
+        int4* d = reinterpret_cast<int4*>(g.dst + off);
+        const int4* f = reinterpret_cast<const int4*>(g.src + off);
+        int4 v[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int i = u * 256 + (int)threadIdx.x;
+            v[u] = g.src && i < nv ? __ldcs(f + i) : make_int4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int i = u * 256 + (int)threadIdx.x;
+            if (i < nv) d[i] = v[u];
+        }
+        const int t = nv * 4 + (int)threadIdx.x;  // the last words
+        if (t < bytes >> 2)
+            reinterpret_cast<int32_t*>(d)[t] = g.src ? reinterpret_cast<const int32_t*>(f)[t] : 0;
+    }
+}
+
+void launch_copy_segments(const CopySeg* segs, int num, int64_t chunks, EpochState* st, int num_sms, cudaStream_t s) {
+    int64_t g = chunks;
+    if (g > (int64_t)num_sms * 8) g = (int64_t)num_sms * 8;
+    if (g < 1) g = 1;
+    k_copy_segments<<<(unsigned)g, 256, 0, s>>>(segs, num, chunks, st);
+}
+
 }  // namespace pg

@@ -475,6 +475,17 @@ void launch_er_epoch(const Arena& A, int64_t delta, double p, const ErPlan& P, c
                      cudaStream_t s);
 // the skip constants of probability p (host)
 ErSkip er_skip_constants(double p);
+// Copies many device ranges in one launch: each segment's bytes (a multiple of 4, both ends 16-byte
+// aligned) from src to dst, or zeroes to dst where src is null.  Segments are cut into chunks of
+// kCopyChunk bytes, `first` the segment's first chunk; st->error is cleared.
+constexpr int64_t kCopyChunk = 32768;
+struct CopySeg {
+    const char* src;
+    char* dst;
+    int64_t bytes;
+    int64_t first;
+};
+void launch_copy_segments(const CopySeg* segs, int num, int64_t chunks, EpochState* st, int num_sms, cudaStream_t s);
 // generic exclusive scan of n values; out has n+1 entries (out[n] = total)
 void launch_scan_i64(const int64_t* in, int64_t* out, int64_t n, int64_t* blocksum, cudaStream_t s);
 void launch_scan_i32_to_i64(const int32_t* in, int64_t* out, int64_t n, int64_t* blocksum,

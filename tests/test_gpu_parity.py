@@ -607,3 +607,29 @@ def test_enumeration_lists_and_race_bit_exact(gpu, n0, delta, lam, beta, anchors
             for k in ("rows_expanded", "elems_streamed", "draws"):
                 assert st[k] == so[k], k
             _compare_state(eng, og)
+
+
+@pytest.mark.parametrize("sizes", [[61], [3000], [1025, 40, 5000, 333, 2048], [400] * 70])
+def test_restore_puts_every_array_back(gpu, sizes):
+    """A restore copies all arrays in one launch, cut into 32 KB chunks: odd ends of every replica's edge
+    regions, regions shorter than a vector, more segments than a chunk search step."""
+    prm = PAParams(mean_out_degree=9.0, growth_rate=0.1, fixed_new_nodes=0)
+    reps = [ReplicaInput(g.pub, g.fitness, g.src, g.dst, prm, planned_epochs=4)
+            for g in (W.plain_pa_seed(n, 1 + i % 7, seed=50 + i) for i, n in enumerate(sizes))]
+    with GrowthEngine(seed=3, replicas=len(reps)) as eng:
+        eng.load_replicas(reps)
+        eng.run_epochs(2, use_graph=False)
+
+        def state():
+            return [x for r in range(len(reps)) for x in (*eng.csr(0, r), *eng.csr(1, r), *eng.degrees(r), *eng.nodes(r))]
+
+        before = state()
+        eng.checkpoint()
+        first = eng.run_epochs(2, use_graph=False)
+        grown = state()
+        eng.restore()
+        for a, b in zip(before, state()):
+            np.testing.assert_array_equal(a, b)
+        assert eng.run_epochs(2, use_graph=False) == first
+        for a, b in zip(grown, state()):
+            np.testing.assert_array_equal(a, b)
