@@ -13,9 +13,11 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <mutex>
 #include <new>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/paragraph_gb300.h"
@@ -44,6 +46,7 @@ template <typename T>
 struct DBuf {
     T* p = nullptr;
     int64_t n = 0;
+    bool own = true;  // false: a part of the arena's one allocation
 };
 
 // A loaded growth trace and the buffers of the likelihood passes.
@@ -105,6 +108,7 @@ struct pg_ctx {
     int64_t B = 0;                // backward-region entries (all replicas)
     int64_t agent_cap = 0, edge_cap = 0, blocks_cap = 0;
     // device buffers
+    DBuf<char> arena;  // the graph's arrays below, one allocation (lay_arena)
     DBuf<Replica> rep;
     DBuf<EpochState> st;
     DBuf<int32_t> tile_rep, pub, indeg, inc, kk, big_list, heavy_list, heavy_mark, e_dst, e_rank, arrivals, hlist, anchors,
@@ -134,6 +138,8 @@ struct pg_ctx {
     DBuf<int32_t> rc_lag, rc_dur, rc_cnt;
     DBuf<uint64_t> rc_ftab;
     DBuf<unsigned long long> rc_acc;
+    char* pinned = nullptr;  // page-locked staging of what a run reads back (read_back)
+    size_t pinned_bytes = 0;
     // host mirror of the last epoch
     EpochState h_st{};
     std::vector<Replica> h_rep;
@@ -156,6 +162,7 @@ struct pg_ctx {
     int32_t* out_dst = nullptr;
     int64_t out_cap = 0, out_epochs = 0;
     DBuf<int64_t> out_counts;
+    int64_t* out_counts_host = nullptr;  // where the run's counts go (pg_run_epochs_out's argument)
     DBuf<int32_t> out_stage_src, out_stage_dst;  // staging when the caller's buffers are pageable
     Checkpoint ckpt;
     LikState lik;
@@ -180,9 +187,10 @@ pg_status fail(pg_ctx* c, pg_status s, const std::string& msg) {
 
 template <typename T>
 cudaError_t dalloc(DBuf<T>& b, int64_t n) {
-    if (b.p) cudaFree(b.p);
+    if (b.p && b.own) cudaFree(b.p);
     b.p = nullptr;
     b.n = 0;
+    b.own = true;
     if (n <= 0) n = 1;
     cudaError_t e = cudaMalloc((void**)&b.p, sizeof(T) * (size_t)n);
     if (e == cudaSuccess) b.n = n;
@@ -191,20 +199,28 @@ cudaError_t dalloc(DBuf<T>& b, int64_t n) {
 
 template <typename T>
 void dfree(DBuf<T>& b) {
-    if (b.p) cudaFree(b.p);
+    if (b.p && b.own) cudaFree(b.p);
     b.p = nullptr;
     b.n = 0;
 }
 
-// Temporaries of a load (raw edges, sort scratch, offset-form CSR) come from a stream-ordered pool
-// owned by the library: freeing them does not synchronise the device, and a later load in the same
-// process reuses the memory instead of mapping it again.  The pool keeps what it holds (release
-// threshold: unlimited) until the process ends: at most one load's temporaries, about 40 bytes per
-// raw edge.
+// Temporaries of a load (raw edges, sort scratch, offset-form CSR) and of a text export come from a
+// stream-ordered pool owned by the library: allocating and freeing them does not synchronise the device,
+// and a later call reuses the memory instead of mapping it again.  The pool holds at most what the
+// largest call needed (about 40 bytes per raw edge of a load, 60 per edge of an export) and is
+// given back when the device's last context is destroyed.
+struct TempPool {
+    cudaMemPool_t pool = nullptr;
+    int contexts = 0;
+};
+std::mutex g_pool_guard;  // contexts of several threads share a device's pool
+TempPool g_pools[64];
+
 cudaMemPool_t temp_pool(int device) {
-    static cudaMemPool_t pools[64] = {};
     if (device < 0 || device >= 64) return nullptr;
-    if (!pools[device]) {
+    const std::lock_guard<std::mutex> hold(g_pool_guard);
+    cudaMemPool_t& pool = g_pools[device].pool;
+    if (!pool) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.handleTypes = cudaMemHandleTypeNone;
@@ -217,9 +233,18 @@ cudaMemPool_t temp_pool(int device) {
         }
         uint64_t keep = ~0ull;
         cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-        pools[device] = p;
+        pool = p;
     }
-    return pools[device];
+    return pool;
+}
+
+// a context begins (+1) or ends (-1) on the device; the last one's end empties the pool
+void pool_contexts(int device, int by) {
+    if (device < 0 || device >= 64) return;
+    const std::lock_guard<std::mutex> hold(g_pool_guard);
+    TempPool& t = g_pools[device];
+    t.contexts += by;
+    if (t.contexts == 0 && t.pool) cudaMemPoolTrimTo(t.pool, 0);
 }
 
 template <typename T>
@@ -491,6 +516,79 @@ struct HostGraph {
     std::vector<int32_t> lag, dur;  // refcompat fitness windows (empty: lag 0, duration 1000)
 };
 
+// The graph's arrays for the arena's S slots, T tiles, M edge slots, B backward entries and R replicas, cut
+// from one allocation: 30 calls of cudaMalloc and cudaFree were 1.6 of the 4.4 ms of a 400k-node load
+// and run.  A load that needs less than the allocation holds, and more than half of it, keeps it.
+cudaError_t lay_arena(pg_ctx* c, int R) {
+    const int64_t S = c->S, T = c->T, M = c->M, B = c->B;
+    const bool rc = c->cfg.weight_model == PG_WEIGHTS_REFCOMPAT;
+    size_t at = 0;
+    char* mem = nullptr;
+    auto take = [&](auto& b, int64_t n) {
+        using E = std::remove_reference_t<decltype(*b.p)>;
+        if (b.p && b.own) cudaFree(b.p);
+        b.p = mem ? reinterpret_cast<E*>(mem + at) : nullptr;
+        b.n = mem ? n : 0;
+        b.own = false;
+        at += (sizeof(E) * (size_t)std::max<int64_t>(n, 1) + 255) / 256 * 256;
+    };
+    auto lay = [&]() {
+        at = 0;
+        take(c->rep, R);
+        take(c->tile_rep, T);
+        take(c->tilesum, std::max<int64_t>(T, R) + 1);
+        take(c->tileoff, T + 1);
+        take(c->pub, S);
+        take(c->fit, S);
+        take(c->indeg, S);
+        take(c->inc, S);
+        take(c->w, S);
+        take(c->cdf, S);
+        take(c->guide, S);
+        take(c->new_start, S);
+        take(c->sort_small, S);
+        take(c->sort_large, S);
+        take(c->sort_large_off, S);
+        take(c->fwd_off, S + R);
+        take(c->fwd_col, M);
+        take(c->brow, S);
+        take(c->bcap, S);
+        take(c->bcol, B);
+        take(c->tables, (int64_t)R * kTableEntries);
+        take(c->hslot, S);
+        take(c->hmask, S * kMaskWords);
+        take(c->hub2, (int64_t)R * kHeavyMax * kMaskWords);
+        take(c->hub_need, (int64_t)R * (kHeavyMax / 32));
+        take(c->hlist, (int64_t)R * kHeavyMax);
+        take(c->hub_rem, (int64_t)R * kHeavyMax);
+        take(c->hub_add, (int64_t)R * kHeavyMax);
+        take(c->hub_cand, (int64_t)R * kHeavyMax);
+        if (rc) {
+            take(c->rc_pa, S);
+            take(c->rc_s32, S);
+            take(c->rc_rec, S);
+            take(c->rc_fit, S);
+            take(c->rc_lag, S);
+            take(c->rc_dur, S);
+            take(c->rc_acc, 4 * (int64_t)R);
+            take(c->rc_cnt, (int64_t)R * kRcAgeMax);
+            take(c->rc_rtab, (int64_t)R * kRcAgeMax);
+        }
+    };
+    lay();  // sizes only
+    const int64_t need = (int64_t)at;
+    if (c->arena.n < need || c->arena.n / 2 > need + (32 << 20)) {
+        const cudaError_t e = dalloc(c->arena, need);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return e;
+        }
+    }
+    mem = c->arena.p;
+    lay();
+    return cudaSuccess;
+}
+
 // raw != nullptr: the replicas' CSRs are built on the device from raw[r].src / raw[r].dst (h.m is
 // an upper bound on entry and the unique edge count on return); else hg holds host CSRs.
 pg_status upload_arena(pg_ctx* c, std::vector<HostRep>& reps, const std::vector<HostGraph>& hg,
@@ -593,38 +691,11 @@ pg_status upload_arena(pg_ctx* c, std::vector<HostRep>& reps, const std::vector<
     c->B = B;
     destroy_graph_exec(c);
     c->ckpt.valid = false;
-    PG_CUDA(c, dalloc(c->rep, R));
-    PG_CUDA(c, dalloc(c->tile_rep, T));
-    PG_CUDA(c, dalloc(c->tilesum, std::max<int64_t>(T, R) + 1));
-    PG_CUDA(c, dalloc(c->tileoff, T + 1));
-    PG_CUDA(c, dalloc(c->pub, S));
-    PG_CUDA(c, dalloc(c->fit, S));
-    PG_CUDA(c, dalloc(c->indeg, S));
-    PG_CUDA(c, dalloc(c->inc, S));
-    PG_CUDA(c, dalloc(c->w, S));
-    PG_CUDA(c, dalloc(c->cdf, S));
-    PG_CUDA(c, dalloc(c->guide, S));
-    PG_CUDA(c, dalloc(c->new_start, S));
-    PG_CUDA(c, dalloc(c->sort_small, S));
-    PG_CUDA(c, dalloc(c->sort_large, S));
-    PG_CUDA(c, dalloc(c->sort_large_off, S));
-    PG_CUDA(c, dalloc(c->fwd_off, S + R));
-    PG_CUDA(c, dalloc(c->fwd_col, M));
-    PG_CUDA(c, dalloc(c->brow, S));
-    PG_CUDA(c, dalloc(c->bcap, S));
-    PG_CUDA(c, dalloc(c->bcol, B));
-    PG_CUDA(c, dalloc(c->tables, (int64_t)R * kTableEntries));
-    PG_CUDA(c, dalloc(c->hslot, S));
-    PG_CUDA(c, dalloc(c->hmask, S * kMaskWords));
-    PG_CUDA(c, dalloc(c->hub2, (int64_t)R * kHeavyMax * kMaskWords));
-    PG_CUDA(c, dalloc(c->hub_need, (int64_t)R * (kHeavyMax / 32)));
-    PG_CUDA(c, dalloc(c->hlist, (int64_t)R * kHeavyMax));
-    PG_CUDA(c, dalloc(c->hub_rem, (int64_t)R * kHeavyMax));
-    PG_CUDA(c, dalloc(c->hub_add, (int64_t)R * kHeavyMax));
-    PG_CUDA(c, dalloc(c->hub_cand, (int64_t)R * kHeavyMax));
+    if (lay_arena(c, R) != cudaSuccess) {
+        c->loaded = false;  // the arrays of the graph that was loaded are gone
+        return fail(c, PG_ERR_CUDA, "out of device memory for the graph");
+    }
     if (c->cfg.weight_model == PG_WEIGHTS_REFCOMPAT) {
-        PG_CUDA(c, dalloc(c->rc_pa, S));
-        PG_CUDA(c, dalloc(c->rc_s32, S));
         if (!c->rc_big_id.p) {
             PG_CUDA(c, dalloc(c->rc_big_id, (int64_t)kRcBigCap * kKMax));
             PG_CUDA(c, dalloc(c->rc_big_meta, (int64_t)kRcBigCap * 3));
@@ -635,13 +706,6 @@ pg_status upload_arena(pg_ctx* c, std::vector<HostRep>& reps, const std::vector<
             PG_CUDA(c, dalloc(c->rc_ticket, kRcBigCap));
             PG_CUDA(c, cudaMemsetAsync(c->rc_ticket.p, 0, 4 * (size_t)kRcBigCap, c->stream));
         }
-        PG_CUDA(c, dalloc(c->rc_rec, S));
-        PG_CUDA(c, dalloc(c->rc_fit, S));
-        PG_CUDA(c, dalloc(c->rc_lag, S));
-        PG_CUDA(c, dalloc(c->rc_dur, S));
-        PG_CUDA(c, dalloc(c->rc_acc, 4 * (int64_t)R));
-        PG_CUDA(c, dalloc(c->rc_cnt, (int64_t)R * kRcAgeMax));
-        PG_CUDA(c, dalloc(c->rc_rtab, (int64_t)R * kRcAgeMax));
         if (!c->rc_ftab.p) {
             std::vector<uint64_t> ft(kRcFitMax);
             rc_fitness_table_host(ft.data());
@@ -912,12 +976,28 @@ pg_status ensure_capacity(pg_ctx* c, int64_t need_n, int64_t need_m) {
     return upload_arena(c, reps, hg);
 }
 
-pg_status read_back(pg_ctx* c) {
-    PG_CUDA(c, cudaMemcpyAsync(&c->h_st, c->st.p, sizeof(EpochState), cudaMemcpyDeviceToHost, c->stream));
-    c->h_rep.resize((size_t)c->R);
-    PG_CUDA(c, cudaMemcpyAsync(c->h_rep.data(), c->rep.p, sizeof(Replica) * (size_t)c->R,
-                               cudaMemcpyDeviceToHost, c->stream));
+// The epoch state, the replicas and (counts != null) the nc citation counts of a run with output, through
+// page-locked memory: one wait for all three (a copy into pageable memory waits by itself, and
+// starts only after the wait before it).
+pg_status read_back(pg_ctx* c, int64_t* counts = nullptr, int64_t nc = 0) {
+    const size_t rb = sizeof(Replica) * (size_t)c->R, cb = counts ? 8 * (size_t)nc : 0;
+    const size_t need = sizeof(EpochState) + rb + cb;
+    if (c->pinned_bytes < need) {
+        if (c->pinned) cudaFreeHost(c->pinned);
+        c->pinned = nullptr;
+        c->pinned_bytes = 0;
+        PG_CUDA(c, cudaHostAlloc((void**)&c->pinned, need + need / 2, cudaHostAllocDefault));
+        c->pinned_bytes = need + need / 2;
+    }
+    char* reps = c->pinned + sizeof(EpochState);
+    PG_CUDA(c, cudaMemcpyAsync(c->pinned, c->st.p, sizeof(EpochState), cudaMemcpyDeviceToHost, c->stream));
+    PG_CUDA(c, cudaMemcpyAsync(reps, c->rep.p, rb, cudaMemcpyDeviceToHost, c->stream));
+    if (cb) PG_CUDA(c, cudaMemcpyAsync(reps + rb, c->out_counts.p, cb, cudaMemcpyDeviceToHost, c->stream));
     PG_CUDA(c, cudaStreamSynchronize(c->stream));
+    std::memcpy(&c->h_st, c->pinned, sizeof(EpochState));
+    c->h_rep.resize((size_t)c->R);
+    std::memcpy(c->h_rep.data(), reps, rb);
+    if (cb) std::memcpy(counts, reps + rb, cb);
     return PG_OK;
 }
 
@@ -1196,6 +1276,7 @@ pg_status pg_create(pg_ctx** out, const pg_config* cfg) {
     c->cfg = *cfg;
     c->R = cfg->num_replicas;
     c->device = cfg->device;
+    pool_contexts(c->device, 1);
     cudaError_t e = cudaSetDevice(c->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
@@ -1281,6 +1362,7 @@ void pg_destroy(pg_ctx* c) {
     dfree(c->zbig);
     dfree(c->src_tmp);
     dfree(c->rep);
+    dfree(c->arena);
     dfree(c->st);
     for (int i = 0; i < 6; ++i)
         if (c->ev[i]) cudaEventDestroy(c->ev[i]);
@@ -1293,6 +1375,8 @@ void pg_destroy(pg_ctx* c) {
     if (c->join) cudaEventDestroy(c->join);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->stream) cudaStreamDestroy(c->stream);
+    if (c->pinned) cudaFreeHost(c->pinned);
+    pool_contexts(c->device, -1);
     delete c;
 }
 
@@ -1537,7 +1621,7 @@ pg_status pg_run_epochs(pg_ctx* c, int32_t num_epochs, int32_t use_graph, int64_
         }
     }
     PG_CUDA(c, cudaGetLastError());
-    s = read_back(c);
+    s = read_back(c, c->out_counts_host, c->out_epochs * c->R);
     if (s != PG_OK) return s;
     s = device_error(c);
     if (s != PG_OK) return s;
@@ -1625,10 +1709,13 @@ pg_status pg_run_epochs_out(pg_ctx* c, int32_t num_epochs, int32_t use_graph, in
     c->out_dst = dd;
     c->out_cap = capacity;
     c->out_epochs = num_epochs;
+    std::vector<int64_t> run_counts((size_t)nc, 0);  // handed over when the run has succeeded
+    c->out_counts_host = run_counts.data();
     int64_t ne = 0;
     pg_status s = pg_run_epochs(c, num_epochs, use_graph, &ne);
     c->out_src = c->out_dst = nullptr;
     c->out_cap = c->out_epochs = 0;
+    c->out_counts_host = nullptr;
     if (s != PG_OK) return s;
     // epochs whose citations did not fit the buffers were grown all the same; the caller learns of it
     const bool short_out = c->h_st.out_short != 0;
@@ -1637,9 +1724,8 @@ pg_status pg_run_epochs_out(pg_ctx* c, int32_t num_epochs, int32_t use_graph, in
         PG_CUDA(c, cudaMemcpyAsync(src, ds, 4 * (size_t)ne, cudaMemcpyDeviceToHost, c->stream));
         PG_CUDA(c, cudaMemcpyAsync(dst, dd, 4 * (size_t)ne, cudaMemcpyDeviceToHost, c->stream));
     }
-    if (counts)
-        PG_CUDA(c, cudaMemcpyAsync(counts, c->out_counts.p, 8 * (size_t)nc, cudaMemcpyDeviceToHost, c->stream));
-    PG_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (counts) std::memcpy(counts, run_counts.data(), 8 * (size_t)nc);
+    if (staged && ne > 0) PG_CUDA(c, cudaStreamSynchronize(c->stream));
     if (new_edges) *new_edges = ne;
     if (short_out)
         return fail(c, PG_ERR_CAPACITY, "output buffers hold " + std::to_string(capacity) + " citations; the run made " +
@@ -2307,22 +2393,23 @@ pg_status pg_format_edges(pg_ctx* c, int32_t replica, const int64_t* ids, int64_
     if (n_ids != h.n) return fail(c, PG_ERR_ARG, "ids must hold one id per node");
     PG_CUDA(c, cudaSetDevice(c->device));
     const int64_t n = h.n, m = h.m;
-    struct Tmp {
+    struct Tmp {  // from the temporaries' pool: allocating and freeing were 1.9 ms of a 2.3 ms export
+        pg_ctx* c;
         DBuf<int64_t> did, off, bs;
         DBuf<int32_t> len;
         DBuf<char> txt;
         ~Tmp() {
-            dfree(did);
-            dfree(off);
-            dfree(bs);
-            dfree(len);
-            dfree(txt);
+            tfree(did, c->device, c->stream);
+            tfree(off, c->device, c->stream);
+            tfree(bs, c->device, c->stream);
+            tfree(len, c->device, c->stream);
+            tfree(txt, c->device, c->stream);
         }
-    } t;
-    PG_CUDA(c, dalloc(t.did, n));
-    PG_CUDA(c, dalloc(t.len, std::max<int64_t>(m, 1)));
-    PG_CUDA(c, dalloc(t.off, m + 1));
-    PG_CUDA(c, dalloc(t.bs, scan_blocks_needed(std::max<int64_t>(m, 1)) + 2));
+    } t{c};
+    PG_CUDA(c, talloc(t.did, n, c->device, c->stream));
+    PG_CUDA(c, talloc(t.len, std::max<int64_t>(m, 1), c->device, c->stream));
+    PG_CUDA(c, talloc(t.off, m + 1, c->device, c->stream));
+    PG_CUDA(c, talloc(t.bs, scan_blocks_needed(std::max<int64_t>(m, 1)) + 2, c->device, c->stream));
     PG_CUDA(c, cudaMemcpyAsync(t.did.p, ids, 8 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
     const int64_t* fo = c->fwd_off.p + h.obase;
     const int32_t* fc = c->fwd_col.p + h.ebase;
@@ -2338,7 +2425,7 @@ pg_status pg_format_edges(pg_ctx* c, int32_t replica, const int64_t* ids, int64_
     if (cap < total)
         return fail(c, PG_ERR_CAPACITY, "the output buffer holds " + std::to_string(cap) + " bytes, the text needs " +
                                             std::to_string(total));
-    PG_CUDA(c, dalloc(t.txt, std::max<int64_t>(total, 1)));
+    PG_CUDA(c, talloc(t.txt, std::max<int64_t>(total, 1), c->device, c->stream));
     launch_text_write(fo, fc, n, m, t.did.p, t.off.p, t.txt.p, c->num_sms, c->stream);
     PG_CUDA(c, cudaGetLastError());
     PG_CUDA(c, cudaMemcpyAsync(out, t.txt.p, (size_t)total, cudaMemcpyDeviceToHost, c->stream));
@@ -2358,30 +2445,31 @@ pg_status pg_format_attributes(pg_ctx* c, int32_t replica, const pg_attr_rows* r
     if (!rows->ids || !rows->draws || !rows->ints || (!rows->generators && rows->num_seed < n))
         return fail(c, PG_ERR_ARG, "ids, draws, ints and generators are required");
     PG_CUDA(c, cudaSetDevice(c->device));
-    struct Tmp {
+    struct Tmp {  // from the temporaries' pool: allocating and freeing were 1.9 ms of a 2.3 ms export
+        pg_ctx* c;
         DBuf<int64_t> did, gen, off, bs;
         DBuf<double> draws;
         DBuf<int32_t> ints, len;
         DBuf<char> txt;
         ~Tmp() {
-            dfree(did);
-            dfree(gen);
-            dfree(off);
-            dfree(bs);
-            dfree(draws);
-            dfree(ints);
-            dfree(len);
-            dfree(txt);
+            tfree(did, c->device, c->stream);
+            tfree(gen, c->device, c->stream);
+            tfree(off, c->device, c->stream);
+            tfree(bs, c->device, c->stream);
+            tfree(draws, c->device, c->stream);
+            tfree(ints, c->device, c->stream);
+            tfree(len, c->device, c->stream);
+            tfree(txt, c->device, c->stream);
         }
-    } t;
+    } t{c};
     const size_t nn = (size_t)std::max<int64_t>(n, 1);
-    PG_CUDA(c, dalloc(t.did, n));
-    PG_CUDA(c, dalloc(t.draws, 4 * n));
-    PG_CUDA(c, dalloc(t.ints, 4 * n));
-    PG_CUDA(c, dalloc(t.gen, 4 * n));
-    PG_CUDA(c, dalloc(t.len, n));
-    PG_CUDA(c, dalloc(t.off, n + 1));
-    PG_CUDA(c, dalloc(t.bs, scan_blocks_needed(std::max<int64_t>(n, 1)) + 2));
+    PG_CUDA(c, talloc(t.did, n, c->device, c->stream));
+    PG_CUDA(c, talloc(t.draws, 4 * n, c->device, c->stream));
+    PG_CUDA(c, talloc(t.ints, 4 * n, c->device, c->stream));
+    PG_CUDA(c, talloc(t.gen, 4 * n, c->device, c->stream));
+    PG_CUDA(c, talloc(t.len, n, c->device, c->stream));
+    PG_CUDA(c, talloc(t.off, n + 1, c->device, c->stream));
+    PG_CUDA(c, talloc(t.bs, scan_blocks_needed(std::max<int64_t>(n, 1)) + 2, c->device, c->stream));
     PG_CUDA(c, cudaMemcpyAsync(t.did.p, rows->ids, 8 * nn, cudaMemcpyHostToDevice, c->stream));
     PG_CUDA(c, cudaMemcpyAsync(t.draws.p, rows->draws, 32 * nn, cudaMemcpyHostToDevice, c->stream));
     PG_CUDA(c, cudaMemcpyAsync(t.ints.p, rows->ints, 16 * nn, cudaMemcpyHostToDevice, c->stream));
@@ -2414,7 +2502,7 @@ pg_status pg_format_attributes(pg_ctx* c, int32_t replica, const pg_attr_rows* r
     if (cap < total)
         return fail(c, PG_ERR_CAPACITY, "the output buffer holds " + std::to_string(cap) + " bytes, the text needs " +
                                             std::to_string(total));
-    PG_CUDA(c, dalloc(t.txt, std::max<int64_t>(total, 1)));
+    PG_CUDA(c, talloc(t.txt, std::max<int64_t>(total, 1), c->device, c->stream));
     launch_attr_text(C, nullptr, t.off.p, t.txt.p, c->num_sms, c->stream);
     PG_CUDA(c, cudaGetLastError());
     PG_CUDA(c, cudaMemcpyAsync(out, t.txt.p, (size_t)total, cudaMemcpyDeviceToHost, c->stream));

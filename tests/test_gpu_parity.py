@@ -633,3 +633,22 @@ def test_restore_puts_every_array_back(gpu, sizes):
         assert eng.run_epochs(2, use_graph=False) == first
         for a, b in zip(grown, state()):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("sizes", [[3000, 60, 2500, 40_000, 3000], [40_000, 900, 39_000]])
+def test_loads_of_other_sizes_into_one_context(gpu, sizes):
+    """A load keeps the context's memory where it fits and is not far too large: smaller, larger and equal
+    graphs in turn grow as they do in a context of their own."""
+    prm = PAParams(mean_out_degree=12.0, growth_rate=0.05, fixed_new_nodes=0)
+    with GrowthEngine(seed=6) as eng:
+        for i, n in enumerate(sizes):
+            g = W.plain_pa_seed(n, 5, seed=70 + i)
+            eng.load_graph(g.pub, g.fitness, g.src, g.dst, prm, planned_epochs=2)
+            with GrowthEngine(seed=6) as own:
+                own.load_graph(g.pub, g.fitness, g.src, g.dst, prm, planned_epochs=2)
+                assert eng.run_epochs(2, use_graph=False) == own.run_epochs(2, use_graph=False)
+                for which in (0, 1):
+                    for a, b in zip(eng.csr(which), own.csr(which)):
+                        np.testing.assert_array_equal(a, b)
+                for a, b in zip((*eng.degrees(), *eng.nodes()), (*own.degrees(), *own.nodes())):
+                    np.testing.assert_array_equal(a, b)
