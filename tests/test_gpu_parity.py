@@ -652,3 +652,33 @@ def test_loads_of_other_sizes_into_one_context(gpu, sizes):
                         np.testing.assert_array_equal(a, b)
                 for a, b in zip((*eng.degrees(), *eng.nodes()), (*own.degrees(), *own.nodes())):
                     np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("deg", [1.5, 8.0, 40.0])
+def test_appended_rows_of_every_sort_class(gpu, deg):
+    """Rows that get 1..8, 9..32, ..256 and more entries in one epoch, several replicas in one sort list."""
+    sizes = [9, 20, 70, 300, 2000]
+    reps = []
+    for i, n in enumerate(sizes):
+        g = W.plain_pa_seed(n, 3, seed=30 + i)
+        reps.append(ReplicaInput(g.pub, g.fitness, g.src, g.dst,
+                                 PAParams(mean_out_degree=deg, fixed_new_nodes=330, growth_rate=0.0), planned_epochs=2))
+    seen = set()
+    with GrowthEngine(seed=6, replicas=len(reps)) as eng:
+        eng.load_replicas(reps)
+        ogs = []
+        for r, ri in enumerate(reps):
+            og = O.OracleGraph(6, r)
+            og.load(ri.pub_epoch, ri.fitness, ri.src, ri.dst)
+            og.set_params(**ri.params.__dict__)
+            ogs.append(og)
+        for _ in range(2):
+            before = [og.degrees()[0] for og in ogs]
+            eng.grow_epoch()
+            for r, og in enumerate(ogs):
+                og.pa_epoch()
+                _compare_state(eng, og, replica=r)
+                new = og.degrees()[0][:len(before[r])] - before[r]
+                seen |= {int(c) for c in np.searchsorted([2, 9, 33, 65, 129, 257], new, side="right")}
+    assert {1, 2} <= seen or deg > 8.0
+    assert seen >= {4, 5, 6} or deg < 8.0
