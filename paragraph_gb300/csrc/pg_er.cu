@@ -205,7 +205,9 @@ __global__ void __launch_bounds__(256) k_er_eoff(Arena A, const int64_t* toff, i
 
 ErSkip er_skip_constants(double p) {
     ErSkip K;
-    K.inv_l = 1.0 / log_pg(1.0 - (p < 1.0 ? p : 1.0));
+    // below 2^-53, 1 - p rounds to 1 and its log to 0: log(1 - p) is -p there (and 1 / p stays finite)
+    const double q = 1.0 - (p < 1.0 ? p : 1.0);
+    K.inv_l = q < 1.0 ? 1.0 / log_pg(q) : -1.0 / (p > 1e-300 ? p : 1e-300);
     K.inv_f = (float)K.inv_l;
     const float a = (float)(fabs(K.inv_l) * 0x1p-23);
     K.dabs = nextafterf(a, INFINITY);  // rounded up

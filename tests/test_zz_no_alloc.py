@@ -90,3 +90,14 @@ def test_noalloc_rejects_oversized_and_small_capacity(gpu):
 
 def pg_max_tasks() -> int:
     return 1 << 18
+
+
+@pytest.mark.parametrize("p", [1e-16, 1e-18, 5e-324])
+def test_probabilities_below_the_rounding_of_one(gpu, p):
+    """1 - p rounds to 1: no edges, from either entry point."""
+    s = W.er_seed(70_000)
+    with GrowthEngine(seed=3) as eng:
+        eng.load_graph(s.pub, s.fitness, s.src, s.dst)
+        assert eng.er_epoch(50, p) == 0
+    st, cnt, _, _ = _noalloc(pg.load_library(), 3, 70_000, 50, p, cap=16)
+    assert (st, cnt) == (pg.PG_OK, 0)
