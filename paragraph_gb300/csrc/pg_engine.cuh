@@ -406,6 +406,48 @@ __device__ __forceinline__ double er_skip(const ErSkip& K, uint32_t lo, uint32_t
     return floor(log_pg(u) * K.inv_l);
 }
 
+// One round of a G(n,p) walk by a group of G lanes.  The gaps of a task (new node i, chunk c) are
+// independent draws, two to a Philox block, so lane l of the group takes block b + l; a prefix sum of
+// 1 + gap over the group turns the 2G gaps into ids after `pos` (relative to the chunk's first id,
+// like len, its length).  q0 and q1 are the lane's ids; the group's successes are those below len, a
+// prefix of its 2G ids in lane order, and their number is returned.  `pos` moves to the group's last
+// id, below len only where all are.  Every lane of the warp has to take part (the shuffles span it);
+// lanes of a group that is done pass act = false.  A gap at or past the chunk's length ends the walk
+// whatever its value, so gaps are cut there and 32 bits hold every sum.
+template <int G>
+__device__ __forceinline__ int er_round(uint64_t seed, uint32_t ep, int64_t i, int64_t c, const ErSkip& K, uint32_t b,
+                                        bool act, int len, int& pos, int& q0, int& q1) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = lane_id(), gl = lane & (G - 1);
+    const unsigned gm = G == 32 ? kAll : (((1u << G) - 1u) << (lane & ~(G - 1)));
+    int s0 = 0, s1 = 0;
+    if (act) {
+        const u32x4 x = draw(seed, kStreamEr, (uint32_t)c, ep, (uint32_t)i, b + (uint32_t)gl);
+        const double k0 = er_skip(K, x.x[0], x.x[1], (float)kErChunk), k1 = er_skip(K, x.x[2], x.x[3], (float)kErChunk);
+        s0 = k0 < (double)kErChunk ? (int)k0 + 1 : (int)kErChunk + 1;
+        s1 = k1 < (double)kErChunk ? (int)k1 + 1 : (int)kErChunk + 1;
+    }
+    int incl = s0 + s1;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+        const int y = __shfl_up_sync(kAll, incl, o, G);
+        if (gl >= o) incl += y;
+    }
+    q1 = pos + incl;
+    q0 = q1 - s1;
+    pos = __shfl_sync(kAll, q1, G - 1, G);
+    return __popc(__ballot_sync(kAll, act && q0 < len) & gm) + __popc(__ballot_sync(kAll, act && q1 < len) & gm);
+}
+
+// Lanes per task of a walk: two gaps per lane, the expected successes of a full chunk and two standard
+// deviations in one round.
+inline int er_lanes(int64_t n, double p) {
+    const double mu = (double)(n < kErChunk ? n : kErChunk) * (p < 1.0 ? p : 1.0);
+    int G = 1;
+    while (G < 32 && 2.0 * G < mu + 2.0 * sqrt(mu)) G <<= 1;
+    return G;
+}
+
 // The device error word as one value for the whole CTA (a barrier and an OR of every thread's
 // read): a body that synchronises its CTA must not let some threads return on an error bit another
 // CTA set a moment later while the rest go on to a barrier.

@@ -69,16 +69,6 @@ __global__ void __launch_bounds__(256) k_er_setup(Arena A, int64_t delta) {
     A.indeg[slot] = 0;
 }
 
-__global__ void __launch_bounds__(256) k_er_walk(Arena A, ErPlan P, ErSkip K, int64_t* cnt, int2* slots) {
-    if (A.st->error) return;
-    const int64_t n = A.rep[0].n;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < P.tasks;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = t / P.chunks, c = t % P.chunks;
-        cnt[t] = er_walk(A, i, c, n, K, er_slots_of(P, c), slots, er_base_of(P, i, c), nullptr, 0);
-    }
-}
-
 __global__ void k_er_check(Arena A, const int64_t* toff, int64_t tasks) {
     if (A.st->error) return;
     const int64_t E = toff[tasks];
@@ -107,43 +97,25 @@ __global__ void __launch_bounds__(256) k_er_overflow(Arena A, ErPlan P, ErSkip K
     }
 }
 
-// The same walk by a group of G lanes: the gaps of a task are independent draws, so the group
-// draws G of them at once (lane l takes draw d0 + l), turns them into positions with a prefix sum
-// of 1 + gap, keeps the prefix that lies below the chunk end and continues from its last position.
-// The positions, their order and the draws consumed are those of er_walk.  Every lane of the warp
-// stays in the loop until all of its groups are done (the shuffles span the warp).
+// The same walk by a group of G lanes (er_round): the positions, their order and the draws consumed
+// are those of er_walk.
 template <int G>
 __device__ __forceinline__ int64_t er_walk_group(const Arena& A, bool live, int64_t i, int64_t c, int64_t n,
                                                  const ErSkip& K, int64_t S, int2* slots, int64_t sbase) {
-    const int lane = lane_id(), gl = lane & (G - 1);
-    const unsigned gm = G == 32 ? kFull : (((1u << G) - 1u) << (lane & ~(G - 1)));
+    const int gl = lane_id() & (G - 1);
     const int64_t lo = c * kErChunk;
-    const int64_t hi = lo + kErChunk < n ? lo + kErChunk : n;
+    const int len = (int)(lo + kErChunk < n ? kErChunk : n - lo);
     const uint32_t ep = (uint32_t)A.st->epoch;
-    int64_t pos = lo - 1, cnt = 0;
+    int64_t cnt = 0;
+    int pos = -1;
     bool act = live;
-    for (uint32_t d0 = 0; __any_sync(kFull, act); d0 += G) {
-        int64_t step = 0;
-        if (act) {
-            const uint32_t d = d0 + (uint32_t)gl;
-            const u32x4 x = draw(A.seed, kStreamEr, (uint32_t)c, ep, (uint32_t)i, d >> 1);
-            const double sk = (d & 1u) ? er_skip(K, x.x[2], x.x[3], (float)kErChunk)
-                                       : er_skip(K, x.x[0], x.x[1], (float)kErChunk);
-            step = sk < 1099511627776.0 ? (int64_t)sk + 1 : ((int64_t)1 << 40);  // 2^40: past any chunk
-        }
-        int64_t incl = step;
-#pragma unroll
-        for (int o = 1; o < G; o <<= 1) {
-            const int64_t y = __shfl_up_sync(kFull, incl, o, G);
-            if (gl >= o) incl += y;
-        }
-        const int64_t q = pos + incl;
-        const bool ok = act && q < hi;  // a prefix of the group: positions increase along it
-        const int nok = __popc(__ballot_sync(kFull, ok) & gm);
-        if (ok) er_put(A, cnt + gl, q, S, slots, sbase, nullptr, 0);
-        cnt += nok;
-        pos = __shfl_sync(kFull, q, G - 1, G);
-        if (nok < G) act = false;
+    for (uint32_t b = 0; __any_sync(kFull, act); b += G) {
+        int q0, q1;
+        const int got = er_round<G>(A.seed, ep, i, c, K, b, act, len, pos, q0, q1);
+        if (act && q0 < len) er_put(A, cnt + 2 * gl, lo + q0, S, slots, sbase, nullptr, 0);
+        if (act && q1 < len) er_put(A, cnt + 2 * gl + 1, lo + q1, S, slots, sbase, nullptr, 0);
+        cnt += got;
+        if (got < 2 * G) act = false;
     }
     return cnt;
 }
@@ -244,15 +216,12 @@ void launch_er_epoch(const Arena& A, int64_t delta, double p, const ErPlan& P, c
         return;
     }
     const ErSkip K = er_skip_constants(p);
-    // lanes per task: about the expected successes of a full chunk (1: one thread walks a task)
-    const double mu = (double)(P.n < kErChunk ? P.n : kErChunk) * (p < 1.0 ? p : 1.0);
-    int G = 1;
-    while (G < 32 && G < mu) G <<= 1;
+    const int G = er_lanes(P.n, p);
     int64_t g = (P.tasks * G + 255) / 256;
     if (g > (int64_t)num_sms * 32) g = (int64_t)num_sms * 32;
     if (g < 1) g = 1;
     switch (G) {
-        case 1: k_er_walk<<<(unsigned)g, 256, 0, s>>>(A, P, K, B.cnt, B.slots); break;
+        case 1: k_er_walk_g<1><<<(unsigned)g, 256, 0, s>>>(A, P, K, B.cnt, B.slots); break;
         case 2: k_er_walk_g<2><<<(unsigned)g, 256, 0, s>>>(A, P, K, B.cnt, B.slots); break;
         case 4: k_er_walk_g<4><<<(unsigned)g, 256, 0, s>>>(A, P, K, B.cnt, B.slots); break;
         case 8: k_er_walk_g<8><<<(unsigned)g, 256, 0, s>>>(A, P, K, B.cnt, B.slots); break;

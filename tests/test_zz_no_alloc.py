@@ -92,6 +92,37 @@ def pg_max_tasks() -> int:
     return 1 << 18
 
 
+@pytest.mark.parametrize("n0,delta,p", [(1, 1, 1.0), (1, 40, 0.5), (1000, 77, 1e-5), (200_000, 40, 3e-5),
+                                        (65_536, 33, 2.5e-4), (65_537, 5, 1e-3), (131_071, 9, 2e-2), (3000, 20, 1.0)])
+def test_noalloc_walks_match_the_oracle(gpu, n0, delta, p):
+    """Every lane-group size of the walk, whole and cut chunks; a buffer one edge short stays untouched."""
+    import oracle as O
+    torch = pytest.importorskip("torch")
+    s = W.er_seed(n0)
+    og = O.OracleGraph(23, 0)
+    og.load(s.pub, s.fitness, s.src, s.dst)
+    og.er_epoch(delta, p)
+    off, col = og.csr(0)
+    ref_src = np.repeat(np.arange(n0 + delta), np.diff(off))
+    lib = pg.load_library()
+    st, cnt, src, dst = _noalloc(lib, 23, n0, delta, p, cap=len(col))
+    assert (st, cnt) == (pg.PG_OK, len(col))
+    np.testing.assert_array_equal(src, ref_src)
+    np.testing.assert_array_equal(dst, col)
+    with GrowthEngine(seed=23) as eng:
+        eng.load_graph(s.pub, s.fitness, s.src, s.dst)
+        eng.er_epoch(delta, p)
+        np.testing.assert_array_equal(eng.csr(0)[1], col)
+    if cnt > 0:
+        buf = torch.full((2, cnt), -7, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        count = C.c_int64(-1)
+        st = lib.pg_er_generate_noalloc(23, 0, n0, delta, p, C.c_void_p(buf[0].data_ptr()),
+                                        C.c_void_p(buf[1].data_ptr()), cnt - 1, C.byref(count), None)
+        assert (st, count.value) == (pg.PG_ERR_CAPACITY, cnt)
+        assert bool((buf == -7).all())
+
+
 @pytest.mark.parametrize("p", [1e-16, 1e-18, 5e-324])
 def test_probabilities_below_the_rounding_of_one(gpu, p):
     """1 - p rounds to 1: no edges, from either entry point."""
