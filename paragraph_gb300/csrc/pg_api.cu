@@ -2407,18 +2407,19 @@ pg_status pg_format_edges(pg_ctx* c, int32_t replica, const int64_t* ids, int64_
         }
     } t{c};
     PG_CUDA(c, talloc(t.did, n, c->device, c->stream));
-    PG_CUDA(c, talloc(t.len, std::max<int64_t>(m, 1), c->device, c->stream));
-    PG_CUDA(c, talloc(t.off, m + 1, c->device, c->stream));
-    PG_CUDA(c, talloc(t.bs, scan_blocks_needed(std::max<int64_t>(m, 1)) + 2, c->device, c->stream));
+    const int64_t tiles = text_tiles(m);
+    PG_CUDA(c, talloc(t.len, std::max<int64_t>(tiles, 1), c->device, c->stream));
+    PG_CUDA(c, talloc(t.off, tiles + 1, c->device, c->stream));
+    PG_CUDA(c, talloc(t.bs, scan_blocks_needed(std::max<int64_t>(tiles, 1)) + 2, c->device, c->stream));
     PG_CUDA(c, cudaMemcpyAsync(t.did.p, ids, 8 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
     const int64_t* fo = c->fwd_off.p + h.obase;
     const int32_t* fc = c->fwd_col.p + h.ebase;
     cudaGetLastError();
-    launch_text_len(fo, fc, n, m, t.did.p, t.len.p, c->num_sms, c->stream);
-    launch_scan_i32_to_i64(t.len.p, t.off.p, m, t.bs.p, c->stream);
+    launch_text(fo, fc, n, m, t.did.p, t.len.p, nullptr, nullptr, c->num_sms, c->stream);
+    launch_scan_i32_to_i64(t.len.p, t.off.p, tiles, t.bs.p, c->stream);
     PG_CUDA(c, cudaGetLastError());
     int64_t total = 0;
-    PG_CUDA(c, cudaMemcpyAsync(&total, t.off.p + m, 8, cudaMemcpyDeviceToHost, c->stream));
+    PG_CUDA(c, cudaMemcpyAsync(&total, t.off.p + tiles, 8, cudaMemcpyDeviceToHost, c->stream));
     PG_CUDA(c, cudaStreamSynchronize(c->stream));
     *bytes = total;
     if (!out) return PG_OK;
@@ -2426,7 +2427,7 @@ pg_status pg_format_edges(pg_ctx* c, int32_t replica, const int64_t* ids, int64_
         return fail(c, PG_ERR_CAPACITY, "the output buffer holds " + std::to_string(cap) + " bytes, the text needs " +
                                             std::to_string(total));
     PG_CUDA(c, talloc(t.txt, std::max<int64_t>(total, 1), c->device, c->stream));
-    launch_text_write(fo, fc, n, m, t.did.p, t.off.p, t.txt.p, c->num_sms, c->stream);
+    launch_text(fo, fc, n, m, t.did.p, nullptr, t.off.p, t.txt.p, c->num_sms, c->stream);
     PG_CUDA(c, cudaGetLastError());
     PG_CUDA(c, cudaMemcpyAsync(out, t.txt.p, (size_t)total, cudaMemcpyDeviceToHost, c->stream));
     PG_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -2467,9 +2468,10 @@ pg_status pg_format_attributes(pg_ctx* c, int32_t replica, const pg_attr_rows* r
     PG_CUDA(c, talloc(t.draws, 4 * n, c->device, c->stream));
     PG_CUDA(c, talloc(t.ints, 4 * n, c->device, c->stream));
     PG_CUDA(c, talloc(t.gen, 4 * n, c->device, c->stream));
-    PG_CUDA(c, talloc(t.len, n, c->device, c->stream));
-    PG_CUDA(c, talloc(t.off, n + 1, c->device, c->stream));
-    PG_CUDA(c, talloc(t.bs, scan_blocks_needed(std::max<int64_t>(n, 1)) + 2, c->device, c->stream));
+    const int64_t tiles = attr_tiles(n);
+    PG_CUDA(c, talloc(t.len, std::max<int64_t>(tiles, 1), c->device, c->stream));
+    PG_CUDA(c, talloc(t.off, tiles + 1, c->device, c->stream));
+    PG_CUDA(c, talloc(t.bs, scan_blocks_needed(std::max<int64_t>(tiles, 1)) + 2, c->device, c->stream));
     PG_CUDA(c, cudaMemcpyAsync(t.did.p, rows->ids, 8 * nn, cudaMemcpyHostToDevice, c->stream));
     PG_CUDA(c, cudaMemcpyAsync(t.draws.p, rows->draws, 32 * nn, cudaMemcpyHostToDevice, c->stream));
     PG_CUDA(c, cudaMemcpyAsync(t.ints.p, rows->ints, 16 * nn, cudaMemcpyHostToDevice, c->stream));
@@ -2492,10 +2494,10 @@ pg_status pg_format_attributes(pg_ctx* c, int32_t replica, const pg_attr_rows* r
     C.peak_int = rows->peak_integer ? 1 : 0;
     cudaGetLastError();
     launch_attr_text(C, t.len.p, nullptr, nullptr, c->num_sms, c->stream);
-    launch_scan_i32_to_i64(t.len.p, t.off.p, n, t.bs.p, c->stream);
+    launch_scan_i32_to_i64(t.len.p, t.off.p, tiles, t.bs.p, c->stream);
     PG_CUDA(c, cudaGetLastError());
     int64_t total = 0;
-    PG_CUDA(c, cudaMemcpyAsync(&total, t.off.p + n, 8, cudaMemcpyDeviceToHost, c->stream));
+    PG_CUDA(c, cudaMemcpyAsync(&total, t.off.p + tiles, 8, cudaMemcpyDeviceToHost, c->stream));
     PG_CUDA(c, cudaStreamSynchronize(c->stream));
     *bytes = total;
     if (!out) return PG_OK;

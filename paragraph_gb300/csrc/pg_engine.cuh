@@ -534,12 +534,11 @@ void launch_scan_i32_to_i64(const int32_t* in, int64_t* out, int64_t n, int64_t*
                             cudaStream_t s);
 int scan_blocks_needed(int64_t n);
 cudaError_t init_agent_kernels();
-// the edge list as text on the device (pg_text.cu)
-void launch_text_len(const int64_t* fo, const int32_t* fc, int64_t n, int64_t m, const int64_t* ids, int32_t* len,
-                     int num_sms, cudaStream_t s);
-void launch_text_write(const int64_t* fo, const int32_t* fc, int64_t n, int64_t m, const int64_t* ids,
-                       const int64_t* off, char* out, int num_sms, cudaStream_t s);
-// the attribute file as text on the device (pg_text.cu); out == nullptr: line lengths into len
+// the edge list as text on the device (pg_text.cu), a size per tile of lines; out == nullptr: the sizes into sums
+int64_t text_tiles(int64_t m);
+void launch_text(const int64_t* fo, const int32_t* fc, int64_t n, int64_t m, const int64_t* ids, int32_t* sums,
+                 const int64_t* off, char* out, int num_sms, cudaStream_t s);
+// the attribute file as text on the device (pg_text.cu); out == nullptr: the tiles' sizes into sums
 struct AttrCols {  // columns of the attribute file (device pointers)
     int64_t n, n_seed;
     const int64_t* ids;     // [n]
@@ -552,7 +551,8 @@ struct AttrCols {  // columns of the attribute file (device pointers)
     const int64_t* fo;      // forward offsets: the out-degree of v is fo[v + 1] - fo[v]
     int32_t peak_int;
 };
-void launch_attr_text(const AttrCols& C, int32_t* len, const int64_t* off, char* out, int num_sms,
+int64_t attr_tiles(int64_t n);
+void launch_attr_text(const AttrCols& C, int32_t* sums, const int64_t* off, char* out, int num_sms,
                       cudaStream_t s);
 // the source of every edge in [first, first + count) of a forward CSR, from its offsets
 void launch_edge_sources(const int64_t* fo, int64_t n, int64_t first, int64_t count, int32_t* out,

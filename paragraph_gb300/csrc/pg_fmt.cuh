@@ -2,13 +2,17 @@
 // and device (the attribute writer formats its floating-point columns on the GPU).
 //
 // Method (exact, no table of powers): for v = m 2^e (m a 53-bit integer) and a decimal exponent
-// guess k, the P significant digits are D = round_half_even(v 10^s), s = P - 1 - k.  A double
-// estimate of v 10^s is within one of the true value (its relative error is ~1e-15 and D < 2^34),
-// so D is decided among three neighbours by exact integer comparisons of v 10^s with D + 1/2:
+// guess k, the P significant digits are D = round_half_even(v 10^s), s = P - 1 - k.  For 0 <= s <= 19
+// and -117 <= e < 0 (the columns' usual values: 1e-10 to 1e9 at P = 10) m 10^s is a 117-bit integer,
+// and D and its rounding are read off its bits.  Otherwise a double estimate of v 10^s is within one
+// of the true value (its relative error is ~1e-15 and D < 2^34), so D is decided among three
+// neighbours by exact integer comparisons of v 10^s with D + 1/2:
 //   2 m 2^e 10^s  <=>  (2D + 1)   becomes   m 2^max(e+1,0) 10^max(s,0)  <=>  (2D + 1) 2^max(-e-1,0) 10^max(-s,0),
 // both sides multi-word integers (at most ~1170 bits for any finite double).  Equality is an exact
 // tie, resolved to the even D as the C library does in its default rounding mode.  If D reaches
 // 10^P the exponent guess was one low (and one high if D < 10^(P-1)); k is corrected and D redone.
+// The multi-word comparisons for every value, and FP64 estimates on a GPU with few FP64 units, were
+// most of an attribute file's time.
 // Then the %g rules: exponent X = k after rounding; fixed notation when -4 <= X < P, else
 // d.ddde+XX (at least two exponent digits); trailing zeros and a bare decimal point are dropped.
 #pragma once
@@ -91,6 +95,37 @@ PG_HD int cmp_half(uint64_t m, int e, int s, uint64_t D) {
     return big_cmp(L, R);
 }
 
+// 10^p for 0 <= p <= 19
+PG_HD uint64_t pow10_u64(int p) {
+    uint64_t r = (p & 1) ? 10u : 1u;
+    if (p & 2) r *= 100u;
+    if (p & 4) r *= 10000u;
+    if (p & 8) r *= 100000000u;
+    if (p & 16) r *= 10000000000000000ull;
+    return r;
+}
+
+// round_half_even(m 10^s 2^-sh) for m < 2^53, 0 <= s <= 19 and 0 < sh <= 117, all in integers.
+PG_HD uint64_t round_scaled_128(uint64_t m, int sh, int s) {
+    const uint64_t t = pow10_u64(s);
+    const uint64_t lo = m * t, hi = mulhi64(m, t);
+    uint64_t D, bit, rest;  // the quotient, the bit below it, and whether any is set below that
+    if (sh < 64) {
+        D = (hi << (64 - sh)) | (lo >> sh);
+        bit = (lo >> (sh - 1)) & 1u;
+        rest = lo & ((1ull << (sh - 1)) - 1u);
+    } else if (sh == 64) {
+        D = hi;
+        bit = lo >> 63;
+        rest = lo << 1;
+    } else {
+        D = hi >> (sh - 64);
+        bit = (hi >> (sh - 65)) & 1u;
+        rest = (hi & ((1ull << (sh - 65)) - 1u)) | lo;
+    }
+    return D + (bit & (uint64_t)(rest != 0u || (D & 1u)));
+}
+
 // round_half_even(v 10^s) for v = m 2^e, from an estimate within one of v 10^s
 PG_HD uint64_t round_scaled(uint64_t m, int e, int s, double est) {
     uint64_t D = est < 1.0 ? 0 : (uint64_t)est;  // floor of the estimate
@@ -151,21 +186,24 @@ PG_HD int fmt_g(double x, int prec, char* out) {
         e = be - 1075;
     }
     const double ax = neg ? -x : x;
-    // decimal exponent guess from the binary exponent (within one)
-    int msb = 63;
+    // decimal exponent guess from the binary exponent (within one): floor of 0.30103 b2 in integers
+    int msb = 52;
     while (!((m >> msb) & 1ull)) --msb;
     const int b2 = e + msb;  // 2^b2 <= ax < 2^(b2+1)
-    int k = (int)floor((double)b2 * 0.30102999566398120);
+    int k = (b2 * 78913) >> 18;
     uint64_t D = 0;
-    uint64_t lo = 1;
-    for (int i = 1; i < prec; ++i) lo *= 10u;
+    const uint64_t lo = pow10_u64(prec - 1);
     const uint64_t hi = lo * 10u;
     for (int it = 0; it < 4; ++it) {
         const int s = prec - 1 - k;
-        // v 10^s in double, scaled in two steps so neither factor overflows
-        const int s1 = s / 2, s2 = s - s1;
-        const double est = ax * pow10_dbl(s1) * pow10_dbl(s2);
-        D = round_scaled(m, e, s, est);
+        if (s >= 0 && s <= 19 && e < 0 && e >= -117) {
+            D = round_scaled_128(m, -e, s);
+        } else {
+            // v 10^s in double, scaled in two steps so neither factor overflows
+            const int s1 = s / 2, s2 = s - s1;
+            const double est = ax * pow10_dbl(s1) * pow10_dbl(s2);
+            D = round_scaled(m, e, s, est);
+        }
         if (D >= hi) {
             ++k;
             continue;
@@ -177,9 +215,11 @@ PG_HD int fmt_g(double x, int prec, char* out) {
         break;
     }
     char dg[20];
+    uint32_t low = (uint32_t)(D % 10000000u), high = (uint32_t)(D / 10000000u);  // D < 10^13
     for (int i = prec - 1; i >= 0; --i) {
-        dg[i] = (char)('0' + (int)(D % 10u));
-        D /= 10u;
+        if (prec - 1 - i == 7) low = high;
+        dg[i] = (char)('0' + (int)(low % 10u));
+        low /= 10u;
     }
     int nd = prec;  // significant digits after dropping trailing zeros
     while (nd > 1 && dg[nd - 1] == '0') --nd;

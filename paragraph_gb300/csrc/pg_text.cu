@@ -4,67 +4,163 @@
 // Restates Graph::WriteGraph (src/graph.cu:909-1003): one "source,target\n" line per edge, sources
 // in ascending sequence id, targets ascending within a source, both printed as the caller's
 // original ids.  The reference formats on the host threads with std::to_chars; here one pass
-// computes every line's length, the engine's scan turns lengths into offsets, and a second pass
-// writes the digits, so a 60M-edge graph becomes text in a few milliseconds and leaves the device
-// in one copy.
+// measures tiles of kTextTile lines, the engine's scan turns their sizes into offsets, and a second
+// pass formats every tile in shared memory and stores it whole, so a 60M-edge graph becomes text in a
+// few milliseconds and leaves the device in one copy.
 #include "pg_engine.cuh"
 #include "pg_fmt.cuh"
 
 namespace pg {
 
+__device__ __forceinline__ uint64_t magnitude(int64_t v) { return v < 0 ? (uint64_t)(-(v + 1)) + 1u : (uint64_t)v; }
+
 __device__ __forceinline__ int dec_len(int64_t v) {
-    uint64_t u = v < 0 ? (uint64_t)(-(v + 1)) + 1u : (uint64_t)v;
-    int n = v < 0 ? 1 : 0;
-    do {
-        ++n;
-        u /= 10u;
-    } while (u);
-    return n;
+    uint64_t u = magnitude(v);
+    int n = v < 0 ? 2 : 1;
+    for (; u >= 1000000000u; u /= 1000000000u) n += 9;  // 32 bits from here
+    const uint32_t w = (uint32_t)u;
+    return n + (w >= 10u) + (w >= 100u) + (w >= 1000u) + (w >= 10000u) + (w >= 100000u) + (w >= 1000000u) +
+           (w >= 10000000u) + (w >= 100000000u);
 }
 
 // writes the decimal text of v into p[0, len)
 __device__ __forceinline__ void dec_write(char* p, int64_t v, int len) {
-    uint64_t u = v < 0 ? (uint64_t)(-(v + 1)) + 1u : (uint64_t)v;
+    uint64_t u = magnitude(v);
     int i = len - 1;
+    for (; u >= 1000000000u; u /= 1000000000u) {
+        uint32_t w = (uint32_t)(u % 1000000000u);
+        for (int k = 0; k < 9; ++k) {
+            p[i--] = (char)('0' + (int)(w % 10u));
+            w /= 10u;
+        }
+    }
+    uint32_t w = (uint32_t)u;
     do {
-        p[i--] = (char)('0' + (int)(u % 10u));
-        u /= 10u;
-    } while (u);
+        p[i--] = (char)('0' + (int)(w % 10u));
+        w /= 10u;
+    } while (w);
     if (v < 0) p[0] = '-';
 }
 
-// source of edge e: the last row whose start is at or before e
-__device__ __forceinline__ int64_t edge_source(const int64_t* fo, int64_t n, int64_t e) {
-    int64_t lo = 0, hi = n - 1;
+// The CTA's staged text, stage[(dst & 15) ..) so that both sides are aligned alike, to dst: whole
+// 16-byte vectors, and bytes at the two ends (neighbouring tiles share those vectors).
+__device__ __forceinline__ void store_text(char* __restrict__ dst, const char* __restrict__ stage, int bytes) {
+    const int skew = (int)((uintptr_t)dst & 15u);
+    char* const base = dst - skew;
+    const int end = skew + bytes;
+    for (int v = threadIdx.x * 16; v < end; v += blockDim.x * 16) {
+        if (v >= skew && v + 16 <= end) {
+            *reinterpret_cast<int4*>(base + v) = *reinterpret_cast<const int4*>(stage + v);
+        } else {
+            for (int i = v < skew ? skew : v; i < v + 16 && i < end; ++i) base[i] = stage[i];
+        }
+    }
+}
+
+// Last row whose start is at or before e, found by the whole warp: 31 probes at a time cut the range
+// to a 32nd (a bisection's 17 dependent loads per edge were most of the pass).
+__device__ __forceinline__ int64_t warp_edge_source(const int64_t* __restrict__ fo, int64_t n, int64_t e) {
+    int64_t lo = 0, hi = n - 1;  // fo[lo] <= e, and the answer is at most hi
     while (lo < hi) {
-        const int64_t mid = (lo + hi + 1) >> 1;
-        if (fo[mid] <= e)
-            lo = mid;
-        else
-            hi = mid - 1;
+        const int64_t step = (hi - lo + 31) >> 5;
+        const int64_t at = lo + (int64_t)(lane_id() + 1) * step;
+        const int below = __popc(__ballot_sync(0xffffffffu, at <= hi && fo[at] <= e));
+        lo += (int64_t)below * step;
+        hi = lo + step - 1 < hi ? lo + step - 1 : hi;
     }
     return lo;
 }
 
-__global__ void __launch_bounds__(256) k_text_len(const int64_t* fo, const int32_t* fc, int64_t n, int64_t m,
-                                                  const int64_t* ids, int32_t* len) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t s = edge_source(fo, n, e);
-        len[e] = dec_len(ids[s]) + dec_len(ids[fc[e]]) + 2;
-    }
-}
+// A tile of kTextTile edges, kTextEdges consecutive ones per thread.  Their sources come from the tile's
+// own row starts: each row marks its first edge (the last of several rows that start at one edge, the
+// others being empty, is the source), and a running maximum carries the marks on.  The pass without an
+// output leaves the tile's bytes in `sums`, the writing pass places the tile at off[tile].  MEASURED_EDGES
+constexpr int kTextThreads = 256;
+constexpr int kTextEdges = 2;
+constexpr int kTextTile = kTextThreads * kTextEdges;
+constexpr int kLineMax = 42;  // two 64-bit ids of 20 characters, a comma and a newline
 
-__global__ void __launch_bounds__(256) k_text_write(const int64_t* fo, const int32_t* fc, int64_t n, int64_t m,
-                                                    const int64_t* ids, const int64_t* off, char* out) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t s = edge_source(fo, n, e);
-        const int64_t a = ids[s], b = ids[fc[e]];
-        const int la = dec_len(a), lb = dec_len(b);
-        char* p = out + off[e];
-        dec_write(p, a, la);
-        p[la] = ',';
-        dec_write(p + la + 1, b, lb);
-        p[la + 1 + lb] = '\n';
+template <bool WRITE>
+__global__ void __launch_bounds__(kTextThreads) k_text(const int64_t* __restrict__ fo, const int32_t* __restrict__ fc,
+                                                       int64_t n, int64_t m, const int64_t* __restrict__ ids,
+                                                       int32_t* __restrict__ sums, const int64_t* __restrict__ off,
+                                                       char* __restrict__ out) {
+    __shared__ int s_row[kTextTile];
+    __shared__ int s_scan[33];
+    __shared__ int64_t s_first;
+    __shared__ __align__(16) char stage[WRITE ? kTextTile * kLineMax + 16 : 16];
+    const int64_t tiles = (m + kTextTile - 1) / kTextTile;
+    const int lane = lane_id(), wid = threadIdx.x >> 5;
+    for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int64_t e0 = t * kTextTile;
+        const int64_t e1 = e0 + kTextTile < m ? e0 + kTextTile : m;
+        for (int i = threadIdx.x; i < kTextTile; i += kTextThreads) s_row[i] = 0;
+        if (wid == 0) {
+            const int64_t f = warp_edge_source(fo, n, e0);
+            if (lane == 0) s_first = f;
+        }
+        __syncthreads();
+        const int64_t first = s_first;
+        // rows after the first, until one starts past the tile
+        for (int64_t r0 = first + 1;; r0 += kTextThreads) {
+            const int64_t r = r0 + threadIdx.x;
+            const int64_t p = r < n ? fo[r] : e1;
+            if (p < e1) atomicMax(&s_row[p - e0], (int)(r - first));
+            if (__syncthreads_or(p >= e1)) break;
+        }
+        int row[kTextEdges], run = 0;
+#pragma unroll
+        for (int k = 0; k < kTextEdges; ++k) {
+            run = max(run, s_row[threadIdx.x * kTextEdges + k]);
+            row[k] = run;
+        }
+        int incl = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl = max(incl, y);
+        }
+        if (lane == 31) s_scan[wid] = incl;
+        int before = __shfl_up_sync(0xffffffffu, incl, 1);
+        if (lane == 0) before = 0;
+        __syncthreads();
+        for (int w = 0; w < wid; ++w) before = max(before, s_scan[w]);
+        __syncthreads();
+        int64_t a[kTextEdges], b[kTextEdges];
+        int la[kTextEdges], lb[kTextEdges], mine = 0;
+#pragma unroll
+        for (int k = 0; k < kTextEdges; ++k) {
+            const int64_t e = e0 + threadIdx.x * kTextEdges + k;
+            la[k] = lb[k] = 0;
+            if (e < e1) {
+                a[k] = ids[first + max(before, row[k])];
+                b[k] = ids[fc[e]];
+                la[k] = dec_len(a[k]);
+                lb[k] = dec_len(b[k]);
+                mine += la[k] + lb[k] + 2;
+            }
+        }
+        int total;
+        int at = block_excl_scan<int>(mine, s_scan, &total);
+        if constexpr (WRITE) {
+            char* const dst = out + off[t];
+            at += (int)((uintptr_t)dst & 15u);
+#pragma unroll
+            for (int k = 0; k < kTextEdges; ++k) {
+                if (la[k]) {
+                    dec_write(stage + at, a[k], la[k]);
+                    stage[at + la[k]] = ',';
+                    dec_write(stage + at + la[k] + 1, b[k], lb[k]);
+                    stage[at + la[k] + 1 + lb[k]] = '\n';
+                    at += la[k] + lb[k] + 2;
+                }
+            }
+            __syncthreads();
+            store_text(dst, stage, total);
+        } else if (threadIdx.x == 0) {
+            sums[t] = total;
+        }
+        __syncthreads();  // the next tile's
     }
 }
 
@@ -90,22 +186,19 @@ void launch_edge_sources(const int64_t* fo, int64_t n, int64_t first, int64_t co
     k_edge_sources<<<(unsigned)g, 256, 0, s>>>(fo, n, first, count, out);
 }
 
-void launch_text_len(const int64_t* fo, const int32_t* fc, int64_t n, int64_t m, const int64_t* ids, int32_t* len,
-                     int num_sms, cudaStream_t s) {
-    if (m <= 0) return;
-    int64_t g = (m + 255) / 256;
-    if (g > (int64_t)num_sms * 16) g = (int64_t)num_sms * 16;
-    k_text_len<<<(unsigned)g, 256, 0, s>>>(fo, fc, n, m, ids, len);
-}
+int64_t text_tiles(int64_t m) { return (m + kTextTile - 1) / kTextTile; }
 
-void launch_text_write(const int64_t* fo, const int32_t* fc, int64_t n, int64_t m, const int64_t* ids,
-                       const int64_t* off, char* out, int num_sms, cudaStream_t s) {
+// out == nullptr: the tiles' bytes into sums
+void launch_text(const int64_t* fo, const int32_t* fc, int64_t n, int64_t m, const int64_t* ids, int32_t* sums,
+                 const int64_t* off, char* out, int num_sms, cudaStream_t s) {
     if (m <= 0) return;
-    int64_t g = (m + 255) / 256;
-    if (g > (int64_t)num_sms * 16) g = (int64_t)num_sms * 16;
-    k_text_write<<<(unsigned)g, 256, 0, s>>>(fo, fc, n, m, ids, off, out);
+    int64_t g = text_tiles(m);
+    if (g > (int64_t)num_sms * 8) g = (int64_t)num_sms * 8;
+    if (out)
+        k_text<true><<<(unsigned)g, kTextThreads, 0, s>>>(fo, fc, n, m, ids, sums, off, out);
+    else
+        k_text<false><<<(unsigned)g, kTextThreads, 0, s>>>(fo, fc, n, m, ids, sums, off, out);
 }
-
 
 // ---------------------------------------------------------------- the attribute file
 // Restates Graph::WriteAttributes (src/graph.cu:1057-1218): one line per node,
@@ -114,98 +207,126 @@ void launch_text_write(const int64_t* fo, const int32_t* fc, int64_t n, int64_t 
 // with the weights and alpha as "%.10g", the peak as "%d" (refcompat's integer peak) or "%.9g" of
 // the fp32 fitness, seeds typed "seed" with "no_generators", agents typed "agent" with their
 // generator ids joined by ';' ("-1" when there is none).  Year, fitness and degrees come from the
-// arena; the per-paper draws, printed ids and generators from the caller.  Pass 1 measures every
-// line (no output buffer), the scan places them, pass 2 writes them.
+// arena; the per-paper draws, printed ids and generators from the caller.  Pass 1 measures tiles of
+// kAttrNodes lines (no output buffer), the scan places them, pass 2 formats and stores them.
 
-struct LineOut {
-    char* p;  // null: count only
+
+// Eight lanes per line, a field or a run of integer fields each, so that a line waits for one "%g" and
+// not for five in a row: fewer nodes than threads fit the GPU, and the conversions' chains are what the
+// pass waits for.  Each lane's text goes to its own shared-memory slot, a scan over the CTA places the
+// slots, and the tile is stored whole.  MEASURED_ATTR
+constexpr int kAttrThreads = 256;
+constexpr int kAttrLanes = 8;
+constexpr int kAttrNodes = kAttrThreads / kAttrLanes;
+constexpr int kFieldMax = 92;  // a lane's text: at most four 64-bit generator ids (84); an odd number of words
+constexpr int kAttrLineMax = 320;  // 38 + 4 x 18 + 42 + 56 + 85, and slack
+
+struct FieldOut {
+    char* p;
     int n;
-    __device__ __forceinline__ void put(char c) {
-        if (p) p[n] = c;
-        ++n;
-    }
+    __device__ __forceinline__ void put(char c) { p[n++] = c; }
     __device__ __forceinline__ void str(const char* s) {
         while (*s) put(*s++);
     }
     __device__ __forceinline__ void dec(int64_t v) {
         const int l = dec_len(v);
-        if (p) dec_write(p + n, v, l);
+        dec_write(p + n, v, l);
         n += l;
-    }
-    __device__ __forceinline__ void g(double x, int prec) {
-        char b[32];
-        const int l = fmt_g(x, prec, b);
-        for (int i = 0; i < l; ++i) put(b[i]);
     }
 };
 
-__device__ int attr_line(const AttrCols& C, int64_t v, char* p) {
-    LineOut o{p, 0};
+// part j of node v's line into p; returns its length
+__device__ __forceinline__ int attr_part(const AttrCols& C, int64_t v, int j, char* p) {
+    FieldOut o{p, 0};
     const bool seed = v < C.n_seed;
-    const double* d = C.draws + v * 4;
     const int32_t* q = C.ints + v * 4;
-    o.dec(C.ids[v]);
-    o.str(seed ? ",seed," : ",agent,");
-    o.dec(C.pub[v]);
-    for (int i = 0; i < 3; ++i) {
+    // integers before the lane's "%g"
+    if (j == 0) {
+        o.dec(C.ids[v]);
+        o.str(seed ? ",seed," : ",agent,");
+        o.dec(C.pub[v]);
+    } else if (j == 4) {
         o.put(',');
-        o.g(d[i], 10);
+        o.dec(q[0]);
     }
-    o.put(',');
-    o.dec(q[0]);
-    o.put(',');
-    if (C.peak_int)
-        o.dec((int64_t)(int32_t)C.fit[v]);
-    else
-        o.g((double)C.fit[v], 9);
-    o.put(',');
-    o.dec(q[1]);
-    o.put(',');
-    o.g(d[3], 10);
-    o.put(',');
-    o.dec(C.indeg[v]);
-    o.put(',');
-    o.dec(C.fo[v + 1] - C.fo[v]);
-    o.put(',');
-    o.dec(q[2]);
-    o.put(',');
-    o.dec(q[3]);
-    o.put(',');
-    if (seed) {
-        o.str("no_generators");
-    } else {
-        int k = 0;
-        for (int i = 0; i < 4; ++i) {
-            const int64_t gid = C.gens[v * 4 + i];
-            if (gid < 0) continue;
-            if (k++) o.put(';');
-            o.dec(gid);
+    // 1..3: the three weights, 4: the peak, 5: alpha
+    if (j >= 1 && j <= 5) {
+        o.put(',');
+        if (j == 4 && C.peak_int) {
+            o.dec((int64_t)(int32_t)C.fit[v]);
+        } else {
+            const double x = j == 4 ? (double)C.fit[v] : C.draws[v * 4 + (j == 5 ? 3 : j - 1)];
+            o.n += fmt_g(x, j == 4 ? 9 : 10, o.p + o.n);
         }
-        if (!k) o.str("-1");
     }
-    o.put('\n');
+    if (j == 4) {
+        o.put(',');
+        o.dec(q[1]);
+    } else if (j == 6) {
+        o.put(',');
+        o.dec(C.indeg[v]);
+        o.put(',');
+        o.dec(C.fo[v + 1] - C.fo[v]);
+        o.put(',');
+        o.dec(q[2]);
+        o.put(',');
+        o.dec(q[3]);
+    } else if (j == 7) {
+        o.put(',');
+        if (seed) {
+            o.str("no_generators");
+        } else {
+            int k = 0;
+            for (int i = 0; i < 4; ++i) {
+                const int64_t gid = C.gens[v * 4 + i];
+                if (gid < 0) continue;
+                if (k++) o.put(';');
+                o.dec(gid);
+            }
+            if (!k) o.str("-1");
+        }
+        o.put('\n');
+    }
     return o.n;
 }
 
-__global__ void __launch_bounds__(128) k_attr_len(AttrCols C, int32_t* len) {
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < C.n; v += (int64_t)gridDim.x * blockDim.x)
-        len[v] = attr_line(C, v, nullptr);
+template <bool WRITE>
+__global__ void __launch_bounds__(kAttrThreads) k_attr(AttrCols C, int32_t* __restrict__ sums,
+                                                       const int64_t* __restrict__ off, char* __restrict__ out) {
+    __shared__ char s_part[kAttrThreads * kFieldMax];
+    __shared__ int s_scan[33];
+    __shared__ __align__(16) char stage[WRITE ? kAttrNodes * kAttrLineMax + 16 : 16];
+    const int64_t tiles = (C.n + kAttrNodes - 1) / kAttrNodes;
+    char* const part = s_part + threadIdx.x * kFieldMax;
+    for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int64_t v = t * kAttrNodes + threadIdx.x / kAttrLanes;
+        const int l = v < C.n ? attr_part(C, v, threadIdx.x % kAttrLanes, part) : 0;
+        int total;
+        int at = block_excl_scan<int>(l, s_scan, &total);
+        if constexpr (WRITE) {
+            char* const dst = out + off[t];
+            at += (int)((uintptr_t)dst & 15u);
+            for (int i = 0; i < l; ++i) stage[at + i] = part[i];
+            __syncthreads();
+            store_text(dst, stage, total);
+        } else if (threadIdx.x == 0) {
+            sums[t] = total;
+        }
+        __syncthreads();  // the next tile's
+    }
 }
 
-__global__ void __launch_bounds__(128) k_attr_write(AttrCols C, const int64_t* off, char* out) {
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < C.n; v += (int64_t)gridDim.x * blockDim.x)
-        attr_line(C, v, out + off[v]);
-}
+int64_t attr_tiles(int64_t n) { return (n + kAttrNodes - 1) / kAttrNodes; }
 
-void launch_attr_text(const AttrCols& C, int32_t* len, const int64_t* off, char* out, int num_sms,
+void launch_attr_text(const AttrCols& C, int32_t* sums, const int64_t* off, char* out, int num_sms,
                       cudaStream_t s) {
     if (C.n <= 0) return;
-    int64_t g = (C.n + 127) / 128;
+    int64_t g = attr_tiles(C.n);
     if (g > (int64_t)num_sms * 16) g = (int64_t)num_sms * 16;
     if (out)
-        k_attr_write<<<(unsigned)g, 128, 0, s>>>(C, off, out);
+        k_attr<true><<<(unsigned)g, kAttrThreads, 0, s>>>(C, sums, off, out);
     else
-        k_attr_len<<<(unsigned)g, 128, 0, s>>>(C, len);
+        k_attr<false><<<(unsigned)g, kAttrThreads, 0, s>>>(C, sums, off, out);
 }
 
 }  // namespace pg

@@ -66,3 +66,16 @@ def test_nan_prints_like_the_c_library(fmt):
     nan = struct.unpack("<d", struct.pack("<Q", 0x7FF8000000000000))[0]
     neg_nan = struct.unpack("<d", struct.pack("<Q", 0xFFF8000000000000))[0]
     assert fmt(nan, 10) == "nan" and fmt(neg_nan, 10) == "-nan"
+
+
+@pytest.mark.parametrize("prec", [1, 9, 10, 13])
+def test_halves_at_every_scale(fmt, prec):
+    """Ties and their neighbours at each power of ten around the 117-bit range and past both its ends."""
+    rng = np.random.default_rng(prec)
+    vals = []
+    for s in range(-3, 24):
+        for d in rng.integers(10 ** (prec - 1), 10 ** prec, 40):
+            v = float(f"{d}.5e{-s}")
+            vals += [v, np.nextafter(v, 0.0), np.nextafter(v, np.inf), -v]
+    vals += [np.ldexp(1.0 + i / 8, -e) for e in range(45, 70) for i in range(8)]
+    _check(fmt, [float(v) for v in vals], prec)

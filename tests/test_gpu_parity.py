@@ -682,3 +682,49 @@ def test_appended_rows_of_every_sort_class(gpu, deg):
                 seen |= {int(c) for c in np.searchsorted([2, 9, 33, 65, 129, 257], new, side="right")}
     assert {1, 2} <= seen or deg > 8.0
     assert seen >= {4, 5, 6} or deg < 8.0
+
+
+@pytest.mark.parametrize("m", [0, 1, 511, 512, 513, 2048, 5003])
+def test_edge_text_at_tile_edges(gpu, m):
+    """Sources with long rows, runs of rows without citations, ids of every length."""
+    rng = np.random.default_rng(m)
+    n = 6000
+    src = np.sort(rng.choice(np.array([700, 701, 1500, 4000, 4001, 4002, 5999]), m)) if m else np.zeros(0, np.int64)
+    pairs = np.unique(np.stack([src, rng.integers(0, 690, m)], 1), axis=0) if m else np.zeros((0, 2), np.int64)
+    k = 0
+    while len(pairs) < m:  # exactly m distinct edges
+        pairs = np.unique(np.concatenate([pairs, [[5000 + k // 600, k % 600]]]), axis=0)
+        k += 1
+    ids = (rng.integers(0, 1 << 62, n) >> rng.integers(0, 62, n)) * rng.choice([1, -1], n)
+    ids[:4] = [0, -(1 << 63), (1 << 63) - 1, 10**9]
+    with GrowthEngine(seed=4) as eng:
+        eng.load_graph(np.full(n, -1, np.int32), np.ones(n, np.float32), pairs[:, 0].astype(np.int32),
+                       pairs[:, 1].astype(np.int32), PAParams(fixed_new_nodes=10), planned_epochs=1)
+        assert eng.counts() == (n, m)
+        txt = eng.format_edges(ids)
+    assert txt == "".join(f"{ids[s]},{ids[d]}\n" for s, d in pairs).encode()
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 1000])
+def test_attribute_text_at_tile_edges(gpu, n):
+    """Whole tiles and remainders; ties, extremes and short values of every column."""
+    rng = np.random.default_rng(n)
+    n0 = n // 2
+    ids = (rng.integers(0, 1 << 62, n) >> rng.integers(0, 62, n)) * rng.choice([1, -1], n)
+    ids[0] = -(1 << 63)
+    vals = np.array([0.0, -0.0, 1.0, 0.5, 1234567890.5, 1234567891.5, 12345678905e-1, 5e-324, -1.7976931348623157e308,
+                     2.2250738585072014e-308, 9999999999.5, 99999999995e-5, 1e10, 1e-5, 123456.7890625, 0.1])
+    draws = rng.choice(vals, (n, 4))
+    ints = rng.choice(np.array([-(1 << 31), -1, 0, 7, (1 << 31) - 1]), (n, 4)).astype(np.int32)
+    gens = rng.choice(np.array([-1, 0, 99, (1 << 63) - 1]), (n, 4))
+    fit = rng.choice(np.array([1.0, 1e-30, 0.1, 123456.79, 3e38]), n).astype(np.float32)
+    with GrowthEngine(seed=4) as eng:
+        eng.load_graph(np.full(n, -1, np.int32), fit, np.zeros(0, np.int32), np.zeros(0, np.int32))
+        txt = eng.format_attributes(ids, draws, ints, gens, n0, False).decode()
+    lines = []
+    for v in range(n):
+        gen = "no_generators" if v < n0 else (";".join(str(x) for x in gens[v] if x >= 0) or "-1")
+        lines.append("%d,%s,%d,%.10g,%.10g,%.10g,%d,%.9g,%d,%.10g,%d,%d,%d,%d,%s\n" % (
+            ids[v], "seed" if v < n0 else "agent", -1, draws[v, 0], draws[v, 1], draws[v, 2], ints[v, 0],
+            float(fit[v]), ints[v, 1], draws[v, 3], 0, 0, ints[v, 2], ints[v, 3], gen))
+    assert txt == "".join(lines)
