@@ -650,8 +650,9 @@ __device__ __forceinline__ void d_edges_check(const Arena& A, int64_t agents) {
 __global__ void k_edges_check(Arena A, int64_t agents) { d_edges_check(A, agents); }
 
 // Shapes of the k <= 64 thinning kernel (pg_tuning.small_hash = HS): 0 -- a 2048-slot frontier hash
-// and 512-entry stage buffers; 1 -- 1024 slots and 1024-entry stages; both 4 CTAs per SM.  The
-// k <= 256 kernel always has 1024 slots and 512-entry stages.  Shapes with more resident warps were
+// (the lean instance: 1024 slots and a filter of 1024 words) and 512-entry stage buffers; 1 -- 1024
+// slots, a filter of 256 words and 1024-entry stages; both 4 CTAs per SM.  The k <= 256 kernel always
+// has 1024 slots, 256 filter words and 512-entry stages.  Shapes with more resident warps were
 // measured on the PA workload and were slower: 1024 slots and 512-entry stages at 5 CTAs per SM (96
 // registers) by 9 %, and 2048 slots and 256-entry stages at 5 CTAs per SM with the heavy agents'
 // instance out of line (the lean one then fits 96 registers) by 8 %.

@@ -465,6 +465,31 @@ __device__ __forceinline__ int replica_of_agent(const Replica* rep, int R, int64
     }
     return lo;
 }
+
+// Searches by a whole warp (all lanes, the same arguments and result): 32 probes cut the range to a
+// 32nd, where a bisection's probes are loads that wait for one another.  `below(i)` holds for a prefix
+// of [0, n) that includes 0; the result is its last index.
+template <typename Below>
+__device__ __forceinline__ int64_t warp_last_below(int64_t n, Below below) {
+    int64_t lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int64_t step = (hi - lo + 31) >> 5;
+        const int64_t at = lo + (int64_t)(lane_id() + 1) * step;
+        const int c = __popc(__ballot_sync(0xffffffffu, at <= hi && below(at)));
+        lo += (int64_t)c * step;
+        hi = lo + step - 1 < hi ? lo + step - 1 : hi;
+    }
+    return lo;
+}
+__device__ __forceinline__ int warp_replica_of_agent(const Replica* rep, int R, int64_t a) {
+    return (int)warp_last_below(R, [&](int64_t r) { return rep[r].abase <= a; });
+}
+// The replica of an agent at or a little after one of replica r: a warp's or tile's agents seldom cross
+// replicas.
+__device__ __forceinline__ int advance_replica(const Replica* rep, int R, int r, int64_t a) {
+    while (r + 1 < R && rep[r + 1].abase <= a) ++r;
+    return r;
+}
 #endif
 
 // ---------------------------------------------------------------- host launchers

@@ -36,7 +36,9 @@ struct BallAux {
 };
 
 constexpr uint32_t kWaitLimit = kWaitPolls;  // polls of a bulk-copy barrier before giving up
-constexpr int kTestU = 4;                  // entries per lane and step of the membership scan
+constexpr uint32_t kHashMul = 0x9E3779B1u;
+constexpr int kFilterWords = 256;
+constexpr int kTestU = 8;                  // entries per lane and step of the membership scan
 
 // STAGE: adjacency entries per stage buffer (two per warp); the struct lives in dynamic shared
 // memory, one per warp.  The exact continuation's lists (chosen ids and their cumulative quantised
@@ -47,9 +49,11 @@ struct ThinSmem {
     static_assert(2 * STAGE * 4 >= KCAP * 12, "continuation lists must fit the stage buffers");
     __align__(16) int32_t stage[2][STAGE];  // candidate rows, two buffers filled by bulk copies
     int32_t H[HCAP];  // frontier hash set, -1 = empty
+    uint32_t F[kFilterWords];  // filter in front of it
     int32_t arr[KCAP];
     BallAux aux;
     unsigned long long bar[2];  // mbarriers of the two stage buffers
+    static_assert(STAGE % (32 * kTestU) == 0, "a step stays inside its buffer");
     __device__ int32_t* c_id() { return &stage[0][0]; }
     __device__ uint64_t* c_cq() { return reinterpret_cast<uint64_t*>(&stage[0][0] + 2 * KCAP); }
 };
@@ -137,7 +141,26 @@ __device__ __forceinline__ bool contains(const int32_t* a, int64_t lo, int64_t h
 // bucket.  With no deletions a bucket always fills as a prefix, so a lookup reads a whole bucket
 // with one 16-byte load and stops at the first bucket whose last slot is free.
 __device__ __forceinline__ uint32_t hslot_of(int32_t v, int bits) {
-    return (((uint32_t)v * 0x9E3779B1u) >> (34 - bits)) << 2;
+    return (((uint32_t)v * kHashMul) >> (34 - bits)) << 2;
+}
+
+// A blocked Bloom filter in front of the shared hash set: two bits of one 32-bit word per entry, 150
+// entries of a usual frontier in 256 words.  Nearly all of the entries a membership scan looks at are
+// not in the frontier, and the filter says so from one 4-byte load (about 4 bank passes for a warp's
+// random words) where the set's bucket takes 16 bytes (about 11); what passes it is looked up in the
+// set.  The agent kernel is bound by instruction issue and by the latency of its short chains at 16
+// warps per SM, and the scan is its largest part (1,535 of a warp's cycles per 512 entries with it).
+// PA at scale, 30 epochs: 37.7 ms of agent kernels without the filter, 33.1 with 256 words, 31.9 with
+// 1,024, and 31.7 with hits taken in any order; 256 replicas x 10 epochs: 67.1, 61.7, 60.1 and 56.5 ms.
+template <int BITS>
+__device__ __forceinline__ bool filter_may_have(const uint32_t* F, uint32_t h) {
+    const uint32_t w = F[h >> (32 - BITS)];
+    return ((w >> (h & 31u)) & (w >> ((h >> 5) & 31u)) & 1u) != 0u;
+}
+template <int BITS>
+__device__ __forceinline__ void filter_insert(uint32_t* F, int32_t v) {
+    const uint32_t h = (uint32_t)v * kHashMul;
+    atomicOr(&F[h >> (32 - BITS)], (1u << (h & 31u)) | (1u << ((h >> 5) & 31u)));
 }
 
 // Insert v into the shared hash set (any lane, concurrently).
@@ -271,6 +294,16 @@ __device__ bool member_warp(const Ball& B, int32_t j, long long& examined) {
     return member_rows_warp(B, j, examined);
 }
 
+// positions in an agent's anchor rows: the lean instance has at most 512
+template <bool GENERAL>
+struct FrontierPos {
+    using type = int64_t;
+};
+template <>
+struct FrontierPos<false> {
+    using type = int;
+};
+
 // Returns false when a bounded wait ran out (the error word is set and the warp must stop).
 // GENERAL = false is the lean instance for the agents the setup did not list as heavy: no hub
 // anchor and anchor rows within the shared frontier, so membership in Z is the frontier hash alone.
@@ -278,11 +311,17 @@ template <int KCAP, int HCAP, int STAGE, bool GENERAL>
 __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KCAP, HCAP, STAGE>& S,
                                    uint32_t& phase) {
     constexpr int kStage = STAGE;
-    constexpr int kHBits = HCAP == 4096 ? 12 : (HCAP == 2048 ? 11 : 10);
-    static_assert(HCAP == (1 << kHBits), "hash capacity must be 1024, 2048 or 4096");
-    constexpr int ZCAP = HCAP / 2;  // entries gathered into the frontier (with repeats)
+    // The lean instance's frontiers have at most 512 entries: where the set has 2048 slots it uses half
+    // of them and lays a filter of 1024 words over the other half.
+    constexpr bool kHalf = !GENERAL && HCAP == 2048;
+    constexpr int kSlots = kHalf ? HCAP / 2 : HCAP;
+    constexpr int kHBits = kSlots == 2048 ? 11 : 10;
+    constexpr int kFBits = kHalf ? 10 : 8;
+    static_assert(kSlots == (1 << kHBits) && kFilterWords == 256, "set and filter sizes");
+    constexpr int ZCAP = kSlots / 2;  // entries gathered into the frontier (with repeats)
+    uint32_t* const F = kHalf ? reinterpret_cast<uint32_t*>(S.H + kSlots) : S.F;
     const int lane = lane_id();
-    const int r = replica_of_agent(A.rep, A.R, a);
+    const int r = warp_replica_of_agent(A.rep, A.R, a);
     const Replica& rp = A.rep[r];
     const int64_t n = rp.n;
     const int64_t al = a - rp.abase;
@@ -315,7 +354,8 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
     for (int w = 0; w < kMaskWords; ++w) ha.w[w] = 0ull;
     const int na = boost ? rp.anchors : 0;
     if (boost) {
-        for (int q = lane; q < HCAP; q += 32) S.H[q] = -1;
+        for (int q = lane; q < kSlots / 4; q += 32) reinterpret_cast<int4*>(S.H)[q] = make_int4(-1, -1, -1, -1);
+        for (int q = lane; q < (1 << kFBits) / 4; q += 32) reinterpret_cast<int4*>(F)[q] = make_int4(0, 0, 0, 0);
         const u32x4 xa = draw(A.seed, kStreamAnchor, rep, ep, unit, 0);
         auto anchor = [&](int i) -> int {
             const uint32_t w = i == 0 ? xa.x[0] : (i == 1 ? xa.x[1] : (i == 2 ? xa.x[2] : xa.x[3]));
@@ -410,41 +450,45 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
         if (lane < na) {
             const int x = anchor(lane & 3);
             hash_insert(S.H, kHBits, x);
+            filter_insert<kFBits>(F, x);
             add_mask(x);
         }
         // the non-hub anchors' rows, flat: entry p belongs to the last row lane whose exclusive
         // offset is at or below p (the rows are laid out in lane order)
         const bool row_in = has_row && r_hs < 0;
-        const int64_t len_in = row_in ? r_len : 0;
-        const int64_t incl = warp_incl_scan(len_in);
-        const int64_t excl = incl - len_in;
-        const int64_t T = __shfl_sync(kFull, incl, 31);
+        using Pos = typename FrontierPos<GENERAL>::type;
+        const Pos len_in = row_in ? (Pos)r_len : 0;
+        const Pos incl = warp_incl_scan<Pos>(len_in);
+        const Pos excl = incl - len_in;
+        const Pos T = __shfl_sync(kFull, incl, 31);
         // 1: into H; 2: into the global table; 0: neither (hub masks only)
         const int into = row_in ? (!((bigm >> rl) & 1u) ? 1 : (G ? 2 : 0)) : 0;
-        for (int64_t p0 = 0; p0 < T; p0 += 64) {
+        for (Pos p0 = 0; p0 < T; p0 += 64) {
             int32_t v[2];
             int ih[2];
             bool ok[2];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                const int64_t p = p0 + 32 * u + lane;
+                const Pos p = p0 + 32 * u + lane;
                 int L = 0;
 #pragma unroll
                 for (int bb = 4; bb >= 1; bb >>= 1)
                     if (__shfl_sync(kFull, excl, L + bb) <= p) L += bb;
-                const int64_t st = __shfl_sync(kFull, r_st, L), e0 = __shfl_sync(kFull, excl, L);
-                ih[u] = __shfl_sync(kFull, into, L);
+                const int64_t st = __shfl_sync(kFull, r_st - excl, L);
+                ih[u] = GENERAL ? __shfl_sync(kFull, into, L) : 1;
                 ok[u] = p < T;
                 // streaming load: the anchor rows are read once per agent
-                v[u] = ok[u] ? __ldcs(&((L & 1) ? B.bc : B.fc)[st + (p - e0)]) : 0;
+                v[u] = ok[u] ? __ldcs(&((L & 1) ? B.bc : B.fc)[st + p]) : 0;
             }
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 if (!ok[u]) continue;
-                if (ih[u] == 1)
+                if (ih[u] == 1) {
                     hash_insert(S.H, kHBits, v[u]);
-                else if (GENERAL && ih[u] == 2)
+                    filter_insert<kFBits>(F, v[u]);
+                } else if (GENERAL && ih[u] == 2) {
                     ghash_insert(G, v[u]);
+                }
                 add_mask(v[u]);
             }
         }
@@ -556,35 +600,39 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
         const int64_t wx = wincl - W;
         const int64_t DW = __shfl_sync(kFull, wincl, 31);
         int64_t mp = d;  // first-hit position of this lane's node (d: none yet)
-        // this lane's part of chunk c0 (empty once its row has a hit)
-        auto part = [&](int64_t c0, int64_t& s0, int64_t& s1) {
-            const int64_t c1 = c0 + kStage < DW ? c0 + kStage : DW;
-            s0 = wx > c0 ? wx : c0;
-            s1 = wx + W < c1 ? wx + W : c1;
-            if (mp < d || s1 < s0) s1 = s0;
+        // this lane's window in the coordinates of chunk c0, cut to -1 and kStage
+        auto window = [&](int64_t c0, int& w0, int& w1) {
+            const int64_t a0 = wx - c0, a1 = a0 + W;
+            w0 = (int)(a0 < -1 ? -1 : (a0 > kStage ? kStage : a0));
+            w1 = (int)(a1 < -1 ? -1 : (a1 > kStage ? kStage : a1));
         };
-        // issue the bulk copies of chunk c0 into buffer `buf`; false when nothing is copied
-        auto issue = [&](int64_t c0, int buf) -> bool {
-            int64_t s0, s1;
-            part(c0, s0, s1);
-            const uint32_t total = __reduce_add_sync(kFull, (uint32_t)(s1 - s0) * 4u);
+        // issue the bulk copies of chunk c0 into buffer `buf` (a lane's part is empty once its row has
+        // a hit); false when nothing is copied
+        auto issue = [&](int64_t c0, int buf, int& w0, int& w1) -> bool {
+            window(c0, w0, w1);
+            const int s0 = w0 > 0 ? w0 : 0;
+            const int len = mp < d || w1 < s0 ? 0 : w1 - s0;
+            const uint32_t total = __reduce_add_sync(kFull, (uint32_t)len * 4u);
             if (total == 0) return false;
             // the warp's reads of this buffer have completed (their values fed its ballots)
             __syncwarp();
             if (lane == 0) mbar_expect_tx(&S.bar[buf], total);
             __syncwarp();
-            if (s1 > s0) bulk_g2s(&S.stage[buf][s0 - c0], wsrc + (s0 - wx), (uint32_t)(s1 - s0) * 4u, &S.bar[buf]);
+            if (len) bulk_g2s(&S.stage[buf][s0], wsrc + (c0 + s0 - wx), (uint32_t)len * 4u, &S.bar[buf]);
             return true;
         };
         // chunks are double-buffered: chunk c+1 is in flight while chunk c is tested
         const bool simple = !GENERAL || (B.small && !B.any_ha);  // membership in Z: the hash alone
         const int64_t nchunk = (DW + kStage - 1) / kStage;
         uint32_t armed = 0;  // bit b: buffer b has copies in flight
-        if (nchunk > 0 && issue(0, 0)) armed = 1u;
+        int wlo, whi, wlo1 = 0, whi1 = 0;  // this lane's window in the current chunk and the next one
+        if (nchunk > 0 && issue(0, 0, wlo1, whi1)) armed = 1u;
         for (int64_t c = 0; c < nchunk; ++c) {
             const int buf = (int)(c & 1);
             const int64_t c0 = c * kStage;
-            if (c + 1 < nchunk && issue(c0 + kStage, buf ^ 1)) armed |= 2u >> buf;
+            wlo = wlo1;
+            whi = whi1;
+            if (c + 1 < nchunk && issue(c0 + kStage, buf ^ 1, wlo1, whi1)) armed |= 2u >> buf;
             if (!((armed >> buf) & 1u)) continue;
             armed &= ~(1u << buf);
             const bool ok = mbar_wait(&S.bar[buf], (phase >> buf) & 1u, A.first_wait_polls);
@@ -599,70 +647,40 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
             }
             const int32_t* stg = S.stage[buf];
             // The chunk is tested flat, kTestU entries per lane and step, whatever row they belong
-            // to; a hit is then given to the lane whose window holds it, which keeps it when its
-            // row has no hit yet and the entry is the row's own (not window padding).  Entries of
+            // to; a hit is then given to the lane whose window holds it, which keeps the row's first
+            // one, if the entry is the row's own (not window padding).  Entries of
             // a row whose hit came in an earlier chunk (copied before the hit was known) or of a
             // row not copied at all (stale) are tested too and their hits dropped.  Chunk
             // position q maps to row position q + x0 (forward row first, then backward).
             const int nq = (int)(DW - c0 < kStage ? DW - c0 : kStage);
+            const int x0 = (int)((c0 - wx) - lead);
+            const int d32 = (int)d;
             for (int i0 = 0; i0 < nq; i0 += 32 * kTestU) {
-                bool hit[kTestU];
-                if (simple) {
-                    // the entries' first buckets are read together; a full bucket without
-                    // the entry (rare at the frontier's load) continues the probe
-                    int32_t v[kTestU];
-                    int4 hb[kTestU];
-#pragma unroll
-                    for (int u = 0; u < kTestU; ++u) {
-                        const int q = i0 + 32 * u + lane;
-                        v[u] = stg[q];  // q < kStage: past nq the entry is stale and masked below
-                        hb[u] = *reinterpret_cast<const int4*>(S.H + hslot_of(v[u], kHBits));
-                    }
-                    bool more[kTestU], anymore = false;
-#pragma unroll
-                    for (int u = 0; u < kTestU; ++u) {
-                        const bool in = i0 + 32 * u + lane < nq;
-                        hit[u] = in && bucket_has(hb[u], v[u]);
-                        more[u] = in && !hit[u] && hb[u].w != -1;
-                        anymore |= more[u];
-                    }
-                    if (__any_sync(kFull, anymore)) {
-#pragma unroll
-                        for (int u = 0; u < kTestU; ++u)
-                            if (more[u]) hit[u] = hash_contains(S.H, kHBits, v[u]);
-                    }
-                } else {
-#pragma unroll
-                    for (int u = 0; u < kTestU; ++u) {
-                        const int q = i0 + 32 * u + lane;
-                        hit[u] = false;
-                        if (q < nq) {  // stale entries may hold any value: only node ids reach the masks
-                            const int32_t v = stg[q];
-                            hit[u] = (uint32_t)v < (uint32_t)n && in_z(B, v);
-                        }
-                    }
-                }
-                // hits are rare: one vote skips the per-entry ballots of a step without any
-                bool anyhit = false;
-#pragma unroll
-                for (int u = 0; u < kTestU; ++u) anyhit |= hit[u];
-                if (!__any_sync(kFull, anyhit)) continue;
-                // a step with hits: this lane's window in chunk coordinates (computed only here)
-                const int64_t wlo64 = wx - c0, whi64 = wx + W - c0;
-                const int wlo = (int)(wlo64 < -1 ? -1 : (wlo64 > kStage ? kStage : wlo64));
-                const int whi = (int)(whi64 < -1 ? -1 : (whi64 > kStage ? kStage : whi64));
-                const int x0 = (int)((c0 - wx) - lead);
-                const int d32 = (int)d;
+                // Bit u of `pass`: entry i0 + 32 u + lane may be in Z.  What is past the filter is rare and
+                // stays in a rolled loop: unrolled, its code no longer fits the instruction cache beside
+                // the rest (27 % slower at 8 entries per lane).  A row keeps its smallest hit, so the order
+                // in which hits are taken does not matter.
+                unsigned pass = 0u;
 #pragma unroll
                 for (int u = 0; u < kTestU; ++u) {
-                    unsigned hm = __ballot_sync(kFull, hit[u]);
-                    while (hm) {
-                        const int qh = i0 + 32 * u + __ffs(hm) - 1;
-                        hm &= hm - 1u;
-                        if (qh >= wlo && qh < whi && mp == d) {
-                            const int x = qh + x0;
-                            if (x >= 0 && x < d32) mp = x;
-                        }
+                    const int q = i0 + 32 * u + lane;  // q < kStage: past nq the entry is stale and masked below
+                    if (!simple || filter_may_have<kFBits>(F, (uint32_t)stg[q] * kHashMul)) pass |= 1u << u;
+                }
+                while (__any_sync(kFull, pass != 0u)) {
+                    int q = nq;
+                    if (pass) {
+                        q = i0 + 32 * (__ffs(pass) - 1) + lane;
+                        pass &= pass - 1u;
+                    }
+                    bool hit = false;
+                    if (q < nq) {  // stale entries may hold any value: only node ids reach the masks
+                        const int32_t v = stg[q];
+                        hit = simple ? hash_contains(S.H, kHBits, v) : (uint32_t)v < (uint32_t)n && in_z(B, v);
+                    }
+                    for (unsigned m = __ballot_sync(kFull, hit); m; m &= m - 1u) {
+                        const int qh = __shfl_sync(kFull, q, __ffs(m) - 1);
+                        const int x = qh + x0;
+                        if (qh >= wlo && qh < whi && x >= 0 && x < d32 && x < mp) mp = x;
                     }
                 }
             }
@@ -691,7 +709,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
         const bool tested = !glob && !pre && lane <= first && ((consumed >> lane) & 1u);
         events += __popc(consumed);
         tests += __popc(__ballot_sync(kFull, tested));
-        scanned += warp_sum<long long>(tested ? ex : 0ll);
+        scanned += tested ? ex : 0ll;
         const unsigned took = am & consumed;
         if ((took >> lane) & 1u) S.arr[nch + __popc(took & below)] = j;
         __syncwarp();
@@ -801,6 +819,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
         }
     }
     if (nch != k && lane == 0) atomicOr(&A.st->error, kErrArg);
+    scanned = warp_sum<long long>(scanned);
     if (lane == 0 && scanned) atomicAdd(&A.st->adj_scanned, (unsigned long long)scanned);
     emit_row<KCAP>(A, rp, a, al, n, S.arr, nch, rows, tests, events);
     return true;

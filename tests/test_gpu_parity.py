@@ -728,3 +728,22 @@ def test_attribute_text_at_tile_edges(gpu, n):
             ids[v], "seed" if v < n0 else "agent", -1, draws[v, 0], draws[v, 1], draws[v, 2], ints[v, 0],
             float(fit[v]), ints[v, 1], draws[v, 3], 0, 0, ints[v, 2], ints[v, 3], gen))
     assert txt == "".join(lines)
+
+
+@pytest.mark.parametrize("small_hash", [0, 1])
+@pytest.mark.parametrize("lo,hi", [(248, 264), (502, 522), (1016, 1034)])
+def test_membership_scan_around_step_and_chunk_sizes(gpu, lo, hi, small_hash):
+    """Candidate rows of about one scan step (256 entries), one stage buffer (512 or 1,024) and two."""
+    g = _popular_seed(20_000, 900, lo, hi, seed=9)
+    prm = PAParams(alpha=1.0, tau=5.0, gamma=1.0, beta=6.0, mean_out_degree=20.0,
+                   growth_rate=0.0, fixed_new_nodes=250, num_anchors=3)
+    with GrowthEngine(seed=78, record_trace=True) as eng:
+        eng.load_graph(g.pub, g.fitness, g.src, g.dst, prm, planned_epochs=2)
+        eng.set_tuning(small_hash=small_hash)
+        og = _oracle_for(g, prm, 78, sampler=PG_SAMPLER_THINNING)
+        for _ in range(2):
+            eng.grow_epoch()
+            og.pa_epoch()
+            assert eng.stats()["adj_scanned"] == og.stats()["adj_scanned"]
+            np.testing.assert_array_equal(eng.arrivals(), og.arrivals())
+        _compare_state(eng, og)
