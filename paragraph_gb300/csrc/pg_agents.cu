@@ -582,7 +582,10 @@ __device__ __forceinline__ void d_agent_setup(const Arena& A, int64_t agents, in
     }
 }
 
-__global__ void __launch_bounds__(256) k_agent_setup(Arena A, int64_t agents) { d_agent_setup(A, agents, blockIdx.x); }
+__global__ void __launch_bounds__(256) k_agent_setup(Arena A, int64_t agents) {
+    pdl_begin();
+    d_agent_setup(A, agents, blockIdx.x);
+}
 
 // Refcompat, after the setup: a generator with many row entries, or a few long ones, makes a long
 // 2-hop stream; such agents are listed for the CTA-wide pass (k_rc_big), mark = list slot + 1.  One
@@ -647,7 +650,10 @@ __device__ __forceinline__ void d_edges_check(const Arena& A, int64_t agents) {
     }
 }
 
-__global__ void k_edges_check(Arena A, int64_t agents) { d_edges_check(A, agents); }
+__global__ void k_edges_check(Arena A, int64_t agents) {
+    pdl_begin();
+    d_edges_check(A, agents);
+}
 
 // Shapes of the k <= 64 thinning kernel (pg_tuning.small_hash = HS): 0 -- a 2048-slot frontier hash
 // (the lean instance: 1024 slots and a filter of 1024 words) and 512-entry stage buffers; 1 -- 1024
@@ -724,6 +730,7 @@ __device__ __forceinline__ void d_agents(const Arena& A, int64_t agents, unsigne
 
 template <int KCAP, bool BIG, int HS = 0>
 __global__ void __launch_bounds__(kAgentWarps * 32, 4) k_agents(Arena A, int64_t agents) {
+    pdl_begin();
     // two stage buffers per warp go past 48 KiB: dynamic
     extern __shared__ __align__(16) unsigned char agent_dsm[];
     constexpr size_t stride = thin_smem_bytes<KCAP, HS>() / kAgentWarps;
@@ -937,12 +944,12 @@ static int g_blocks_hs[2] = {0, 0};             // thinning, k <= 64, by shape (
 
 void launch_agent_setup(const Arena& A, int64_t agents, cudaStream_t s) {
     if (agents <= 0) return;
-    k_agent_setup<<<(unsigned)((agents + 255) / 256), 256, 0, s>>>(A, agents);
+    launch_dependent(k_agent_setup, (agents + 255) / 256, 256, 0, s, A, agents);
     if (A.weight_model == 1) {
         k_rc_route<<<(unsigned)((agents + 7) / 8), 256, 0, s>>>(A, agents);
     }
     scan_impl<int32_t>(A.kk, A.eoff, agents, A.blocksum, s, false);
-    k_edges_check<<<1, 256, 0, s>>>(A, agents);
+    launch_dependent(k_edges_check, 1, 256, 0, s, A, agents);
 }
 
 // Occupancy of the persistent agent kernels; called once per process before any capture.
@@ -996,10 +1003,10 @@ void launch_agents(const Arena& A, int64_t agents, int num_sms, cudaStream_t s) 
         return;
     }
     if (hs == 1)
-        k_agents<kKSmall, false, 1><<<(unsigned)grid, th, thin_smem_bytes<kKSmall, 1>(), s>>>(A, agents);
+        launch_dependent(k_agents<kKSmall, false, 1>, grid, th, thin_smem_bytes<kKSmall, 1>(), s, A, agents);
     else
-        k_agents<kKSmall, false, 0><<<(unsigned)grid, th, thin_smem_bytes<kKSmall, 0>(), s>>>(A, agents);
-    k_agents<kKMax, true><<<(unsigned)(num_sms * g_blocks_big), th, thin_smem_bytes<kKMax, 0>(), s>>>(A, agents);
+        launch_dependent(k_agents<kKSmall, false, 0>, grid, th, thin_smem_bytes<kKSmall, 0>(), s, A, agents);
+    launch_dependent(k_agents<kKMax, true>, num_sms * g_blocks_big, th, thin_smem_bytes<kKMax, 0>(), s, A, agents);
 }
 
 

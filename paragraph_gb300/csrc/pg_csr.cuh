@@ -144,7 +144,10 @@ __device__ __forceinline__ void d_bwd_grow(const Arena& A, int64_t agents) {
     if (lane == 0 && moved) atomicAdd(&A.st->bwd_moved, moved);
 }
 
-__global__ void __launch_bounds__(256) k_bwd_grow(Arena A, int64_t agents) { d_bwd_grow(A, agents); }
+__global__ void __launch_bounds__(256) k_bwd_grow(Arena A, int64_t agents) {
+    pdl_begin();
+    d_bwd_grow(A, agents);
+}
 
 // The old spans of the rows that moved (forward row copy and entries), one listed chunk (at most
 // kRelocChunk entries) per warp: source and destination are 16-byte aligned, the copy goes in int4
@@ -188,7 +191,10 @@ __device__ __forceinline__ void d_bwd_reloc(const Arena& A) {
     }
 }
 
-__global__ void __launch_bounds__(256) k_bwd_reloc(Arena A) { d_bwd_reloc(A); }
+__global__ void __launch_bounds__(256) k_bwd_reloc(Arena A) {
+    pdl_begin();
+    d_bwd_reloc(A);
+}
 
 // One warp per agent: each edge at its row's start of new entries + rank.  The agent is a new node:
 // its hub-index entry is written here (no hub bit, and a mask of the hubs it cites), so the next
@@ -233,7 +239,10 @@ __device__ __forceinline__ void d_bwd_place(const Arena& A, int64_t agents) {
     }
 }
 
-__global__ void __launch_bounds__(256) k_bwd_place(Arena A, int64_t agents) { d_bwd_place(A, agents); }
+__global__ void __launch_bounds__(256) k_bwd_place(Arena A, int64_t agents) {
+    pdl_begin();
+    d_bwd_place(A, agents);
+}
 
 // A run's citation output (pg_run_epochs_out): the epoch's citations, (source, target), at the
 // run's running count, written in whole lines -- the writes cross the host link, where a partial
@@ -290,6 +299,7 @@ __device__ __forceinline__ void d_copy_out(const Arena& A, int64_t agents, int32
 }
 
 __global__ void __launch_bounds__(256) k_copy_out(Arena A, int64_t agents) {
+    pdl_begin();
     __shared__ int32_t stage[kCopyTile];
     d_copy_out(A, agents, stage);
 }
@@ -380,7 +390,10 @@ __device__ __forceinline__ void d_sort_small(const Arena& A) {
     }
 }
 
-__global__ void __launch_bounds__(256) k_sort_small(Arena A) { d_sort_small(A); }
+__global__ void __launch_bounds__(256) k_sort_small(Arena A) {
+    pdl_begin();
+    d_sort_small(A);
+}
 
 // Rows with more than kSortMid appended entries: one CTA, shared bitmap bm of bm_words words over
 // [n, n + delta), in chunks when the range is longer.
@@ -441,6 +454,7 @@ __device__ __forceinline__ void d_sort_large(const Arena& A, uint32_t* bm, int64
 // where that fits, so two CTAs share an SM.  1024 threads per CTA: a hub's row can take tens of
 // thousands of new entries in one epoch, and that one row sets the kernel's length.
 __global__ void __launch_bounds__(1024) k_sort_large(Arena A, int64_t bm_words) {
+    pdl_begin();
     extern __shared__ uint32_t bm[];
     d_sort_large(A, bm, bm_words);
 }
@@ -469,7 +483,10 @@ __device__ __forceinline__ void d_epoch_end(const Arena& A, int64_t agents) {
     }
 }
 
-__global__ void k_epoch_end(Arena A, int64_t agents) { d_epoch_end(A, agents); }
+__global__ void k_epoch_end(Arena A, int64_t agents) {
+    pdl_begin();
+    d_epoch_end(A, agents);
+}
 
 // The large-segment sort uses 160 KiB of dynamic shared memory; called once per process.
 cudaError_t init_csr_kernels() {
@@ -479,10 +496,14 @@ cudaError_t init_csr_kernels() {
 
 void launch_bwd_append(const Arena& A, int64_t agents, int num_sms, cudaStream_t s, cudaStream_t side,
                        cudaEvent_t fork, cudaEvent_t join) {
+    // a warp per agent up to what fills the SMs; the passes over lists, which a small epoch keeps short,
+    // start no more CTAs than that, or one per SM
     int64_t ga = (agents + 7) / 8;
     if (ga > (int64_t)num_sms * 16) ga = (int64_t)num_sms * 16;
     if (ga < 1) ga = 1;
-    k_bwd_grow<<<(unsigned)ga, 256, 0, s>>>(A, agents);
+    auto at_most = [](int64_t x, int64_t most) { return x < most ? x : most; };
+    const int64_t gl = ga > num_sms ? ga : num_sms;
+    launch_dependent(k_bwd_grow, ga, 256, 0, s, A, agents);
     const int copy_per_sm = A.tune_copy_ctas > 0 ? A.tune_copy_ctas : 8;
     // the moved rows' old entries and the new entries' placement and sorts write disjoint
     // positions: with a side stream they overlap
@@ -491,19 +512,21 @@ void launch_bwd_append(const Arena& A, int64_t agents, int num_sms, cudaStream_t
         cudaEventRecord(fork, s);
         cudaStreamWaitEvent(side, fork, 0);
     }
-    k_bwd_reloc<<<(unsigned)(num_sms * copy_per_sm), 256, 0, two ? side : s>>>(A);
+    launch_dependent(k_bwd_reloc, at_most(gl, (int64_t)num_sms * copy_per_sm), 256, 0, two ? side : s, A);
     // one CTA per SM: the copy is bound by the host link, and the placement and sorts beside it
     // keep the rest of the SMs (beside the grow pass it made that pass 1.8 times as long)
-    if (A.out_src) k_copy_out<<<(unsigned)num_sms, 256, 0, two ? side : s>>>(A, agents);
+    if (A.out_src) launch_dependent(k_copy_out, num_sms, 256, 0, two ? side : s, A, agents);
     if (two) cudaEventRecord(join, side);
-    k_bwd_place<<<(unsigned)ga, 256, 0, s>>>(A, agents);
-    k_sort_small<<<(unsigned)num_sms * 8, 256, 0, s>>>(A);
+    launch_dependent(k_bwd_place, ga, 256, 0, s, A, agents);
+    launch_dependent(k_sort_small, at_most(gl, (int64_t)num_sms * 8), 256, 0, s, A);
     // a replica's new ids span at most the epoch's agents
     int64_t words = (agents + 31) / 32 + 1;
     if (words > kBitmapWords) words = kBitmapWords;
-    k_sort_large<<<(unsigned)num_sms * 2, 1024, (size_t)words * 4, s>>>(A, words);
+    // a listed row has more than kSortMid of the epoch's at most edge_cap entries
+    const int64_t rows = A.edge_cap / (kSortMid + 1) + 1;
+    launch_dependent(k_sort_large, at_most(rows, (int64_t)num_sms * 2), 1024, (size_t)words * 4, s, A, words);
     if (two) cudaStreamWaitEvent(s, join, 0);
-    k_epoch_end<<<1, 256, 0, s>>>(A, agents);
+    launch_dependent(k_epoch_end, 1, 256, 0, s, A, agents);
 }
 
 }  // namespace pg

@@ -20,7 +20,7 @@ int scan_blocks_needed(int64_t n) { return (int)((n + kScanBlock - 1) / kScanBlo
 
 // block vb of the reduce step (kScanThreads threads)
 template <typename TIn>
-__device__ __forceinline__ void d_scan_reduce(const TIn* __restrict__ in, int64_t n, int64_t* __restrict__ blocksum,
+__device__ __forceinline__ void d_scan_reduce(const TIn* in, int64_t n, int64_t* blocksum,
                                               int vb) {
     __shared__ int64_t sw[33];
     const int64_t base = (int64_t)vb * kScanBlock;
@@ -41,14 +41,15 @@ __device__ __forceinline__ void d_scan_reduce(const TIn* __restrict__ in, int64_
 }
 
 template <typename TIn>
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const TIn* __restrict__ in, int64_t n,
-                                                              int64_t* __restrict__ blocksum) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const TIn* in, int64_t n,
+                                                              int64_t* blocksum) {
+    pdl_begin();
     d_scan_reduce<TIn>(in, n, blocksum, blockIdx.x);
 }
 
 // One CTA (any multiple of 32 threads up to 1024): exclusive scan of blocksum[0..nb) in place;
 // blocksum[nb] = total.
-__device__ __forceinline__ void d_scan_blocksums(int64_t* __restrict__ blocksum, int nb) {
+__device__ __forceinline__ void d_scan_blocksums(int64_t* blocksum, int nb) {
     __shared__ int64_t sw[33];
     __shared__ int64_t carry;
     if (threadIdx.x == 0) carry = 0;
@@ -66,14 +67,15 @@ __device__ __forceinline__ void d_scan_blocksums(int64_t* __restrict__ blocksum,
     if (threadIdx.x == 0) blocksum[nb] = carry;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_blocksums(int64_t* __restrict__ blocksum, int nb) {
+__global__ void __launch_bounds__(1024) k_scan_blocksums(int64_t* blocksum, int nb) {
+    pdl_begin();
     d_scan_blocksums(blocksum, nb);
 }
 
 // block vb of the apply step (kScanThreads threads)
 template <typename TIn>
-__device__ __forceinline__ void d_scan_apply(const TIn* __restrict__ in, int64_t n, const int64_t* __restrict__ blocksum,
-                                             int nb, int64_t* __restrict__ out, int vb) {
+__device__ __forceinline__ void d_scan_apply(const TIn* in, int64_t n, const int64_t* blocksum,
+                                             int nb, int64_t* out, int vb) {
     __shared__ int64_t sw[33];
     const int64_t base = (int64_t)vb * kScanBlock + (int64_t)threadIdx.x * kScanItems;
     int64_t v[kScanItems];
@@ -96,17 +98,19 @@ __device__ __forceinline__ void d_scan_apply(const TIn* __restrict__ in, int64_t
 }
 
 template <typename TIn>
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const TIn* __restrict__ in, int64_t n,
-                                                             const int64_t* __restrict__ blocksum,
-                                                             int nb, int64_t* __restrict__ out) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const TIn* in, int64_t n,
+                                                             const int64_t* blocksum,
+                                                             int nb, int64_t* out) {
+    pdl_begin();
     d_scan_apply<TIn>(in, n, blocksum, nb, out, blockIdx.x);
 }
 
 // The apply step from the tiles' own sums.
 template <typename TIn>
-__global__ void __launch_bounds__(kScanThreads) k_scan_direct(const TIn* __restrict__ in, int64_t n,
-                                                              const int64_t* __restrict__ sums, int nb,
-                                                              int64_t* __restrict__ out) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_direct(const TIn* in, int64_t n,
+                                                              const int64_t* sums, int nb,
+                                                              int64_t* out) {
+    pdl_begin();
     __shared__ int64_t sw[33];
     const int vb = blockIdx.x;
     int64_t before = 0;
@@ -142,13 +146,13 @@ static void scan_impl(const TIn* in, int64_t* out, int64_t n, int64_t* blocksum,
     }
     const int nb = scan_blocks_needed(n);
     direct = direct && nb <= kScanDirect;
-    if (nb > 1 || !direct) k_scan_reduce<TIn><<<nb, kScanThreads, 0, s>>>(in, n, blocksum);
+    if (nb > 1 || !direct) launch_dependent(k_scan_reduce<TIn>, nb, kScanThreads, 0, s, in, n, blocksum);
     if (direct) {
-        k_scan_direct<TIn><<<nb, kScanThreads, 0, s>>>(in, n, blocksum, nb, out);
+        launch_dependent(k_scan_direct<TIn>, nb, kScanThreads, 0, s, in, n, blocksum, nb, out);
         return;
     }
-    k_scan_blocksums<<<1, 1024, 0, s>>>(blocksum, nb);
-    k_scan_apply<TIn><<<nb, kScanThreads, 0, s>>>(in, n, blocksum, nb, out);
+    launch_dependent(k_scan_blocksums, 1, 1024, 0, s, blocksum, nb);
+    launch_dependent(k_scan_apply<TIn>, nb, kScanThreads, 0, s, in, n, blocksum, nb, out);
 }
 
 void launch_scan_i64(const int64_t* in, int64_t* out, int64_t n, int64_t* blocksum, cudaStream_t s) {

@@ -78,7 +78,10 @@ __device__ __forceinline__ void d_epoch_begin(const Arena& A, int64_t epoch, int
     }
 }
 
-__global__ void __launch_bounds__(1024) k_epoch_begin(Arena A, int64_t epoch, int64_t delta_override) { d_epoch_begin(A, epoch, delta_override); }
+__global__ void __launch_bounds__(1024) k_epoch_begin(Arena A, int64_t epoch, int64_t delta_override) {
+    pdl_begin();
+    d_epoch_begin(A, epoch, delta_override);
+}
 
 // w_j for active nodes; per-replica max (as float bits, valid for non-negative floats) and count
 // of positive weights.
@@ -148,7 +151,10 @@ __device__ __forceinline__ void d_weights(const Arena& A, int vb) {
     }
 }
 
-__global__ void __launch_bounds__(kTileThreads) k_weights(Arena A) { d_weights(A, blockIdx.x); }
+__global__ void __launch_bounds__(kTileThreads) k_weights(Arena A) {
+    pdl_begin();
+    d_weights(A, blockIdx.x);
+}
 
 // q_j = quantise(w_j, s_r); tile-local inclusive scan into cdf, tile total into tilesum.
 __device__ __forceinline__ void d_cdf_tiles(const Arena& A, int vb) {
@@ -188,7 +194,10 @@ __device__ __forceinline__ void d_cdf_tiles(const Arena& A, int vb) {
     if (threadIdx.x == 0) A.tilesum[t] = tot;
 }
 
-__global__ void __launch_bounds__(kTileThreads) k_cdf_tiles(Arena A) { d_cdf_tiles(A, blockIdx.x); }
+__global__ void __launch_bounds__(kTileThreads) k_cdf_tiles(Arena A) {
+    pdl_begin();
+    d_cdf_tiles(A, blockIdx.x);
+}
 
 // One CTA: tileoff[t] = sum of tilesum over the earlier tiles of the same replica (mod 2^64, which
 // is exact because every replica's own total is below 2^63); each replica's total goes to wq_total.
@@ -222,7 +231,10 @@ __device__ __forceinline__ void d_tile_scan(const Arena& A) {
     for (int i = threadIdx.x; i < T; i += blockDim.x) A.tileoff[i] -= A.tilesum[A.tile_rep[i]];
 }
 
-__global__ void __launch_bounds__(1024) k_tile_scan(Arena A) { d_tile_scan(A); }
+__global__ void __launch_bounds__(1024) k_tile_scan(Arena A) {
+    pdl_begin();
+    d_tile_scan(A);
+}
 
 // Tile offsets into the CDF, and the guide table's marks: node v whose CDF interval
 // [cdf[v-1], cdf[v]) contains bucket starts g 2^gs marks the first of them, guide[g] = v.
@@ -262,7 +274,10 @@ __device__ __forceinline__ void d_cdf_add(const Arena& A, int vb) {
     }
 }
 
-__global__ void __launch_bounds__(kTileThreads) k_cdf_add(Arena A) { d_cdf_add(A, blockIdx.x); }
+__global__ void __launch_bounds__(kTileThreads) k_cdf_add(Arena A) {
+    pdl_begin();
+    d_cdf_add(A, blockIdx.x);
+}
 
 // Guide table fill: guide[g] = smallest v with cdf[v] > g 2^gs, for g < used(Wq, n).  Each tile of
 // buckets takes the running maximum of its marks, starting from the node that owns its first
@@ -323,7 +338,10 @@ __device__ __forceinline__ void d_guide_fill(const Arena& A, int vb) {
     *gp = m;
 }
 
-__global__ void __launch_bounds__(kTileThreads) k_guide_fill(Arena A) { d_guide_fill(A, blockIdx.x); }
+__global__ void __launch_bounds__(kTileThreads) k_guide_fill(Arena A) {
+    pdl_begin();
+    d_guide_fill(A, blockIdx.x);
+}
 
 // ---------------------------------------------------------------- hub index
 // Ball membership of a high-degree node j needs adj(j) intersected with the agent's 1-hop
@@ -378,7 +396,10 @@ __device__ __forceinline__ void d_hub_hist(const Arena& A, int vb) {
     }
 }
 
-__global__ void __launch_bounds__(kTileThreads) k_hub_hist(Arena A) { d_hub_hist(A, blockIdx.x); }
+__global__ void __launch_bounds__(kTileThreads) k_hub_hist(Arena A) {
+    pdl_begin();
+    d_hub_hist(A, blockIdx.x);
+}
 
 // Threshold and cleared lists of replica r (one CTA of kHeavyMax threads or more).
 __device__ __forceinline__ void d_hub_pick(const Arena& A, int r) {
@@ -413,7 +434,10 @@ __device__ __forceinline__ void d_hub_pick(const Arena& A, int r) {
 }
 
 // one CTA per replica: one for all of them took 98 us for the 256 of an ensemble
-__global__ void __launch_bounds__(kHeavyMax) k_hub_pick(Arena A) { d_hub_pick(A, blockIdx.x); }
+__global__ void __launch_bounds__(kHeavyMax) k_hub_pick(Arena A) {
+    pdl_begin();
+    d_hub_pick(A, blockIdx.x);
+}
 
 // Nodes leaving the hub set give up their bit (hub_rem), nodes joining it are listed (hub_cand).
 __device__ __forceinline__ void d_hub_collect(const Arena& A, int vb) {
@@ -448,7 +472,10 @@ __device__ __forceinline__ void d_hub_collect(const Arena& A, int vb) {
     }
 }
 
-__global__ void __launch_bounds__(kTileThreads) k_hub_collect(Arena A) { d_hub_collect(A, blockIdx.x); }
+__global__ void __launch_bounds__(kTileThreads) k_hub_collect(Arena A) {
+    pdl_begin();
+    d_hub_collect(A, blockIdx.x);
+}
 
 // Bits of the epoch, one warp per replica: the bits given up are freed, and the q-th joining node
 // takes the q-th free bit.  (At most kHeavyMax nodes have degree >= heavy_thr, so there are always
@@ -502,7 +529,10 @@ __device__ __forceinline__ void d_hub_assign(const Arena& A) {
     }
 }
 
-__global__ void __launch_bounds__(256) k_hub_assign(Arena A) { d_hub_assign(A); }
+__global__ void __launch_bounds__(256) k_hub_assign(Arena A) {
+    pdl_begin();
+    d_hub_assign(A);
+}
 
 // The replica's bits that `want` names, listed in shared memory by a CTA of at least kHeavyMax threads;
 // their number.
@@ -558,7 +588,10 @@ __device__ __forceinline__ void d_hub_mask(const Arena& A, int G, int vb) {
 }
 
 template <bool SET>
-__global__ void __launch_bounds__(kHeavyMax) k_hub_mask(Arena A, int G) { d_hub_mask<SET>(A, G, blockIdx.x); }
+__global__ void __launch_bounds__(kHeavyMax) k_hub_mask(Arena A, int G) {
+    pdl_begin();
+    d_hub_mask<SET>(A, G, blockIdx.x);
+}
 
 // hub2[b] = OR of hmask over the hub's neighbours: the hubs sharing a neighbour with hub b; only for
 // the hubs that are some agent's anchor (no other row is read).  CTAs as in d_hub_mask.
@@ -607,7 +640,10 @@ __device__ __forceinline__ void d_hub_pairs(const Arena& A, int G, int vb) {
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kHeavyMax) k_hub_pairs(Arena A, int G) { d_hub_pairs(A, G, blockIdx.x); }
+__global__ void __launch_bounds__(kHeavyMax) k_hub_pairs(Arena A, int G) {
+    pdl_begin();
+    d_hub_pairs(A, G, blockIdx.x);
+}
 
 // CTAs per replica of the hub kernels that walk rows: two per SM over all replicas, at least eight
 int hub_ctas(int R, int num_sms) {
@@ -617,35 +653,35 @@ int hub_ctas(int R, int num_sms) {
 
 void launch_hubs(const Arena& A, int num_sms, cudaStream_t s) {
     const int G = hub_ctas(A.R, num_sms);
-    k_hub_hist<<<A.ntiles, kTileThreads, 0, s>>>(A);
-    k_hub_pick<<<A.R, kHeavyMax, 0, s>>>(A);
-    k_hub_collect<<<A.ntiles, kTileThreads, 0, s>>>(A);
-    k_hub_assign<<<(unsigned)((A.R + 7) / 8), 256, 0, s>>>(A);  // a warp per replica (one CTA for 256: 190 us)
-    k_hub_mask<false><<<(unsigned)(A.R * G), kHeavyMax, 0, s>>>(A, G);
-    k_hub_mask<true><<<(unsigned)(A.R * G), kHeavyMax, 0, s>>>(A, G);
+    launch_dependent(k_hub_hist, A.ntiles, kTileThreads, 0, s, A);
+    launch_dependent(k_hub_pick, A.R, kHeavyMax, 0, s, A);
+    launch_dependent(k_hub_collect, A.ntiles, kTileThreads, 0, s, A);
+    launch_dependent(k_hub_assign, (A.R + 7) / 8, 256, 0, s, A);  // a warp per replica (one CTA for 256: 190 us)
+    launch_dependent(k_hub_mask<false>, A.R * G, kHeavyMax, 0, s, A, G);
+    launch_dependent(k_hub_mask<true>, A.R * G, kHeavyMax, 0, s, A, G);
 }
 
 void launch_hub_pairs(const Arena& A, int num_sms, cudaStream_t s) {
     const int G = hub_ctas(A.R, num_sms);
-    k_hub_pairs<<<(unsigned)(A.R * G), kHeavyMax, 0, s>>>(A, G);
+    launch_dependent(k_hub_pairs, A.R * G, kHeavyMax, 0, s, A, G);
 }
 
 void launch_epoch_begin(const Arena& A, int64_t epoch, int pa_mode, cudaStream_t s) {
     (void)pa_mode;
-    k_epoch_begin<<<1, 1024, 0, s>>>(A, epoch, -1);
+    launch_dependent(k_epoch_begin, 1, 1024, 0, s, A, epoch, -1);
 }
 
 void launch_epoch_begin_delta(const Arena& A, int64_t epoch, int64_t delta, cudaStream_t s) {
-    k_epoch_begin<<<1, 1024, 0, s>>>(A, epoch, delta);
+    launch_dependent(k_epoch_begin, 1, 1024, 0, s, A, epoch, delta);
 }
 
 void launch_weights(const Arena& A, cudaStream_t s) {
-    k_weights<<<A.ntiles, kTileThreads, 0, s>>>(A);
-    k_cdf_tiles<<<A.ntiles, kTileThreads, 0, s>>>(A);
-    k_tile_scan<<<1, 1024, 0, s>>>(A);
-    k_cdf_add<<<A.ntiles, kTileThreads, 0, s>>>(A);
+    launch_dependent(k_weights, A.ntiles, kTileThreads, 0, s, A);
+    launch_dependent(k_cdf_tiles, A.ntiles, kTileThreads, 0, s, A);
+    launch_dependent(k_tile_scan, 1, 1024, 0, s, A);
+    launch_dependent(k_cdf_add, A.ntiles, kTileThreads, 0, s, A);
 }
 
-void launch_guide(const Arena& A, cudaStream_t s) { k_guide_fill<<<A.ntiles, kTileThreads, 0, s>>>(A); }
+void launch_guide(const Arena& A, cudaStream_t s) { launch_dependent(k_guide_fill, A.ntiles, kTileThreads, 0, s, A); }
 
 }  // namespace pg

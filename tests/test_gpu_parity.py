@@ -747,3 +747,23 @@ def test_membership_scan_around_step_and_chunk_sizes(gpu, lo, hi, small_hash):
             assert eng.stats()["adj_scanned"] == og.stats()["adj_scanned"]
             np.testing.assert_array_equal(eng.arrivals(), og.arrivals())
         _compare_state(eng, og)
+
+
+@pytest.mark.parametrize("delta", [1, 6072, 6080, 6088])
+def test_epochs_on_both_sides_of_the_dependent_launch_size(gpu, delta):
+    """Launches of 194,560 threads and fewer start while the kernel before them runs: single epochs and
+    one captured run equal the oracle."""
+    g = W.plain_pa_seed(4000, 6, seed=12)
+    prm = PAParams(mean_out_degree=5.0, growth_rate=0.0, fixed_new_nodes=delta)
+    og = _oracle_for(g, prm, 31, sampler=PG_SAMPLER_THINNING)
+    for _ in range(3):
+        og.pa_epoch()
+    for graph in (False, True):
+        with GrowthEngine(seed=31) as eng:
+            eng.load_graph(g.pub, g.fitness, g.src, g.dst, prm, planned_epochs=3)
+            if graph:
+                eng.run_epochs(3, use_graph=True)
+            else:
+                for _ in range(3):
+                    eng.grow_epoch()
+            _compare_state(eng, og)
