@@ -57,12 +57,57 @@ __device__ __forceinline__ void store_text(char* __restrict__ dst, const char* _
     }
 }
 
-// A tile of kTextTile edges, kTextEdges consecutive ones per thread.  Their sources come from the tile's
-// own row starts: each row marks its first edge (the last of several rows that start at one edge, the
-// others being empty, is the source), and a running maximum carries the marks on.  The pass without an
-// output leaves the tile's bytes in `sums`, the writing pass places the tile at off[tile].  1.2M edges: 12 us
-// to measure and 25 to write, where a thread per edge, each with its bisection, took 31 and 62.
 constexpr int kTextThreads = 256;
+
+// Rows of the tile's edges [e0, e1), EDGES consecutive ones per thread, all kTextThreads threads.  They
+// come from the tile's own row starts: each row marks its first edge (the last of several rows that
+// start at one edge, the others being empty, is the source), and a running maximum carries the marks on.
+template <int EDGES>
+__device__ __forceinline__ void tile_sources(const int64_t* __restrict__ fo, int64_t n, int64_t e0, int64_t e1,
+                                             int64_t (&row)[EDGES]) {
+    __shared__ int s_row[kTextThreads * EDGES];
+    __shared__ int s_max[kTextThreads / 32];
+    __shared__ int64_t s_first;
+    const int lane = lane_id(), wid = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < kTextThreads * EDGES; i += kTextThreads) s_row[i] = 0;
+    if (wid == 0) {
+        const int64_t f = warp_last_below(n, [&](int64_t r) { return fo[r] <= e0; });
+        if (lane == 0) s_first = f;
+    }
+    __syncthreads();
+    const int64_t first = s_first;
+    // rows after the first, until one starts past the tile
+    for (int64_t r0 = first + 1;; r0 += kTextThreads) {
+        const int64_t r = r0 + threadIdx.x;
+        const int64_t p = r < n ? fo[r] : e1;
+        if (p < e1) atomicMax(&s_row[p - e0], (int)(r - first));
+        if (__syncthreads_or(p >= e1)) break;
+    }
+    int mark[EDGES], run = 0;
+#pragma unroll
+    for (int k = 0; k < EDGES; ++k) {
+        run = max(run, s_row[threadIdx.x * EDGES + k]);
+        mark[k] = run;
+    }
+    int incl = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl = max(incl, y);
+    }
+    if (lane == 31) s_max[wid] = incl;
+    int before = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) before = 0;
+    __syncthreads();
+    for (int w = 0; w < wid; ++w) before = max(before, s_max[w]);
+#pragma unroll
+    for (int k = 0; k < EDGES; ++k) row[k] = first + max(before, mark[k]);
+    __syncthreads();  // the shared arrays are the next tile's
+}
+
+// A tile of kTextTile edges.  The pass without an output leaves the tile's bytes in `sums`, the writing
+// pass places the tile at off[tile].  1.2M edges: 12 us to measure and 25 to write, where a thread per
+// edge, each with its bisection, took 31 and 62.
 constexpr int kTextEdges = 2;
 constexpr int kTextTile = kTextThreads * kTextEdges;
 constexpr int kLineMax = 42;  // two 64-bit ids of 20 characters, a comma and a newline
@@ -72,47 +117,14 @@ __global__ void __launch_bounds__(kTextThreads) k_text(const int64_t* __restrict
                                                        int64_t n, int64_t m, const int64_t* __restrict__ ids,
                                                        int32_t* __restrict__ sums, const int64_t* __restrict__ off,
                                                        char* __restrict__ out) {
-    __shared__ int s_row[kTextTile];
     __shared__ int s_scan[33];
-    __shared__ int64_t s_first;
     __shared__ __align__(16) char stage[WRITE ? kTextTile * kLineMax + 16 : 16];
     const int64_t tiles = (m + kTextTile - 1) / kTextTile;
-    const int lane = lane_id(), wid = threadIdx.x >> 5;
     for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         const int64_t e0 = t * kTextTile;
         const int64_t e1 = e0 + kTextTile < m ? e0 + kTextTile : m;
-        for (int i = threadIdx.x; i < kTextTile; i += kTextThreads) s_row[i] = 0;
-        if (wid == 0) {
-            const int64_t f = warp_last_below(n, [&](int64_t r) { return fo[r] <= e0; });
-            if (lane == 0) s_first = f;
-        }
-        __syncthreads();
-        const int64_t first = s_first;
-        // rows after the first, until one starts past the tile
-        for (int64_t r0 = first + 1;; r0 += kTextThreads) {
-            const int64_t r = r0 + threadIdx.x;
-            const int64_t p = r < n ? fo[r] : e1;
-            if (p < e1) atomicMax(&s_row[p - e0], (int)(r - first));
-            if (__syncthreads_or(p >= e1)) break;
-        }
-        int row[kTextEdges], run = 0;
-#pragma unroll
-        for (int k = 0; k < kTextEdges; ++k) {
-            run = max(run, s_row[threadIdx.x * kTextEdges + k]);
-            row[k] = run;
-        }
-        int incl = run;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl = max(incl, y);
-        }
-        if (lane == 31) s_scan[wid] = incl;
-        int before = __shfl_up_sync(0xffffffffu, incl, 1);
-        if (lane == 0) before = 0;
-        __syncthreads();
-        for (int w = 0; w < wid; ++w) before = max(before, s_scan[w]);
-        __syncthreads();
+        int64_t row[kTextEdges];
+        tile_sources<kTextEdges>(fo, n, e0, e1, row);
         int64_t a[kTextEdges], b[kTextEdges];
         int la[kTextEdges], lb[kTextEdges], mine = 0;
 #pragma unroll
@@ -120,7 +132,7 @@ __global__ void __launch_bounds__(kTextThreads) k_text(const int64_t* __restrict
             const int64_t e = e0 + threadIdx.x * kTextEdges + k;
             la[k] = lb[k] = 0;
             if (e < e1) {
-                a[k] = ids[first + max(before, row[k])];
+                a[k] = ids[row[k]];
                 b[k] = ids[fc[e]];
                 la[k] = dec_len(a[k]);
                 lb[k] = dec_len(b[k]);
@@ -151,26 +163,33 @@ __global__ void __launch_bounds__(kTextThreads) k_text(const int64_t* __restrict
     }
 }
 
-// Sources of the edges [first, first + count): one thread per row writes the row's part of the
-// range (rows are contiguous in edge order, so the writes of neighbouring rows are adjacent).
-__global__ void __launch_bounds__(256) k_edge_sources(const int64_t* fo, int64_t n, int64_t first, int64_t count,
-                                                      int32_t* out) {
-    const int64_t last = first + count;
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        int64_t p0 = fo[v], p1 = fo[v + 1];
-        if (p1 <= first || p0 >= last) continue;
-        p0 = p0 > first ? p0 : first;
-        p1 = p1 < last ? p1 : last;
-        for (int64_t p = p0; p < p1; ++p) out[p - first] = (int32_t)v;
+// Sources of the edges [first, first + count), a tile of kSrcTile edges per CTA and step, stored whole (a
+// thread per row wrote its row entry by entry: 125 us for 10M edges of 100-entry rows, now 33).
+constexpr int kSrcEdges = 4;
+constexpr int kSrcTile = kTextThreads * kSrcEdges;
+__global__ void __launch_bounds__(kTextThreads) k_edge_sources(const int64_t* __restrict__ fo, int64_t n, int64_t first,
+                                                               int64_t count, int32_t* __restrict__ out) {
+    for (int64_t t0 = (int64_t)blockIdx.x * kSrcTile; t0 < count; t0 += (int64_t)gridDim.x * kSrcTile) {
+        const int64_t t1 = t0 + kSrcTile < count ? t0 + kSrcTile : count;
+        int64_t row[kSrcEdges];
+        tile_sources<kSrcEdges>(fo, n, first + t0, first + t1, row);
+        const int64_t at = t0 + threadIdx.x * kSrcEdges;
+        if (at + kSrcEdges <= t1) {  // `out` is an allocation's start: 16-byte aligned
+            *reinterpret_cast<int4*>(out + at) = make_int4((int)row[0], (int)row[1], (int)row[2], (int)row[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kSrcEdges; ++k)
+                if (at + k < t1) out[at + k] = (int32_t)row[k];
+        }
     }
 }
 
 void launch_edge_sources(const int64_t* fo, int64_t n, int64_t first, int64_t count, int32_t* out,
                          int num_sms, cudaStream_t s) {
     if (count <= 0 || n <= 0) return;
-    int64_t g = (n + 255) / 256;
-    if (g > (int64_t)num_sms * 16) g = (int64_t)num_sms * 16;
-    k_edge_sources<<<(unsigned)g, 256, 0, s>>>(fo, n, first, count, out);
+    int64_t g = (count + kSrcTile - 1) / kSrcTile;
+    if (g > (int64_t)num_sms * 8) g = (int64_t)num_sms * 8;
+    k_edge_sources<<<(unsigned)g, kTextThreads, 0, s>>>(fo, n, first, count, out);
 }
 
 int64_t text_tiles(int64_t m) { return (m + kTextTile - 1) / kTextTile; }

@@ -767,3 +767,22 @@ def test_epochs_on_both_sides_of_the_dependent_launch_size(gpu, delta):
                 for _ in range(3):
                     eng.grow_epoch()
             _compare_state(eng, og)
+
+
+@pytest.mark.parametrize("first,count", [(0, 1), (0, 1023), (1, 1024), (3, 1025), (2999, 3000), (0, 6001), (6000, 1)])
+def test_edge_sources_of_ranges(gpu, first, count):
+    """Ranges that start and end inside rows and tiles, past runs of rows without citations."""
+    rng = np.random.default_rng(5)
+    src = np.sort(rng.choice(np.array([900, 901, 905, 2500, 2501, 2999]), 6001 * 2))
+    pairs = np.unique(np.stack([src, rng.integers(0, 899, len(src))], 1), axis=0)
+    k = 0
+    while len(pairs) < 6001:
+        pairs = np.unique(np.concatenate([pairs, [[2000 + k // 800, k % 800]]]), axis=0)
+        k += 1
+    pairs = pairs[:6001]
+    with GrowthEngine(seed=4) as eng:
+        eng.load_graph(np.full(3000, -1, np.int32), np.ones(3000, np.float32), pairs[:, 0].astype(np.int32),
+                       pairs[:, 1].astype(np.int32), PAParams(fixed_new_nodes=10), planned_epochs=1)
+        s, d = eng.edges(first, count)
+    np.testing.assert_array_equal(s, pairs[first:first + count, 0])
+    np.testing.assert_array_equal(d, pairs[first:first + count, 1])
