@@ -697,11 +697,11 @@ def loglik_measure(args, world, rank, local, dist, with_cpu: bool = True) -> dic
         "ball_elements": st["lik_ball_elems"], "adjacency_entries": st["lik_adj_entries"],
         "weight_evals_per_s": 2 * st["lik_ball_elems"] * len(pts) * args.steps / ((ms_f + ms_b) / 1000.0),
         "ms_forward": ms_f / args.steps, "ms_adjoint": ms_b / args.steps,
-        "roofline": {"bound": "hbm", "kernel": "k_lik_global + k_lik_agents (forward + adjoint)",
+        "roofline": {"bound": "hbm", "kernel": "k_lik_global + k_lik_table2 (forward + adjoint)",
                      "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": achieved / peak if peak else None, "traffic": None,
-                     "note": "at 64 points the passes are bound by the per-point exp of every ball "
-                             "element, not by HBM"},
+                     "note": "at 64 points the forward is bound by its weight rows' way from L2 and "
+                             "the adjoint by the fp32 pipe, not by HBM"},
         "serial": {"ms_per_step": ser_ms, "speedup": ser_ms / (ms_max / args.steps)},
         "exact_arithmetic": {"value": evals / (ms_x / 1000.0), "unit": "gradient evals/s",
                              "ms_per_step": ms_x / args.steps, "serial_ms_per_step": ser_x,

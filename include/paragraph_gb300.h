@@ -375,7 +375,7 @@ pg_status pg_trace_load(pg_ctx* ctx, const pg_trace_desc* trace);
  * and product on its own into compensated sums.  The per-node roundings of exact = 0 do not
  * average out and leave about 1e-5 of the gradient's norm where the gradient nearly vanishes (at a
  * trace's generating parameters; 1e-7 elsewhere); exact = 1 keeps the gradient within 1e-6 of the
- * FP64 value there too, at about a third of the throughput. */
+ * FP64 value there too, at about half of the throughput. */
 pg_status pg_lik_set_exact_exp2(pg_ctx* ctx, int32_t exact);
 /* log L at each of batch points theta[b] = (alpha, tau, gamma, beta) (row-major [batch][4]).  Saves
  * the per-agent normalisers Z_a for pg_loglik_bwd. */

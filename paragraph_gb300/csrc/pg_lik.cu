@@ -18,7 +18,7 @@
 //   exact_exp2  every product and sum of the exponent keeps its rounding error, log f is an FP64 log
 //               carried as high part plus packed remainder, 2^(h + l) from exp2_exact (fp32
 //               arithmetic, about 2 ulp), and every ball weight and product is summed on its own
-//               (BallSum): ~3e-7 of the gradient's norm there, at about a third of the throughput.
+//               (BallSum): ~3e-7 of the gradient's norm there, at about half of the throughput.
 // The same weight function feeds every sum below, so the normalisers and the citations' prefix
 // sums agree: an error that is a smooth function of the weight (such as the unit's) largely
 // cancels between them.  The per-epoch sums over all nodes are shared by every agent of the epoch, so they are
