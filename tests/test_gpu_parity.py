@@ -786,3 +786,17 @@ def test_edge_sources_of_ranges(gpu, first, count):
         s, d = eng.edges(first, count)
     np.testing.assert_array_equal(s, pairs[first:first + count, 0])
     np.testing.assert_array_equal(d, pairs[first:first + count, 1])
+
+
+@pytest.mark.parametrize("n0,delta,deg", [(3, 20_000, 2.0), (60, 8193, 3.0), (40, 1025, 20.0), (700, 40_000, 12.0)])
+def test_long_appended_rows(gpu, n0, delta, deg):
+    """Rows with from 257 to 20,000 new entries, dense and sparse in the epoch's ids, whole and cut words."""
+    g = W.plain_pa_seed(n0, 2, seed=3)
+    prm = PAParams(mean_out_degree=deg, growth_rate=0.0, fixed_new_nodes=delta)
+    with GrowthEngine(seed=8) as eng:
+        eng.load_graph(g.pub, g.fitness, g.src, g.dst, prm, planned_epochs=1)
+        og = _oracle_for(g, prm, 8)
+        eng.grow_epoch()
+        og.pa_epoch()
+        assert og.degrees()[0][:n0].max() > 256
+        _compare_state(eng, og)
