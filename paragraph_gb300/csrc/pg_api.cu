@@ -1074,7 +1074,7 @@ pg_status enqueue_pa_epoch(pg_ctx* c, int64_t epoch, int64_t agents, cudaEvent_t
         launch_rc_scores(A, s);
         PG_STAGE("refcompat scores");
         if (events) record_event(ev[1], s);
-        launch_agent_setup(A, agents, s);
+        launch_agent_setup(A, agents, c->num_sms, s);
         PG_STAGE("agent setup");
         if (events) record_event(ev[2], s);
         launch_rc_agents(A, agents, c->num_sms, s, c->side, c->fork, c->join);
@@ -1106,12 +1106,11 @@ pg_status enqueue_pa_epoch(pg_ctx* c, int64_t epoch, int64_t agents, cudaEvent_t
         c->launches += kThinKernels;
     }
     if (events) record_event(ev[1], s);
-    launch_agent_setup(A, agents, s);
+    if (thin)
+        launch_agent_setup(A, agents, c->num_sms, s, c->side, c->fork, c->join);
+    else
+        launch_agent_setup(A, agents, c->num_sms, s);
     PG_STAGE("agent setup");
-    if (c->cfg.sampler == PG_SAMPLER_THINNING) {
-        launch_hub_pairs(A, c->num_sms, s);  // for the hubs the setup found among the anchors
-        PG_STAGE("hub pairs");
-    }
     if (events) record_event(ev[2], s);
     launch_agents(A, agents, c->num_sms, s);
     PG_STAGE("agents");

@@ -540,7 +540,9 @@ void launch_weights(const Arena& A, cudaStream_t s);
 void launch_hubs(const Arena& A, int num_sms, cudaStream_t s);
 void launch_hub_pairs(const Arena& A, int num_sms, cudaStream_t s);
 void launch_guide(const Arena& A, cudaStream_t s);
-void launch_agent_setup(const Arena& A, int64_t agents, cudaStream_t s);
+// With a side stream (thinning): the hub pairs beside the offset scan.
+void launch_agent_setup(const Arena& A, int64_t agents, int num_sms, cudaStream_t s, cudaStream_t side = nullptr,
+                        cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
 void launch_agents(const Arena& A, int64_t agents, int num_sms, cudaStream_t s);
 // The whole thinning PA epoch (baseline weights) as one cooperative persistent kernel: every stage
 // above as a phase, grid barriers between dependent phases.  epoch_kernel_ctas() is its grid (0
