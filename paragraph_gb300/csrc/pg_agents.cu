@@ -656,7 +656,7 @@ __global__ void k_edges_check(Arena A, int64_t agents) {
 }
 
 // Shapes of the k <= 64 thinning kernel (pg_tuning.small_hash = HS): 0 -- a 2048-slot frontier hash
-// (the lean instance: 1024 slots and a filter of 1024 words) and 512-entry stage buffers; 1 -- 1024
+// and 512-entry stage buffers (the lean instance: 1024 slots, a filter of 512 words and 768-entry stages); 1 -- 1024
 // slots, a filter of 256 words and 1024-entry stages; both 4 CTAs per SM.  The k <= 256 kernel always
 // has 1024 slots, 256 filter words and 512-entry stages.  Shapes with more resident warps were
 // measured on the PA workload and were slower: 1024 slots and 512-entry stages at 5 CTAs per SM (96

@@ -12,6 +12,7 @@
 //   its length at the region's bump pointer.
 #pragma once
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "pg_core.cuh"

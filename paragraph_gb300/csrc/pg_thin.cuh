@@ -152,6 +152,7 @@ __device__ __forceinline__ uint32_t hslot_of(int32_t v, int bits) {
 // warps per SM, and the scan is its largest part (1,535 of a warp's cycles per 512 entries with it).
 // PA at scale, 30 epochs: 37.7 ms of agent kernels without the filter, 33.1 with 256 words, 31.9 with
 // 1,024, and 31.7 with hits taken in any order; 256 replicas x 10 epochs: 67.1, 61.7, 60.1 and 56.5 ms.
+// 512 words and stage buffers of 768 entries instead of 1,024 and 512 took the run from 34.9 to 34.7 ms.
 template <int BITS>
 __device__ __forceinline__ bool filter_may_have(const uint32_t* F, uint32_t h) {
     const uint32_t w = F[h >> (32 - BITS)];
@@ -310,16 +311,22 @@ struct FrontierPos<false> {
 template <int KCAP, int HCAP, int STAGE, bool GENERAL>
 __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KCAP, HCAP, STAGE>& S,
                                    uint32_t& phase) {
-    constexpr int kStage = STAGE;
-    // The lean instance's frontiers have at most 512 entries: where the set has 2048 slots it uses half
-    // of them and lays a filter of 1024 words over the other half.
-    constexpr bool kHalf = !GENERAL && HCAP == 2048;
-    constexpr int kSlots = kHalf ? HCAP / 2 : HCAP;
+    // The lean instance's frontiers have at most 512 entries: where the set has 2048 slots it needs half of
+    // them, and lays the warp's 13 KB out anew: stage buffers of 768 entries, 1024 slots, and a filter of
+    // 512 words.
+    constexpr bool kLean = !GENERAL && HCAP == 2048 && STAGE == 512;
+    constexpr int kStage = kLean ? 768 : STAGE;
+    constexpr int kSlots = kLean ? HCAP / 2 : HCAP;
     constexpr int kHBits = kSlots == 2048 ? 11 : 10;
-    constexpr int kFBits = kHalf ? 10 : 8;
-    static_assert(kSlots == (1 << kHBits) && kFilterWords == 256, "set and filter sizes");
+    constexpr int kFBits = kLean ? 9 : 8;
+    static_assert(kSlots == (1 << kHBits) && kFilterWords == 256 && kStage % (32 * kTestU) == 0, "shared-memory layout");
+    using Smem = ThinSmem<KCAP, HCAP, STAGE>;
+    static_assert(!kLean || offsetof(Smem, arr) >= 4 * (2 * kStage + kSlots + (1 << kFBits)),
+                  "the lean layout fits in front of the rest");
     constexpr int ZCAP = kSlots / 2;  // entries gathered into the frontier (with repeats)
-    uint32_t* const F = kHalf ? reinterpret_cast<uint32_t*>(S.H + kSlots) : S.F;
+    int32_t* const stage = reinterpret_cast<int32_t*>(&S);  // the struct's first member
+    int32_t* const H = kLean ? stage + 2 * kStage : S.H;
+    uint32_t* const F = kLean ? reinterpret_cast<uint32_t*>(H + kSlots) : S.F;
     const int lane = lane_id();
     const int r = warp_replica_of_agent(A.rep, A.R, a);
     const Replica& rp = A.rep[r];
@@ -334,7 +341,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
     B.bc = A.bcol + rp.bbase;
     B.hslot = A.hslot + rp.nbase;
     B.hmask = reinterpret_cast<const unsigned long long*>(A.hmask) + rp.nbase * kMaskWords;
-    B.H = S.H;
+    B.H = H;
     B.G = nullptr;
     B.X = &S.aux;
     B.hbits = kHBits;
@@ -354,7 +361,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
     for (int w = 0; w < kMaskWords; ++w) ha.w[w] = 0ull;
     const int na = boost ? rp.anchors : 0;
     if (boost) {
-        for (int q = lane; q < kSlots / 4; q += 32) reinterpret_cast<int4*>(S.H)[q] = make_int4(-1, -1, -1, -1);
+        for (int q = lane; q < kSlots / 4; q += 32) reinterpret_cast<int4*>(H)[q] = make_int4(-1, -1, -1, -1);
         for (int q = lane; q < (1 << kFBits) / 4; q += 32) reinterpret_cast<int4*>(F)[q] = make_int4(0, 0, 0, 0);
         const u32x4 xa = draw(A.seed, kStreamAnchor, rep, ep, unit, 0);
         auto anchor = [&](int i) -> int {
@@ -449,7 +456,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
         };
         if (lane < na) {
             const int x = anchor(lane & 3);
-            hash_insert(S.H, kHBits, x);
+            hash_insert(H, kHBits, x);
             filter_insert<kFBits>(F, x);
             add_mask(x);
         }
@@ -484,7 +491,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
             for (int u = 0; u < 2; ++u) {
                 if (!ok[u]) continue;
                 if (ih[u] == 1) {
-                    hash_insert(S.H, kHBits, v[u]);
+                    hash_insert(H, kHBits, v[u]);
                     filter_insert<kFBits>(F, v[u]);
                 } else if (GENERAL && ih[u] == 2) {
                     ghash_insert(G, v[u]);
@@ -567,7 +574,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
             const int64_t jf0 = B.fo[j], jf1 = B.fo[j + 1];
             int64_t jb0, jb1;
             bspan(B.br, j, jb0, jb1);
-            if (GENERAL ? in_z(B, j) : hash_contains(S.H, kHBits, j)) {
+            if (GENERAL ? in_z(B, j) : hash_contains(H, kHBits, j)) {
                 mem = true;
             } else if (hs >= 0) {
                 mem = (B.X->hm[hs >> 6] >> (hs & 63)) & 1ull;
@@ -618,7 +625,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
             __syncwarp();
             if (lane == 0) mbar_expect_tx(&S.bar[buf], total);
             __syncwarp();
-            if (len) bulk_g2s(&S.stage[buf][s0], wsrc + (c0 + s0 - wx), (uint32_t)len * 4u, &S.bar[buf]);
+            if (len) bulk_g2s(stage + buf * kStage + s0, wsrc + (c0 + s0 - wx), (uint32_t)len * 4u, &S.bar[buf]);
             return true;
         };
         // chunks are double-buffered: chunk c+1 is in flight while chunk c is tested
@@ -645,7 +652,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
                 if (armed) mbar_wait(&S.bar[buf ^ 1], (phase >> (buf ^ 1)) & 1u);
                 return false;
             }
-            const int32_t* stg = S.stage[buf];
+            const int32_t* stg = stage + buf * kStage;
             // The chunk is tested flat, kTestU entries per lane and step, whatever row they belong
             // to; a hit is then given to the lane whose window holds it, which keeps the row's first
             // one, if the entry is the row's own (not window padding).  Entries of
@@ -675,7 +682,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
                     bool hit = false;
                     if (q < nq) {  // stale entries may hold any value: only node ids reach the masks
                         const int32_t v = stg[q];
-                        hit = simple ? hash_contains(S.H, kHBits, v) : (uint32_t)v < (uint32_t)n && in_z(B, v);
+                        hit = simple ? hash_contains(H, kHBits, v) : (uint32_t)v < (uint32_t)n && in_z(B, v);
                     }
                     for (unsigned m = __ballot_sync(kFull, hit); m; m &= m - 1u) {
                         const int qh = __shfl_sync(kFull, q, __ffs(m) - 1);

@@ -731,9 +731,9 @@ def test_attribute_text_at_tile_edges(gpu, n):
 
 
 @pytest.mark.parametrize("small_hash", [0, 1])
-@pytest.mark.parametrize("lo,hi", [(248, 264), (502, 522), (1016, 1034)])
+@pytest.mark.parametrize("lo,hi", [(248, 264), (502, 522), (758, 778), (1016, 1034), (1526, 1546)])
 def test_membership_scan_around_step_and_chunk_sizes(gpu, lo, hi, small_hash):
-    """Candidate rows of about one scan step (256 entries), one stage buffer (512 or 1,024) and two."""
+    """Candidate rows of about one scan step (256 entries), one stage buffer (512, 768 or 1,024) and two."""
     g = _popular_seed(20_000, 900, lo, hi, seed=9)
     prm = PAParams(alpha=1.0, tau=5.0, gamma=1.0, beta=6.0, mean_out_degree=20.0,
                    growth_rate=0.0, fixed_new_nodes=250, num_anchors=3)
