@@ -209,7 +209,7 @@ struct Arena {
     int32_t* anchors_out;      // [agent cap][4] anchors of each agent, or null (record_trace)
     int32_t* big_list;         // [agent cap]
     int32_t* heavy_list;       // [agent cap] agents with a hub or a large frontier (k <= kKSmall)
-    int32_t* heavy_mark;       // [agent cap] 1 when the agent is on heavy_list
+    int32_t* heavy_mark;       // [agent cap] 1 when the agent is heavy (on heavy_list where k <= kKSmall)
     int32_t* zbig;             // [agent-kernel warp slots][1 << kGBits] rows of anchors too large for H
     int32_t* rc_big_id;        // [kRcBigCap][kKMax] sorted top of each listed refcompat agent's 2-hop stream
     long long* rc_big_meta;    // [kRcBigCap][3] entries, rows, elements of that stream

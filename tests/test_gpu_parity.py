@@ -800,3 +800,19 @@ def test_long_appended_rows(gpu, n0, delta, deg):
         og.pa_epoch()
         assert og.degrees()[0][:n0].max() > 256
         _compare_state(eng, og)
+
+
+@pytest.mark.parametrize("n0,lam,pareto", [(3000, 90.0, False), (900, 130.0, False), (20_000, 70.0, True)])
+def test_large_out_degrees_lean_and_heavy(gpu, n0, lam, pareto):
+    """Out-degrees past 64 with anchor rows on both sides of the shared frontier's 512 entries."""
+    g = W.pareto_seed(n0, mean_indeg=60.0, seed=6) if pareto else W.plain_pa_seed(n0, 80, seed=6)
+    prm = PAParams(mean_out_degree=lam, growth_rate=0.0, fixed_new_nodes=150)
+    with GrowthEngine(seed=19, record_trace=True) as eng:
+        eng.load_graph(g.pub, g.fitness, g.src, g.dst, prm, planned_epochs=2)
+        og = _oracle_for(g, prm, 19)
+        for _ in range(2):
+            eng.grow_epoch()
+            og.pa_epoch()
+            assert eng.stats()["adj_scanned"] == og.stats()["adj_scanned"]
+            np.testing.assert_array_equal(eng.arrivals(), og.arrivals())
+        _compare_state(eng, og)
