@@ -90,6 +90,15 @@ struct Checkpoint {
     int64_t chunks = 0;
 };
 
+// What the launches of a captured run hold by value: the arena (buffers, capacities, outputs, tuning), the
+// first epoch, and every epoch's agents, which set the grids.
+struct RunKey {
+    int64_t epoch0 = -1;
+    std::vector<int64_t> agents;
+    std::vector<char> arena;
+    bool operator==(const RunKey& o) const { return epoch0 == o.epoch0 && agents == o.agents && arena == o.arena; }
+};
+
 }  // namespace
 
 struct pg_ctx {
@@ -152,11 +161,10 @@ struct pg_ctx {
     cudaEvent_t tev[2] = {};          // pg_timer_start / pg_timer_stop
     cudaEvent_t lev[2] = {};          // around each likelihood pass
     int64_t launches = 0;             // kernels enqueued by the last run
-    // CUDA graph of a multi-epoch run
+    // CUDA graph of a multi-epoch run, and what its launches hold by value (RunKey): it is launched again
+    // for a run that would hold the same
     cudaGraphExec_t gexec = nullptr;
-    int64_t g_epoch0 = -1;
-    int g_epochs = 0;
-    const void* g_out = nullptr;  // the output buffers a captured run writes to (baked into it)
+    RunKey g_key;
     // citation output of the current pg_run_epochs_out call (device-visible pointers; null otherwise)
     int32_t* out_src = nullptr;
     int32_t* out_dst = nullptr;
@@ -290,7 +298,8 @@ int64_t edge_bound(int64_t d, double lambda, int64_t n, int32_t kmax = 0) {
 }
 
 Arena make_arena(pg_ctx* c) {
-    Arena A{};
+    Arena A;
+    std::memset(&A, 0, sizeof(A));  // padding too: a captured run is known by these bytes
     A.rep = c->rep.p;
     A.R = c->R;
     A.ntiles = (int32_t)c->T;
@@ -465,7 +474,7 @@ void free_lik(LikState& L) {
 void destroy_graph_exec(pg_ctx* c) {
     if (c->gexec) cudaGraphExecDestroy(c->gexec);
     c->gexec = nullptr;
-    c->g_epoch0 = -1;
+    c->g_key = RunKey{};
 }
 
 pg_status alloc_epoch_buffers(pg_ctx* c, int64_t agent_cap, int64_t edge_cap, int64_t tasks) {
@@ -1592,7 +1601,10 @@ pg_status pg_run_epochs(pg_ctx* c, int32_t num_epochs, int32_t use_graph, int64_
     };
     cudaGetLastError();  // errors of earlier, unrelated calls are not this run's
     if (use_graph) {
-        if (!(c->gexec && c->g_epoch0 == e0 && c->g_epochs == num_epochs && c->g_out == (const void*)c->out_src)) {
+        RunKey key{e0, agents, std::vector<char>(sizeof(Arena))};
+        const Arena A = make_arena(c);
+        std::memcpy(key.arena.data(), &A, sizeof(A));
+        if (!(c->gexec && c->g_key == key)) {
             destroy_graph_exec(c);
             cudaGraph_t graph;
             PG_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -1606,9 +1618,7 @@ pg_status pg_run_epochs(pg_ctx* c, int32_t num_epochs, int32_t use_graph, int64_
             ce = cudaGraphInstantiate(&c->gexec, graph, 0);
             cudaGraphDestroy(graph);
             if (ce != cudaSuccess) return fail(c, PG_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
-            c->g_epoch0 = e0;
-            c->g_epochs = num_epochs;
-            c->g_out = c->out_src;
+            c->g_key = std::move(key);
         }
         PG_CUDA(c, cudaGraphLaunch(c->gexec, c->stream));
     } else {
@@ -1719,6 +1729,7 @@ pg_status pg_run_epochs_out(pg_ctx* c, int32_t num_epochs, int32_t use_graph, in
     // epochs whose citations did not fit the buffers were grown all the same; the caller learns of it
     const bool short_out = c->h_st.out_short != 0;
     if (short_out) ne = (int64_t)c->h_st.out_count;
+    if (ne > capacity) return fail(c, PG_ERR_STATE, "the run wrote more citations than the buffers hold");
     if (staged && ne > 0) {
         PG_CUDA(c, cudaMemcpyAsync(src, ds, 4 * (size_t)ne, cudaMemcpyDeviceToHost, c->stream));
         PG_CUDA(c, cudaMemcpyAsync(dst, dd, 4 * (size_t)ne, cudaMemcpyDeviceToHost, c->stream));

@@ -816,3 +816,53 @@ def test_large_out_degrees_lean_and_heavy(gpu, n0, lam, pareto):
             assert eng.stats()["adj_scanned"] == og.stats()["adj_scanned"]
             np.testing.assert_array_equal(eng.arrivals(), og.arrivals())
         _compare_state(eng, og)
+
+
+def test_captured_run_with_other_outputs_and_another_start(gpu):
+    """A run repeated from a checkpoint into other buffers, shorter buffers, and from the same epoch number with
+    another number of nodes: each delivers what a run launched without a graph does."""
+    torch = pytest.importorskip("torch")
+    g = W.plain_pa_seed(3000, 8, seed=5)
+    cap = 60_000
+
+    def pinned():
+        return torch.full((cap,), -7, dtype=torch.int32).pin_memory().numpy()
+
+    src, d1, d2 = pinned(), pinned(), pinned()
+    with GrowthEngine(seed=6) as eng:
+        eng.load_graph(g.pub, g.fitness, g.src, g.dst, PAParams(mean_out_degree=12.0, growth_rate=0.05, fixed_new_nodes=0),
+                       planned_epochs=8)
+        eng.reserve(20_000, 200_000)
+        eng.checkpoint()
+        ne, _ = eng.run_epochs_out(4, (src, d1), use_graph=False)
+        want = (src[:ne].copy(), d1[:ne].copy())
+        for dst, other in ((d1, d2), (d2, d1)):
+            for a in (src, d1, d2):
+                a[:] = -7
+            eng.restore()
+            assert eng.run_epochs_out(4, (src, dst))[0] == ne
+            np.testing.assert_array_equal(src[:ne], want[0])
+            np.testing.assert_array_equal(dst[:ne], want[1])
+            assert (other == -7).all() and (dst[ne:] == -7).all()
+        buf = (np.full(cap, -7, np.int32), np.full(cap, -7, np.int32))
+        for n in (ne, ne - 1, cap, ne // 2):
+            buf[0][:], buf[1][:] = -7, -7
+            eng.restore()
+            if n >= ne:
+                assert eng.run_epochs_out(4, (buf[0][:n], buf[1][:n]))[0] == ne
+                np.testing.assert_array_equal(buf[1][:ne], want[1])
+            else:
+                with pytest.raises(PGError) as err:
+                    eng.run_epochs_out(4, (buf[0][:n], buf[1][:n]))
+                assert err.value.status == PG_ERR_CAPACITY
+            assert (buf[0][n:] == -7).all() and (buf[1][n:] == -7).all()
+        for delta in (20, 700):
+            runs = []
+            for use_graph in (True, False):
+                eng.restore()
+                eng.run_er_epochs(2, delta, 2e-3)
+                m0 = eng.counts()[1]
+                k = eng.run_epochs(2, use_graph=use_graph)
+                runs.append(eng.edges(m0, k))
+            np.testing.assert_array_equal(runs[0][0], runs[1][0])
+            np.testing.assert_array_equal(runs[0][1], runs[1][1])

@@ -1,0 +1,139 @@
+"""The library's host code on a CUDA runtime of host memory (fake_runtime.cpp), in place of a GPU: what a
+captured run may be used for again, what a failed allocation leaves behind, and what the memory that the
+library keeps does to later calls.  The kernels do nothing but keep an epoch's counts (every agent cites
+itself), so results of the sampling are not looked at here."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+import paragraph_gb300 as pg
+from paragraph_gb300 import PG_ERR_CAPACITY, GrowthEngine, PAParams, PGError
+from paragraph_gb300.build import PKG, ROOT, build_library, nvcc
+
+
+@pytest.fixture(scope="module")
+def fake(built, tmp_path_factory):
+    d = tmp_path_factory.mktemp("fake")
+    cuda = Path(nvcc()).resolve().parents[1] / "include"
+    if not list((PKG / "_build").glob("*.o")):
+        build_library(force=True)
+    objs = sorted(str(p) for p in (PKG / "_build").glob("*.o"))
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-Wl,--no-undefined",
+                    "-I", str(cuda), "-I", str(ROOT / "include"), "-o", str(d / "libfake.so"),
+                    str(ROOT / "tests" / "fake_runtime.cpp"), *objs, "-lpthread"], check=True)
+    lib = pg.load_library(d / "libfake.so")
+    lib.fake_reset.argtypes = [C.c_int64, C.c_int32]
+    lib.fake_fail_in.argtypes = [C.c_int64]
+    lib.fake_hold.argtypes = [C.c_int64]
+    for f in ("fake_mallocs", "fake_memory_queries", "fake_free_bytes", "fake_hold"):
+        getattr(lib, f).restype = C.c_int64
+    lib.fake_launches.argtypes = [C.c_char_p]
+    lib.fake_launches.restype = C.c_int32
+    lib.fake_dependent_range.argtypes = [C.c_char_p, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
+    lib.fake_page_locked.argtypes = [C.c_int64]
+    lib.fake_page_locked.restype = C.c_void_p
+    lib.fake_page_locked_free.argtypes = [C.c_void_p]
+    return lib
+
+
+@pytest.fixture
+def host(fake, monkeypatch):
+    """Engines made in the test run on the fake runtime."""
+    monkeypatch.setattr(pg, "_lib", fake)
+    fake.fake_reset(64 << 30, 152)
+    return fake
+
+
+def _engine(n=1000, new=40, epochs=8, **kw):
+    eng = GrowthEngine(seed=1, **kw)
+    eng.load_graph(np.zeros(n, np.int32), np.ones(n, np.float32), np.zeros(0, np.int32), np.zeros(0, np.int32),
+                   PAParams(fixed_new_nodes=new, growth_rate=0.0), planned_epochs=epochs)
+    return eng
+
+
+class _PageLocked:
+    def __init__(self, lib, count):
+        self.lib, self.p = lib, lib.fake_page_locked(4 * count)
+        self.a = np.ctypeslib.as_array((C.c_int32 * count).from_address(self.p))
+        self.a[:] = -7
+
+    def free(self):
+        self.a = None
+        self.lib.fake_page_locked_free(self.p)
+
+
+# ---------------------------------------------------------------- captured runs
+def test_captured_run_follows_its_output_buffers(host):
+    """A run repeated from a checkpoint with the same page-locked sources and other targets writes the
+    targets it was given."""
+    bufs = [_PageLocked(host, 1000) for _ in range(3)]
+    src, d1, d2 = (b.a for b in bufs)
+    with _engine() as eng:
+        eng.checkpoint()
+        ne, counts = eng.run_epochs_out(3, (src, d1))
+        assert ne == 120 and (d1[:120] == np.arange(1000, 1120)).all() and counts.sum() == 120
+        d1[:] = -7
+        eng.restore()
+        ne, _ = eng.run_epochs_out(3, (src, d2))
+        assert ne == 120 and (d2[:120] == np.arange(1000, 1120)).all()
+        assert (d1 == -7).all()
+    del src, d1, d2
+    for b in bufs:
+        b.free()
+
+
+@pytest.mark.parametrize("page_locked", [False, True])
+def test_captured_run_follows_its_capacity(host, page_locked):
+    """Buffers of another length from the same checkpoint: too short is reported and nothing is written past
+    the end, long enough again is no error."""
+    bufs = [_PageLocked(host, 1000) for _ in range(2)] if page_locked else []
+    s, d = (b.a for b in bufs) if page_locked else (np.full(1000, -7, np.int32), np.full(1000, -7, np.int32))
+    with _engine() as eng:
+        eng.checkpoint()
+        for cap in (120, 100, 1000, 40, 39, 120):
+            s[:], d[:] = -7, -7
+            if cap >= 120:
+                assert eng.run_epochs_out(3, (s[:cap], d[:cap]))[0] == 120
+                done = 120
+            else:
+                with pytest.raises(PGError) as err:
+                    eng.run_epochs_out(3, (s[:cap], d[:cap]))
+                assert err.value.status == PG_ERR_CAPACITY
+                done = cap // 40 * 40
+            for a in (s, d):
+                assert (a[:done] == np.arange(1000, 1000 + done)).all() and (a[done:] == -7).all()
+            eng.restore()
+    del s, d
+    for b in bufs:
+        b.free()
+
+
+def test_captured_run_follows_the_graph_it_starts_from(host):
+    """The same epoch number reached with another number of nodes: the captured run was for other epochs'
+    agents."""
+    with _engine(epochs=12) as eng:
+        eng.set_params(PAParams(growth_rate=0.05, fixed_new_nodes=0))
+        eng.reserve(6000, 6000)
+        eng.checkpoint()
+        eng.run_er_epochs(3, 10, 1e-3)
+        first = eng.run_epochs(2)
+        eng.restore()
+        eng.run_er_epochs(3, 400, 1e-3)
+        n0 = eng.counts()[0]
+        again = eng.run_epochs(2)
+        assert again == eng.counts()[0] - n0 > first
+
+
+def test_captured_run_is_used_again(host):
+    """Nothing changed: the run is not captured a second time."""
+    with _engine() as eng:
+        eng.checkpoint()
+        out = (np.empty(500, np.int32), np.empty(500, np.int32))
+        eng.run_epochs_out(3, out)
+        eng.restore()
+        host.fake_clear_launches()
+        eng.run_epochs_out(3, out)
+        assert host.fake_launches(b"k_epoch_begin") == 0
