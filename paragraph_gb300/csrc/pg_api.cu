@@ -2043,6 +2043,19 @@ pg_status pg_checkpoint(pg_ctx* c) {
     if (c->poisoned) return fail(c, PG_ERR_STATE, "state is inconsistent after a device error");
     Checkpoint& k = c->ckpt;
     cudaStream_t s = c->stream;
+    // the backward entries in use per replica (the device bump pointers)
+    std::vector<Replica> dr((size_t)c->R);
+    PG_CUDA(c, cudaMemcpyAsync(dr.data(), c->rep.p, sizeof(Replica) * (size_t)c->R, cudaMemcpyDeviceToHost, s));
+    PG_CUDA(c, cudaStreamSynchronize(s));
+    std::vector<int64_t> b_top((size_t)c->R, 0);
+    for (int r = 0; r < c->R; ++r) {
+        const int64_t top = (int64_t)dr[(size_t)r].b_top;
+        if (top < 0 || top > c->hrep[(size_t)r].b_cap) return fail(c, PG_ERR_STATE, "backward region state out of range");
+        b_top[(size_t)r] = top;
+    }
+    // from here on the arrays of an earlier checkpoint are overwritten: nothing to restore until all is saved
+    k.valid = false;
+    k.b_top = std::move(b_top);
     if (k.pub.n != c->S) {
         PG_CUDA(c, dalloc(k.pub, c->S));
         PG_CUDA(c, dalloc(k.indeg, c->S));
@@ -2054,16 +2067,6 @@ pg_status pg_checkpoint(pg_ctx* c) {
     }
     if (k.fwd_col.n != c->M) PG_CUDA(c, dalloc(k.fwd_col, c->M));
     if (k.bcol.n != c->B) PG_CUDA(c, dalloc(k.bcol, c->B));
-    // the backward entries in use per replica (the device bump pointers)
-    std::vector<Replica> dr((size_t)c->R);
-    PG_CUDA(c, cudaMemcpyAsync(dr.data(), c->rep.p, sizeof(Replica) * (size_t)c->R, cudaMemcpyDeviceToHost, s));
-    PG_CUDA(c, cudaStreamSynchronize(s));
-    k.b_top.assign((size_t)c->R, 0);
-    for (int r = 0; r < c->R; ++r) {
-        const int64_t top = (int64_t)dr[(size_t)r].b_top;
-        if (top < 0 || top > c->hrep[(size_t)r].b_cap) return fail(c, PG_ERR_STATE, "backward region state out of range");
-        k.b_top[(size_t)r] = top;
-    }
     const cudaMemcpyKind d2d = cudaMemcpyDeviceToDevice;
     if (c->cfg.weight_model == PG_WEIGHTS_REFCOMPAT) {
         if (k.rc_lag.n != c->S) {
@@ -2084,11 +2087,11 @@ pg_status pg_checkpoint(pg_ctx* c) {
     PG_CUDA(c, cudaMemset2DAsync(reinterpret_cast<char*>(k.rep.p) + offsetof(Replica, hub_valid), sizeof(Replica), 0,
                                  sizeof(int32_t), (size_t)c->R, s));
     std::vector<CopySeg> segs;
-    k.chunks = 0;
+    int64_t chunks = 0;
     auto put_back = [&](void* dst, const void* src, size_t bytes) {
         if (!bytes) return;
-        segs.push_back(CopySeg{static_cast<const char*>(src), static_cast<char*>(dst), (int64_t)bytes, k.chunks});
-        k.chunks += ((int64_t)bytes + kCopyChunk - 1) / kCopyChunk;
+        segs.push_back(CopySeg{static_cast<const char*>(src), static_cast<char*>(dst), (int64_t)bytes, chunks});
+        chunks += ((int64_t)bytes + kCopyChunk - 1) / kCopyChunk;
     };
     const size_t S = (size_t)c->S;
     static_assert(sizeof(Replica) % 4 == 0 && sizeof(BRow) % 4 == 0, "whole words");
@@ -2112,10 +2115,11 @@ pg_status pg_checkpoint(pg_ctx* c) {
         put_back(c->fwd_col.p + h.ebase, k.fwd_col.p + h.ebase, 4 * (size_t)h.m);
         put_back(c->bcol.p + h.bbase, k.bcol.p + h.bbase, 4 * (size_t)top);
     }
-    k.num_segs = (int)segs.size();
     if (k.segs.n < (int64_t)segs.size()) PG_CUDA(c, dalloc(k.segs, (int64_t)segs.size()));
     PG_CUDA(c, cudaMemcpyAsync(k.segs.p, segs.data(), sizeof(CopySeg) * segs.size(), cudaMemcpyHostToDevice, s));
     PG_CUDA(c, cudaStreamSynchronize(s));
+    k.num_segs = (int)segs.size();
+    k.chunks = chunks;
     k.epoch = c->epoch;
     k.hrep = c->hrep;
     k.valid = true;

@@ -32,6 +32,7 @@ size_t g_pool_used = 0, g_pool_reserved = 0;
 uint64_t g_pool_keep = 0;
 int64_t g_fail_in = -1;        // device allocations from now until one fails; < 0: none
 int64_t g_mallocs = 0, g_queries = 0;
+int64_t g_faults = 0;          // kernels that would have read a null table
 int g_sms = 152;
 std::map<uintptr_t, Block> g_blocks;
 std::map<const void*, std::string> g_kernels;
@@ -113,6 +114,10 @@ void epoch_end(const Arena& A, int64_t agents) {
     if (A.out_src && (int64_t)A.st->out_count + A.st->agents <= A.out_cap) A.st->out_count += (unsigned long long)A.st->agents;
 }
 void copy_segments(const pg::CopySeg* s, int num, pg::EpochState* st) {
+    if (!s) {
+        ++g_faults;
+        return;
+    }
     for (int i = 0; i < num; ++i) {
         if (s[i].src)
             memcpy(s[i].dst, s[i].src, (size_t)s[i].bytes);
@@ -155,11 +160,12 @@ void fake_reset(int64_t total_bytes, int32_t sms) {
     g_total = (size_t)total_bytes;
     g_sms = sms;
     g_fail_in = -1;
-    g_mallocs = g_queries = 0;
+    g_mallocs = g_queries = g_faults = 0;
     g_launches.clear();
 }
 void fake_fail_in(int64_t n) { g_fail_in = n; }
 int64_t fake_mallocs(void) { return g_mallocs; }
+int64_t fake_faults(void) { return g_faults; }
 int64_t fake_memory_queries(void) { return g_queries; }
 int64_t fake_free_bytes(void) { return (int64_t)(g_total - g_used); }
 int64_t fake_hold(int64_t bytes) {  // memory of another user of the device; negative: given back

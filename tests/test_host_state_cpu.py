@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import paragraph_gb300 as pg
-from paragraph_gb300 import PG_ERR_CAPACITY, GrowthEngine, PAParams, PGError
+from paragraph_gb300 import PG_ERR_CAPACITY, PG_ERR_STATE, GrowthEngine, PAParams, PGError
 from paragraph_gb300.build import PKG, ROOT, build_library, nvcc
 
 
@@ -28,7 +28,7 @@ def fake(built, tmp_path_factory):
     lib.fake_reset.argtypes = [C.c_int64, C.c_int32]
     lib.fake_fail_in.argtypes = [C.c_int64]
     lib.fake_hold.argtypes = [C.c_int64]
-    for f in ("fake_mallocs", "fake_memory_queries", "fake_free_bytes", "fake_hold"):
+    for f in ("fake_mallocs", "fake_faults", "fake_memory_queries", "fake_free_bytes", "fake_hold"):
         getattr(lib, f).restype = C.c_int64
     lib.fake_launches.argtypes = [C.c_char_p]
     lib.fake_launches.restype = C.c_int32
@@ -137,3 +137,36 @@ def test_captured_run_is_used_again(host):
         host.fake_clear_launches()
         eng.run_epochs_out(3, out)
         assert host.fake_launches(b"k_epoch_begin") == 0
+
+
+# ---------------------------------------------------------------- checkpoints
+def test_failed_checkpoint_leaves_nothing_to_restore(host):
+    """A second checkpoint that fails on the way has overwritten parts of the first: a restore is refused,
+    and the next whole checkpoint is restored."""
+    with _engine() as eng:
+        eng.checkpoint()  # no citations yet: one copied range fewer than later
+        eng.run_epochs(2)
+        host.fake_fail_in(0)
+        with pytest.raises(PGError):
+            eng.checkpoint()
+        with pytest.raises(PGError) as err:
+            eng.restore()
+        assert err.value.status == PG_ERR_STATE
+        assert host.fake_faults() == 0
+        host.fake_fail_in(-1)
+        eng.checkpoint()
+        at = eng.counts()
+        eng.run_epochs(1)
+        eng.restore()
+        assert eng.counts() == at == (1080, 80)
+
+
+def test_refused_checkpoint_keeps_the_earlier_one(host):
+    with GrowthEngine(seed=1) as eng:
+        with pytest.raises(PGError):
+            eng.checkpoint()
+    with _engine() as eng:
+        eng.checkpoint()
+        eng.run_epochs(1)
+        eng.restore()
+        assert eng.counts() == (1000, 0)
