@@ -705,7 +705,7 @@ pg_status upload_arena(pg_ctx* c, std::vector<HostRep>& reps, const std::vector<
         return fail(c, PG_ERR_CUDA, "out of device memory for the graph");
     }
     if (c->cfg.weight_model == PG_WEIGHTS_REFCOMPAT) {
-        if (!c->rc_big_id.p) {
+        if (!c->rc_ticket.p) {  // the last of them: a load that failed among them starts over
             PG_CUDA(c, dalloc(c->rc_big_id, (int64_t)kRcBigCap * kKMax));
             PG_CUDA(c, dalloc(c->rc_big_meta, (int64_t)kRcBigCap * 3));
             PG_CUDA(c, dalloc(c->rc_part, kRcBigCap));

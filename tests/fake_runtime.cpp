@@ -32,7 +32,7 @@ size_t g_pool_used = 0, g_pool_reserved = 0;
 uint64_t g_pool_keep = 0;
 int64_t g_fail_in = -1;        // device allocations from now until one fails; < 0: none
 int64_t g_mallocs = 0, g_queries = 0;
-int64_t g_faults = 0;          // kernels that would have read a null table
+int64_t g_faults = 0;          // kernels that would have read through a null pointer
 int g_sms = 152;
 std::map<uintptr_t, Block> g_blocks;
 std::map<const void*, std::string> g_kernels;
@@ -141,6 +141,10 @@ cudaError_t launch(const void* f, dim3 grid, dim3 block, void** args, int attrs)
         const int64_t agents = *(int64_t*)args[1];
         const bool end = is("k_epoch_end");
         submit([=]() { end ? epoch_end(A, agents) : copy_out(A, agents); });
+    } else if (is("k_rc_big")) {
+        const Arena& A = *(Arena*)args[0];
+        if (!A.rc_big_id || !A.rc_big_meta || !A.rc_part || !A.rc_item || !A.rc_item_list || !A.rc_item_meta || !A.rc_ticket)
+            ++g_faults;
     } else if (is("k_copy_segments")) {
         const pg::CopySeg* s = *(pg::CopySeg**)args[0];
         const int num = *(int*)args[1];

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import paragraph_gb300 as pg
-from paragraph_gb300 import PG_ERR_CAPACITY, PG_ERR_STATE, GrowthEngine, PAParams, PGError
+from paragraph_gb300 import PG_ERR_CAPACITY, PG_ERR_STATE, PG_WEIGHTS_REFCOMPAT, GrowthEngine, PAParams, PGError, RCParams
 from paragraph_gb300.build import PKG, ROOT, build_library, nvcc
 
 
@@ -170,3 +170,28 @@ def test_refused_checkpoint_keeps_the_earlier_one(host):
         eng.run_epochs(1)
         eng.restore()
         assert eng.counts() == (1000, 0)
+
+
+# ---------------------------------------------------------------- failed loads
+@pytest.mark.parametrize("weight_model", [0, PG_WEIGHTS_REFCOMPAT])
+def test_load_after_a_failed_load(host, weight_model):
+    """Whichever device allocation of a load fails, the next load has everything its epochs use."""
+    seed = [np.zeros(500, np.int32), np.ones(500, np.float32), np.zeros(0, np.int32), np.zeros(0, np.int32)]
+    prm = PAParams(fixed_new_nodes=20, growth_rate=0.0)
+    failed = 0
+    for n in range(100):
+        with GrowthEngine(seed=1, weight_model=weight_model) as eng:
+            host.fake_fail_in(n)
+            try:
+                eng.load_graph(*seed, prm, planned_epochs=2)
+            except PGError:
+                failed += 1
+            else:
+                break
+            finally:
+                host.fake_fail_in(-1)
+            eng.load_graph(*seed, prm, planned_epochs=2)
+            if weight_model:
+                eng.rc_configure(RCParams(growth_rate=0.04), np.full(10, 5), np.full(4, 0.25))
+            assert eng.run_epochs(2) >= 40
+    assert failed >= (8 if weight_model else 1) and host.fake_faults() == 0
