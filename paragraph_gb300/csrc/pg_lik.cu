@@ -354,30 +354,6 @@ __device__ __forceinline__ DF df_recip(const DF a) {
     return df_add(DF{r, 0.0f}, df_mulf(e, r));
 }
 
-// log a for 2^-16 < a < 1 to about 2e-11: a = 2^e m, m in (sqrt(2)/2, sqrt(2)], log m = 2 atanh(s) =
-// 2 s (1 + s^2/3 + s^4/5 + ...), s = (m - 1) / (m + 1) in [-0.172, 0.172]; the first two terms in
-// double-float, the rest (below 2e-4 of the sum) in fp32.
-__device__ __forceinline__ DF df_log(const DF a) {
-    int e = (int)(__float_as_uint(a.h) >> 23) - 127;
-    float sc = __int_as_float((127 - e) << 23);
-    if (a.h * sc > kSqrt2F) {
-        sc *= 0.5f;
-        e += 1;
-    }
-    const DF m{a.h * sc, a.l * sc};
-    const DF s = df_mul(df_add(m, DF{-1.0f, 0.0f}), df_recip(df_add(m, DF{1.0f, 0.0f})));
-    const DF z = df_mul(s, s);
-    float p = 1.0f / 13.0f;
-    p = __fmaf_rn(p, z.h, 1.0f / 11.0f);
-    p = __fmaf_rn(p, z.h, 1.0f / 9.0f);
-    p = __fmaf_rn(p, z.h, 1.0f / 7.0f);
-    p = __fmaf_rn(p, z.h, 1.0f / 5.0f);
-    constexpr float third = 1.0f / 3.0f;
-    const DF t = df_add(df_mul(z, DF{third, (float)(1.0 / 3.0 - (double)third)}), DF{z.h * z.h * p, 0.0f});
-    const DF l = df_add(s, df_mul(s, t));
-    return df_add(DF{2.0f * l.h, 2.0f * l.l}, df_mulf(DF{kLn2HiF, kLn2LoF}, (float)e));
-}
-
 // log(1 - u) for u in [0, 0.5): -2 atanh(t), t = u / (2 - u) in [0, 1/3), by the odd Taylor series
 // of atanh, t + t^3/3 + ... + t^17/17 (truncation below 1e-9 relative at t = 1/3).
 __device__ __forceinline__ float log1m_pg(float u) {
@@ -672,8 +648,6 @@ __device__ __forceinline__ void lik_agent(const LikTrace& T, const LikBatch& P, 
         // the sums of x_i (its two parts), of log(1 - u_i) and of P compensated in fp32
         const double logZ = log_pg(Z);
         const float invZ = 1.0f / (float)Z, betaf = (float)beta;
-        const DF Zd = df_of(Z), invZd = df_recip(Zd);
-        DF far{0.0f, 0.0f};
         Kahan sh, sl, slr, pc;
         double lr_far = 0.0;
         int n_in = 0;
@@ -686,20 +660,15 @@ __device__ __forceinline__ void lik_agent(const LikTrace& T, const LikBatch& P, 
             const float u = (pc.s - pc.c) * invZ;
             if (u < 0.5f)
                 kadd(slr, log1m_pg(u));
-            else {  // 1 - u is small: from the difference in double-float, or FP64 when little is left
-                const DF left = df_mul(df_add(Zd, df_norm(-pc.s, pc.c)), invZd);
-                if (left.h > 0x1p-16f)
-                    far = df_add(far, df_log(left));
-                else
-                    lr_far += log_pg(Z - kval(pc)) - logZ;
-            }
+            else  // 1 - u is small: log(Z - P) - log Z from the FP64 difference
+                lr_far += log_pg(Z - kval(pc)) - logZ;
             kadd(sh, x2.h);
             kadd(sl, x2.l);
             n_in += in ? 1 : 0;
             kadd(pc, W);
         }
         const double l = (kval(sh) + kval(sl)) * kLn2d + (double)n_in * lbe -
-                         ((double)k * logZ + kval(slr) + (df_val(far) + lr_far));
+                         ((double)k * logZ + kval(slr) + lr_far);
         P.out[a * P.B + b] = l;
     } else {
         // g_k = sum_i [gk_i - (dZ_k - dP_k,i) / D_i],  D_i = Z_a - P_i,  dP_k,i = sum_{j<i} W_j gk_j

@@ -8,11 +8,13 @@ points drawn from the parameter ranges.  At the generating point theta* the grad
 zero -- the trace was drawn there -- so errors that do not average out over the trace are a larger
 share of it: the default arithmetic (special-function-unit exp2, pairwise ball sums) is held to
 1e-5 there, the exact arithmetic (pg_lik_set_exact_exp2) to 1e-6 like every other point."""
+import math
+
 import numpy as np
 import pytest
 
 import oracle as O
-from paragraph_gb300 import GrowthEngine, PGError
+from paragraph_gb300 import GrowthEngine, PGError, TraceInput
 from paragraph_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -222,3 +224,32 @@ def test_weight_table_in_several_parts(gpu):
     tr = W.grow_trace(g, prm, 4, seed=7)
     balls, rows = _check_against_oracle(tr, W.theta_batch(3, seed=9))
     assert 8 * balls >= rows
+
+
+def _unit_weight_trace(nodes, cites):
+    """`nodes` papers without citations, of fitness 1, published in the epoch itself: every weight is 1, the
+    first paper is every agent's only anchor and its ball, and one agent cites papers 0, 1, ... in order."""
+    n = nodes + 1
+    return TraceInput(pub=np.zeros(n, np.int32), fitness=np.ones(n, np.float32), seed_src=np.zeros(0, np.int32),
+                      seed_dst=np.zeros(0, np.int32), epoch_nodes=np.array([nodes, n]), epoch_t=np.array([0]),
+                      anchors=np.array([[0, -1, -1, -1]], np.int32), cite_off=np.array([0, cites]),
+                      cites=np.arange(cites, dtype=np.int32), num_anchors=1)
+
+
+@pytest.mark.parametrize("exact", [False, True])
+@pytest.mark.parametrize("nodes,cites", [(3, 2), (3, 3), (40, 30), (1000, 60)])
+def test_drawn_weight_above_half_in_64_bits(gpu, nodes, cites, exact):
+    """Once more than half of an agent's weight is drawn, log(1 - P / Z) is taken in 64 bits.  Here Z and every P
+    are whole numbers and the first citation, of weight beta > nodes, is all that comes before: l = log beta -
+    sum_i log D_i, D = Z, then nodes - 1, nodes - 2, ...  Each log is below 12 and good to two ulp (4e-15), twice
+    per citation, and every addition rounds a total below 12 per citation."""
+    beta = np.random.default_rng(nodes + cites).integers(2 * nodes, 50_000, 40).astype(np.float64)
+    pts = np.stack([np.ones(40), np.full(40, 5.0), np.ones(40), beta], axis=1)
+    with GrowthEngine(seed=1) as eng:
+        eng.set_lik_exact_exp2(exact)
+        eng.load_trace(_unit_weight_trace(nodes, cites))
+        ll = np.concatenate([eng.loglik(pts), eng.loglik(pts[:7])])
+    beta = np.concatenate([beta, beta[:7]])
+    left = math.fsum(math.log(nodes - i) for i in range(1, cites))
+    want = np.log(beta) - np.log(nodes - 1 + beta) - left
+    assert np.abs(ll - want).max() <= cites * (8e-15 + 2.0**-53 * 12 * cites)
