@@ -27,8 +27,8 @@
 //
 // Per launch (forward or adjoint):
 //   k_lik_global      per epoch: sum_{j<n_e} w_j (forward) or sum_j w_j g_j (adjoint), one CTA per
-//                     1024-node chunk; fp32 with every rounding error kept for 32 terms, then FP64
-//                     (fixed order, so results are reproducible).  It also writes the epochs' weight
+//                     1024-node chunk, to 64-bit accuracy (32 terms in fp32 with the roundings kept, then
+//                     FP64, in a fixed order, so results are reproducible).  It also writes the epochs' weight
 //                     table (LikBatch::wt) when the agent pass gathers from one.
 //   k_lik_global_sum  chunks -> one FP64 value per (epoch, point).
 //   k_lik_ball        (once per trace, or per chunk of agents and pass) the agent's 2-hop ball as
@@ -45,6 +45,7 @@
 //                     have fewer elements than the epochs have nodes, and where a table has no room.
 //   k_lik_sum         agents -> totals per point (fixed order).
 #include "pg_lik.cuh"
+#include "pg_sums.cuh"
 
 #include <cuda_fp16.h>
 
@@ -233,29 +234,6 @@ __device__ __forceinline__ float ex2_sfu(float x) {
 struct X2 {
     float h, l;
 };
-// a + b = s + err exactly (Knuth's two-sum; the build neither contracts nor reassociates)
-__device__ __forceinline__ float two_sum(float a, float b, float& err) {
-    const float s = a + b;
-    const float bb = s - a;
-    err = (a - (s - bb)) + (b - bb);
-    return s;
-}
-// A short sum of fp32 values or products with every rounding error accumulated beside it.
-struct ErrSum {
-    float s = 0.f, e = 0.f;
-    __device__ __forceinline__ void add(float v) {
-        float r;
-        s = two_sum(s, v, r);
-        e += r;
-    }
-    __device__ __forceinline__ void add_product(float a, float b) {
-        const float p = a * b, q = __fmaf_rn(a, b, -p);
-        float r;
-        s = two_sum(s, p, r);
-        e += r + q;
-    }
-    __device__ __forceinline__ double value() const { return (double)s + (double)e; }
-};
 // the low-order terms of the exponent: the constants' remainders times the features' high parts,
 // the constants times the features' remainders (the exact layout also carries log f's)
 template <bool EXACT>
@@ -407,9 +385,11 @@ __global__ void __launch_bounds__(kLikThreads) k_lik_global(LikTrace T, LikBatch
     const int64_t lo = (int64_t)blockIdx.x * kLikChunk;
     const int BE = P.BE, B = P.B;
     const int b = tid & (BE - 1), sub = tid / BE, nsub = kLikThreads / BE;
-    // sums of at most 32 terms as fp32 pairs with every rounding error kept (two-sums, FMA residuals),
-    // then FP64: GB300 does two FP64 operations per clock and SM, and the adjoint's four FP64
-    // operations and four conversions per weight were 2.87 ms of a 64-point pass of a 200k-node trace
+    // Sums of at most 32 terms in fp32 with their rounding errors (ErrSum: the exact sum to 64 bits), then FP64:
+    // GB300 does two FP64 operations per clock and SM, and the adjoint's four FP64 operations and four
+    // conversions per weight were 2.87 ms of a 64-point pass of a 200k-node trace, now 0.65
+    // (forward 0.34).  Terms out of ErrSum's range (weights of the batch together above 2^90 or below 2^-60)
+    // are summed in FP64.
     double s = 0.0, t0 = 0.0, t1 = 0.0, t2 = 0.0;
     if (b < B && lo < ne) {
         const LikC c = lik_c(P.pp + b * kLikPP);
@@ -417,6 +397,7 @@ __global__ void __launch_bounds__(kLikThreads) k_lik_global(LikTrace T, LikBatch
         const float4* F = T.feat + (int64_t)e * T.n;
         float* tab = P.wt ? P.wt + blockIdx.y * P.wt_n * BE + b : nullptr;
         for (int64_t j = lo + sub; j < hi;) {
+            const int64_t j0 = j;
             ErrSum ps, p0, p1, p2;
 #pragma unroll 4
             for (int q = 0; q < 32; ++q, j += nsub) {
@@ -424,17 +405,31 @@ __global__ void __launch_bounds__(kLikThreads) k_lik_global(LikTrace T, LikBatch
                 const float4 f = F[j];
                 const float w = lik_w<EXACT>(lik_x2<EXACT>(f, c));
                 if (tab) tab[j * BE] = w;
-                ps.add(w);
+                err_add(ps, w);
                 if (ADJ) {
-                    p0.add_product(w, f.y);
-                    p1.add_product(w, f.z);
-                    p2.add_product(w, f.x);
+                    err_add_product(p0, w, f.y);
+                    err_add_product(p1, w, f.z);
+                    err_add_product(p2, w, f.x);
                 }
             }
-            s += ps.value();
-            t0 += p0.value();
-            t1 += p1.value();
-            t2 += p2.value();
+            if (err_ranges_hold(ps)) {
+                s += err_value(ps);
+                t0 += err_value(p0);
+                t1 += err_value(p1);
+                t2 += err_value(p2);
+            } else {
+#pragma unroll 1
+                for (int64_t i = j0; i < j; i += nsub) {
+                    const float4 f = F[i];
+                    const double w = (double)lik_w<EXACT>(lik_x2<EXACT>(f, c));
+                    s += w;
+                    if (ADJ) {
+                        t0 = __fma_rn(w, (double)f.y, t0);
+                        t1 = __fma_rn(w, (double)f.z, t1);
+                        t2 = __fma_rn(w, (double)f.x, t2);
+                    }
+                }
+            }
         }
     }
     red[tid * 4 + 0] = s;

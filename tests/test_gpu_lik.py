@@ -253,3 +253,22 @@ def test_drawn_weight_above_half_in_64_bits(gpu, nodes, cites, exact):
     left = math.fsum(math.log(nodes - i) for i in range(1, cites))
     want = np.log(beta) - np.log(nodes - 1 + beta) - left
     assert np.abs(ll - want).max() <= cites * (8e-15 + 2.0**-53 * 12 * cites)
+
+
+@pytest.mark.parametrize("exact", [False, True])
+@pytest.mark.parametrize("fitness", [1e38, 1e-30])
+def test_weights_at_the_ends_of_the_range(gpu, fitness, exact):
+    """A hundred equal weights of 1e38, whose sum is no fp32 number, or of 1e-30: one citation of one of them has
+    log-likelihood -log 100, to the fp32 weights' accuracy (1e-7 each in the weight and its logarithm, of which the
+    second is relative to 126)."""
+    n = 101
+    tr = TraceInput(pub=np.zeros(n, np.int32), fitness=np.full(n, fitness, np.float32), seed_src=np.zeros(0, np.int32),
+                    seed_dst=np.zeros(0, np.int32), epoch_nodes=np.array([100, n]), epoch_t=np.array([0]),
+                    anchors=np.array([[0, -1, -1, -1]], np.int32), cite_off=np.array([0, 1]),
+                    cites=np.array([5], np.int32), num_anchors=1)
+    pts = np.tile([1.0, 5.0, 1.0, 1.0], (40, 1))
+    with GrowthEngine(seed=1) as eng:
+        eng.set_lik_exact_exp2(exact)
+        eng.load_trace(tr)
+        for b in (1, 8, 40):
+            assert np.abs(eng.loglik(pts[:b]) + math.log(100.0)).max() <= 2e-5
