@@ -62,27 +62,42 @@ constexpr int kTextThreads = 256;
 // Rows of the tile's edges [e0, e1), EDGES consecutive ones per thread, all kTextThreads threads.  They
 // come from the tile's own row starts: each row marks its first edge (the last of several rows that
 // start at one edge, the others being empty, is the source), and a running maximum carries the marks on.
+// Where nearly all rows are empty a tile spans a great many of them, and its edges are searched between the
+// tile's first and last row instead.  500 edges of 2M rows: sources copied out in 43 us and text in 280, where
+// walking the rows took 2,030 and 6,260; one gap of 2M rows among 1.4M edges 110 and 1,890 (2,060 and 7,750).
+// The line: from 1,024 rows to 16,384 nothing differs by 3 % at 1 to 4,000 rows per edge; with 65,536, 31,000
+// edges of 2M rows take 72 us instead of 43.
+constexpr int kMarkRows = 4096;
 template <int EDGES>
 __device__ __forceinline__ void tile_sources(const int64_t* __restrict__ fo, int64_t n, int64_t e0, int64_t e1,
                                              int64_t (&row)[EDGES]) {
     __shared__ int s_row[kTextThreads * EDGES];
     __shared__ int s_max[kTextThreads / 32];
-    __shared__ int64_t s_first;
+    __shared__ int64_t s_span[2];  // the first and last edge's rows
     const int lane = lane_id(), wid = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < kTextThreads * EDGES; i += kTextThreads) s_row[i] = 0;
-    if (wid == 0) {
-        const int64_t f = warp_last_below(n, [&](int64_t r) { return fo[r] <= e0; });
-        if (lane == 0) s_first = f;
+    if (wid < 2) {
+        const int64_t e = wid == 0 ? e0 : e1 - 1;
+        const int64_t r = warp_last_below(n, [&](int64_t i) { return fo[i] <= e; });
+        if (lane == 0) s_span[wid] = r;
     }
     __syncthreads();
-    const int64_t first = s_first;
-    // rows after the first, until one starts past the tile
-    for (int64_t r0 = first + 1;; r0 += kTextThreads) {
-        const int64_t r = r0 + threadIdx.x;
-        const int64_t p = r < n ? fo[r] : e1;
-        if (p < e1) atomicMax(&s_row[p - e0], (int)(r - first));
-        if (__syncthreads_or(p >= e1)) break;
+    const int64_t first = s_span[0], rows = s_span[1] - first;
+    if (rows > kMarkRows) {
+#pragma unroll
+        for (int k = 0; k < EDGES; ++k) row[k] = first;
+        for (int64_t step = 1ll << (63 - __clzll(rows)); step; step >>= 1) {
+#pragma unroll
+            for (int k = 0; k < EDGES; ++k) {
+                const int64_t r = row[k] + step;
+                if (r - first <= rows && fo[r] <= e0 + threadIdx.x * EDGES + k) row[k] = r;
+            }
+        }
+        __syncthreads();  // the shared arrays are the next tile's
+        return;
     }
+    for (int r = 1 + (int)threadIdx.x; r <= (int)rows; r += kTextThreads) atomicMax(&s_row[fo[first + r] - e0], r);
+    __syncthreads();
     int mark[EDGES], run = 0;
 #pragma unroll
     for (int k = 0; k < EDGES; ++k) {

@@ -866,3 +866,49 @@ def test_captured_run_with_other_outputs_and_another_start(gpu):
                 runs.append(eng.edges(m0, k))
             np.testing.assert_array_equal(runs[0][0], runs[1][0])
             np.testing.assert_array_equal(runs[0][1], runs[1][1])
+
+
+@pytest.mark.parametrize("gaps", [[0], [1, 2, 255, 256, 257], [4094, 4095, 4096, 4097, 4098], [70_000, 3, 4096, 9000]])
+@pytest.mark.parametrize("m", [1, 7, 512, 1025, 4000])
+def test_sources_and_text_across_empty_rows(gpu, m, gaps):
+    """Edges whose rows lie apart by runs of empty rows around the length from which a tile searches instead of
+    marking, one or several edges a row: sources by ranges and text equal the CSR's."""
+    rng = np.random.default_rng(m + len(gaps))
+    row, src = 1 + gaps[0], []
+    while len(src) < m:
+        src += [row] * int(min(row, rng.integers(1, 4)))
+        row += 1 + int(rng.choice(gaps)) * int(rng.random() < 0.01 or len(src) < 4 or m < 20)
+    src = np.array(src[:m], np.int32)
+    start = np.searchsorted(src, src)
+    dst = (np.arange(m) - start).astype(np.int32)  # below the source: a row has at most as many edges
+    n = int(src[-1]) + 1 + max(gaps)
+    with GrowthEngine(seed=1) as eng:
+        eng.load_graph(np.zeros(n, np.int32), np.ones(n, np.float32), src, dst, PAParams(), planned_epochs=1)
+        assert eng.counts() == (n, m)
+        for first in sorted({0, m // 3, m - 1}):
+            s, d = eng.edges(first, m - first)
+            np.testing.assert_array_equal(s, src[first:])
+            np.testing.assert_array_equal(d, dst[first:])
+        ids = np.arange(n, dtype=np.int64) * 3 - 5
+        assert eng.format_edges(ids) == "".join(f"{ids[a]},{ids[b]}\n" for a, b in zip(src, dst)).encode()
+
+
+def test_empty_rows_cost_little(gpu):
+    """Copy-out of 600 edges spread over 2M rows against the same number side by side: they differ by a search of
+    21 steps (about 1.3 times), not by a walk over the rows (60 times)."""
+    import time
+    n, m, took = 2_000_000, 600, []
+    spread = np.linspace(1, n - 1, m).astype(np.int32)
+    for src in (n // 2 + np.arange(m, dtype=np.int32), spread):
+        with GrowthEngine(seed=1) as eng:
+            eng.load_graph(np.zeros(n, np.int32), np.ones(n, np.float32), src, np.zeros(m, np.int32), PAParams(),
+                           planned_epochs=1)
+            out = (np.empty(m, np.int32), np.empty(m, np.int32))
+            best = 1.0
+            for _ in range(20):
+                t = time.perf_counter()
+                eng.edges(0, m, out=out)
+                best = min(best, time.perf_counter() - t)
+            np.testing.assert_array_equal(out[0], src)
+            took.append(best)
+    assert took[1] < 6 * took[0], took
