@@ -55,6 +55,7 @@ struct LikState {
     int64_t n = 0, n0 = 0, agents = 0;
     int epochs = 0, num_anchors = 0, words = 0, chunks = 0, ball_grid = 0, eval_grid[2] = {0, 0};
     int wt_span = 1;           // epochs per weight table
+    int64_t wt_refused = 0;    // the smallest table (floats) there was no room for; 0: none was refused
     int64_t chunk_agents = 0;  // > 0: at most this many agents' balls per chunk (pg_tuning)
     DBuf<int64_t> epoch_nodes, fo, bo, coff, boff, bcnt, badj;
     DBuf<int32_t> epoch_t, fc, bc, pub, anchors, cites, agent_epoch, bids, order;
@@ -463,6 +464,7 @@ void free_lik(LikState& L) {
     dfree(L.feat);
     dfree(L.err);
     dfree(L.wt);
+    L.wt_refused = 0;
     L.hboff.clear();
     L.hnodes.clear();
     L.ball_chunks.clear();
@@ -2601,11 +2603,15 @@ int lik_table_epochs(pg_ctx* c, int BE) {
     if (BE > 32 ? L.ball_elems < 4 * rows : 8 * L.ball_elems < rows) return 0;
     const int64_t need = L.wt_span * std::max<int64_t>(L.hnodes[(size_t)L.epochs - 1], 1) * BE;
     if (L.wt.n < need) {
-        dfree(L.wt);
+        if (L.wt_refused > 0 && need >= L.wt_refused) return 0;  // asked before, for this trace
         size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || 4 * need > (int64_t)(free_b / 8) ||
-            dalloc(L.wt, need) != cudaSuccess) {
-            cudaGetLastError();  // no room: the direct walk
+        bool room = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess;
+        // the table that goes makes room; one that stays serves the smaller batches
+        room = room && 4 * need <= ((int64_t)free_b + 4 * L.wt.n) / 8;
+        if (room) room = dalloc(L.wt, need) == cudaSuccess;
+        if (!room) {
+            cudaGetLastError();  // the direct walk
+            L.wt_refused = need;
             return 0;
         }
     }

@@ -18,6 +18,7 @@ namespace pg {
 struct ErSkip;  // device code only
 }
 #include "../paragraph_gb300/csrc/pg_engine.cuh"
+#include "../paragraph_gb300/csrc/pg_lik.cuh"
 
 using pg::Arena;
 
@@ -32,6 +33,7 @@ size_t g_pool_used = 0, g_pool_reserved = 0;
 uint64_t g_pool_keep = 0;
 int64_t g_fail_in = -1;        // device allocations from now until one fails; < 0: none
 int64_t g_mallocs = 0, g_queries = 0;
+int64_t g_ball = 1;            // elements of every agent's ball
 int64_t g_faults = 0;          // kernels that would have read through a null pointer
 int g_sms = 152;
 std::map<uintptr_t, Block> g_blocks;
@@ -145,6 +147,10 @@ cudaError_t launch(const void* f, dim3 grid, dim3 block, void** args, int attrs)
         const Arena& A = *(Arena*)args[0];
         if (!A.rc_big_id || !A.rc_big_meta || !A.rc_part || !A.rc_item || !A.rc_item_list || !A.rc_item_meta || !A.rc_ticket)
             ++g_faults;
+    } else if (name.find("pg::k_lik_ball<false>(") != std::string::npos) {
+        const pg::LikBalls B = *(pg::LikBalls*)args[1];
+        const int64_t a0 = *(int64_t*)args[2], a1 = *(int64_t*)args[3];
+        for (int64_t a = a0; a < a1; ++a) B.cnt[a] = g_ball;
     } else if (is("k_copy_segments")) {
         const pg::CopySeg* s = *(pg::CopySeg**)args[0];
         const int num = *(int*)args[1];
@@ -168,6 +174,7 @@ void fake_reset(int64_t total_bytes, int32_t sms) {
     g_launches.clear();
 }
 void fake_fail_in(int64_t n) { g_fail_in = n; }
+void fake_ball(int64_t elements) { g_ball = elements; }
 int64_t fake_mallocs(void) { return g_mallocs; }
 int64_t fake_faults(void) { return g_faults; }
 int64_t fake_memory_queries(void) { return g_queries; }

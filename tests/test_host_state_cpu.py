@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import paragraph_gb300 as pg
-from paragraph_gb300 import PG_ERR_CAPACITY, PG_ERR_STATE, PG_WEIGHTS_REFCOMPAT, GrowthEngine, PAParams, PGError, RCParams
+from paragraph_gb300 import PG_ERR_CAPACITY, PG_ERR_STATE, PG_WEIGHTS_REFCOMPAT, GrowthEngine, PAParams, PGError, RCParams, TraceInput
 from paragraph_gb300.build import PKG, ROOT, build_library, nvcc
 
 
@@ -27,7 +27,7 @@ def fake(built, tmp_path_factory):
     lib = pg.load_library(d / "libfake.so")
     lib.fake_reset.argtypes = [C.c_int64, C.c_int32]
     lib.fake_fail_in.argtypes = [C.c_int64]
-    lib.fake_hold.argtypes = [C.c_int64]
+    lib.fake_hold.argtypes = lib.fake_ball.argtypes = [C.c_int64]
     for f in ("fake_mallocs", "fake_faults", "fake_memory_queries", "fake_free_bytes", "fake_hold"):
         getattr(lib, f).restype = C.c_int64
     lib.fake_launches.argtypes = [C.c_char_p]
@@ -195,3 +195,59 @@ def test_load_after_a_failed_load(host, weight_model):
                 eng.rc_configure(RCParams(growth_rate=0.04), np.full(10, 5), np.full(4, 0.25))
             assert eng.run_epochs(2) >= 40
     assert failed >= (8 if weight_model else 1) and host.fake_faults() == 0
+
+
+# ---------------------------------------------------------------- the likelihood's weight table
+def _trace(n, agents):
+    """`agents` papers of one epoch, each with one citation, after a seed of n."""
+    t = n + agents
+    return TraceInput(pub=np.zeros(t, np.int32), fitness=np.ones(t, np.float32), seed_src=np.zeros(0, np.int32),
+                      seed_dst=np.zeros(0, np.int32), epoch_nodes=np.array([n, t]), epoch_t=np.array([0]),
+                      anchors=np.tile(np.array([0, -1, -1, -1], np.int32), (agents, 1)),
+                      cite_off=np.arange(agents + 1), cites=np.zeros(agents, np.int32), num_anchors=1)
+
+
+def _points(b):
+    return np.tile([1.0, 5.0, 1.0, 4.0], (b, 1))
+
+
+def test_refused_weight_table_is_asked_for_once(host):
+    """The table of 64 points has no room (51 MB of 200 MB free, an eighth may be taken), that of 4 points has:
+    batches in turn neither free and allocate nor ask for the free memory again, and the small batches keep
+    their table."""
+    host.fake_ball(16_000)
+    with GrowthEngine(seed=1) as eng:
+        eng.load_trace(_trace(200_000, 100))
+        held = host.fake_free_bytes() - (200 << 20)
+        host.fake_hold(held)
+        for b in (4, 64):
+            eng.loglik(_points(b))
+            eng.loglik_grad(_points(b))
+        host.fake_clear_launches()
+        before = host.fake_mallocs(), host.fake_memory_queries()
+        for b in (64, 4, 64, 4):
+            eng.loglik(_points(b))
+            eng.loglik_grad(_points(b))
+        assert (host.fake_mallocs(), host.fake_memory_queries()) == before
+        assert host.fake_launches(b"k_lik_table1") == 4 and host.fake_launches(b"k_lik_eval") == 4
+        host.fake_hold(-held)
+        eng.load_trace(_trace(200_000, 100))  # another trace asks again
+        host.fake_clear_launches()
+        eng.loglik(_points(64))
+        assert host.fake_launches(b"k_lik_table2") == 1
+
+
+def test_larger_weight_table_counts_the_one_it_replaces(host):
+    host.fake_ball(16_000)
+    with GrowthEngine(seed=1) as eng:
+        eng.load_trace(_trace(200_000, 100))
+        eng.loglik(_points(32))  # 26 MB
+        eng.loglik(_points(64))  # the buffers of 64 points
+        eng.load_trace(_trace(200_000, 100))
+        eng.loglik(_points(32))
+        held = host.fake_free_bytes() - (400 << 20)
+        host.fake_hold(held)
+        host.fake_clear_launches()
+        eng.loglik(_points(64))  # 51 MB of 400 + 26
+        assert host.fake_launches(b"k_lik_table2") == 1
+        host.fake_hold(-held)
