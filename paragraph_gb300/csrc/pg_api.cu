@@ -195,18 +195,6 @@ pg_status fail(pg_ctx* c, pg_status s, const std::string& msg) {
     } while (0)
 
 template <typename T>
-cudaError_t dalloc(DBuf<T>& b, int64_t n) {
-    if (b.p && b.own) cudaFree(b.p);
-    b.p = nullptr;
-    b.n = 0;
-    b.own = true;
-    if (n <= 0) n = 1;
-    cudaError_t e = cudaMalloc((void**)&b.p, sizeof(T) * (size_t)n);
-    if (e == cudaSuccess) b.n = n;
-    return e;
-}
-
-template <typename T>
 void dfree(DBuf<T>& b) {
     if (b.p && b.own) cudaFree(b.p);
     b.p = nullptr;
@@ -216,8 +204,11 @@ void dfree(DBuf<T>& b) {
 // Temporaries of a load (raw edges, sort scratch, offset-form CSR) and of a text export come from a
 // stream-ordered pool owned by the library: allocating and freeing them does not synchronise the device,
 // and a later call reuses the memory instead of mapping it again.  The pool holds at most what the
-// largest call needed (about 40 bytes per raw edge of a load, 60 per edge of an export) and is
-// given back when the device's last context is destroyed.
+// largest load needed (about 40 bytes per raw edge); an export (60 bytes per edge) leaves it at kPoolKeep or at
+// what it held before.  What it holds idle counts as free memory where a decision depends on that
+// (device_room), is given up when an allocation finds no room (dalloc), and is all given back when the
+// device's last context is destroyed.
+constexpr size_t kPoolKeep = 256ull << 20;  // 4M edges' text; beyond, the copy to the host dwarfs the mapping
 struct TempPool {
     cudaMemPool_t pool = nullptr;
     int contexts = 0;
@@ -254,6 +245,76 @@ void pool_contexts(int device, int by) {
     TempPool& t = g_pools[device];
     t.contexts += by;
     if (t.contexts == 0 && t.pool) cudaMemPoolTrimTo(t.pool, 0);
+}
+
+// bytes the device's pool has reserved, and those of them in use
+void pool_bytes(int device, size_t& reserved, size_t& used) {
+    reserved = used = 0;
+    if (device < 0 || device >= 64) return;
+    const std::lock_guard<std::mutex> hold(g_pool_guard);
+    const cudaMemPool_t pool = g_pools[device].pool;
+    uint64_t r = 0, u = 0;
+    if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &r) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &u) == cudaSuccess) {
+        reserved = (size_t)r;
+        used = (size_t)u;
+    }
+}
+
+// the current device's pool gives up what it holds idle; false: nothing
+bool pool_give_up() {
+    int device = -1;
+    size_t reserved = 0, used = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    pool_bytes(device, reserved, used);
+    if (reserved <= used) return false;
+    const std::lock_guard<std::mutex> hold(g_pool_guard);
+    return cudaMemPoolTrimTo(g_pools[device].pool, 0) == cudaSuccess;
+}
+
+// free device memory, with what the pool holds idle
+cudaError_t device_room(int device, size_t& bytes) {
+    size_t total = 0, reserved = 0, used = 0;
+    const cudaError_t e = cudaMemGetInfo(&bytes, &total);
+    pool_bytes(device, reserved, used);
+    if (e == cudaSuccess && reserved > used) bytes += reserved - used;
+    return e;
+}
+
+// An export's use of the pool: declared before the export's temporaries, so that they are freed first.
+struct PoolExport {
+    int device;
+    cudaStream_t stream;
+    size_t before = 0;
+    PoolExport(int d, cudaStream_t s) : device(d), stream(s) {
+        size_t used = 0;
+        pool_bytes(device, before, used);
+    }
+    ~PoolExport() {
+        size_t reserved = 0, used = 0;
+        pool_bytes(device, reserved, used);
+        const size_t keep = std::max(before, kPoolKeep);
+        if (reserved <= keep) return;
+        cudaStreamSynchronize(stream);  // the frees have taken place
+        const std::lock_guard<std::mutex> hold(g_pool_guard);
+        cudaMemPoolTrimTo(g_pools[device].pool, keep);
+    }
+};
+
+template <typename T>
+cudaError_t dalloc(DBuf<T>& b, int64_t n) {
+    if (b.p && b.own) cudaFree(b.p);
+    b.p = nullptr;
+    b.n = 0;
+    b.own = true;
+    if (n <= 0) n = 1;
+    cudaError_t e = cudaMalloc((void**)&b.p, sizeof(T) * (size_t)n);
+    if (e == cudaErrorMemoryAllocation && pool_give_up()) {
+        cudaGetLastError();
+        e = cudaMalloc((void**)&b.p, sizeof(T) * (size_t)n);
+    }
+    if (e == cudaSuccess) b.n = n;
+    return e;
 }
 
 template <typename T>
@@ -2409,6 +2470,7 @@ pg_status pg_format_edges(pg_ctx* c, int32_t replica, const int64_t* ids, int64_
     if (n_ids != h.n) return fail(c, PG_ERR_ARG, "ids must hold one id per node");
     PG_CUDA(c, cudaSetDevice(c->device));
     const int64_t n = h.n, m = h.m;
+    const PoolExport pool(c->device, c->stream);
     struct Tmp {  // from the temporaries' pool: allocating and freeing were 1.9 ms of a 2.3 ms export
         pg_ctx* c;
         DBuf<int64_t> did, off, bs;
@@ -2462,6 +2524,7 @@ pg_status pg_format_attributes(pg_ctx* c, int32_t replica, const pg_attr_rows* r
     if (!rows->ids || !rows->draws || !rows->ints || (!rows->generators && rows->num_seed < n))
         return fail(c, PG_ERR_ARG, "ids, draws, ints and generators are required");
     PG_CUDA(c, cudaSetDevice(c->device));
+    const PoolExport pool(c->device, c->stream);
     struct Tmp {  // from the temporaries' pool: allocating and freeing were 1.9 ms of a 2.3 ms export
         pg_ctx* c;
         DBuf<int64_t> did, gen, off, bs;
@@ -2604,8 +2667,8 @@ int lik_table_epochs(pg_ctx* c, int BE) {
     const int64_t need = L.wt_span * std::max<int64_t>(L.hnodes[(size_t)L.epochs - 1], 1) * BE;
     if (L.wt.n < need) {
         if (L.wt_refused > 0 && need >= L.wt_refused) return 0;  // asked before, for this trace
-        size_t free_b = 0, total_b = 0;
-        bool room = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess;
+        size_t free_b = 0;
+        bool room = device_room(c->device, free_b) == cudaSuccess;
         // the table that goes makes room; one that stays serves the smaller batches
         room = room && 4 * need <= ((int64_t)free_b + 4 * L.wt.n) / 8;
         if (room) room = dalloc(L.wt, need) == cudaSuccess;
@@ -2879,8 +2942,8 @@ pg_status pg_trace_load(pg_ctx* c, const pg_trace_desc* t) {
     const int64_t pass_ids = (int64_t)L.words * 32;
     const int64_t bstride = (nmax + pass_ids - 1) / pass_ids * L.words;
     {
-        size_t free0 = 0, total0 = 0;
-        PG_CUDA(c, cudaMemGetInfo(&free0, &total0));
+        size_t free0 = 0;
+        PG_CUDA(c, device_room(c->device, free0));
         if ((double)std::max<int64_t>(agents, 1) * (double)bstride * 4.0 <= (double)free0 / 8.0 &&
             talloc(bmap, std::max<int64_t>(agents, 1) * bstride, c->device, c->stream) != cudaSuccess) {
             cudaGetLastError();  // no room after all: the emit pass walks the rows
@@ -2909,8 +2972,8 @@ pg_status pg_trace_load(pg_ctx* c, const pg_trace_desc* t) {
     L.ball_elems = L.hboff[(size_t)agents];
     L.citations = mc;
     if ((s = upload(c, L.boff, L.hboff.data(), agents + 1)) != PG_OK) return s;
-    size_t free_b = 0, total_b = 0;
-    PG_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
+    size_t free_b = 0;
+    PG_CUDA(c, device_room(c->device, free_b));
     const int64_t budget = std::max<int64_t>(biggest, (int64_t)(free_b / 4) / 4);  // ids in a quarter of free memory
     int64_t a = 0;
     while (a < agents) {

@@ -31,7 +31,7 @@ size_t g_total = 64ull << 30;  // device memory
 size_t g_used = 0;             // device allocations, and what the pool has reserved
 size_t g_pool_used = 0, g_pool_reserved = 0;
 uint64_t g_pool_keep = 0;
-int64_t g_fail_in = -1;        // device allocations from now until one fails; < 0: none
+int64_t g_fail_in = -1;        // device allocations from now until they fail; < 0: they do not
 int64_t g_mallocs = 0, g_queries = 0;
 int64_t g_ball = 1;            // elements of every agent's ball
 int64_t g_faults = 0;          // kernels that would have read through a null pointer
@@ -55,8 +55,8 @@ void submit(std::function<void()> f) {
 
 bool fails() {
     ++g_mallocs;
-    if (g_fail_in < 0) return false;
-    return g_fail_in-- == 0;
+    if (g_fail_in > 0) return g_fail_in--, false;
+    return g_fail_in == 0;
 }
 
 void* take(size_t bytes, int kind) {
@@ -179,6 +179,7 @@ int64_t fake_mallocs(void) { return g_mallocs; }
 int64_t fake_faults(void) { return g_faults; }
 int64_t fake_memory_queries(void) { return g_queries; }
 int64_t fake_free_bytes(void) { return (int64_t)(g_total - g_used); }
+int64_t fake_pool_idle(void) { return (int64_t)(g_pool_reserved - g_pool_used); }
 int64_t fake_hold(int64_t bytes) {  // memory of another user of the device; negative: given back
     g_used += bytes;
     return (int64_t)g_used;

@@ -28,7 +28,7 @@ def fake(built, tmp_path_factory):
     lib.fake_reset.argtypes = [C.c_int64, C.c_int32]
     lib.fake_fail_in.argtypes = [C.c_int64]
     lib.fake_hold.argtypes = lib.fake_ball.argtypes = [C.c_int64]
-    for f in ("fake_mallocs", "fake_faults", "fake_memory_queries", "fake_free_bytes", "fake_hold"):
+    for f in ("fake_mallocs", "fake_faults", "fake_pool_idle", "fake_memory_queries", "fake_free_bytes", "fake_hold"):
         getattr(lib, f).restype = C.c_int64
     lib.fake_launches.argtypes = [C.c_char_p]
     lib.fake_launches.restype = C.c_int32
@@ -250,4 +250,67 @@ def test_larger_weight_table_counts_the_one_it_replaces(host):
         host.fake_clear_launches()
         eng.loglik(_points(64))  # 51 MB of 400 + 26
         assert host.fake_launches(b"k_lik_table2") == 1
+        host.fake_hold(-held)
+
+
+# ---------------------------------------------------------------- temporaries kept between calls
+def _pool_idle(host, edges=3_000_000):
+    """A context whose load of `edges` citations of few papers has left the temporaries' pool that much idle."""
+    eng = GrowthEngine(seed=1)
+    eng.load_graph(np.zeros(1000, np.int32), np.ones(1000, np.float32), np.ones(edges, np.int32),
+                   np.zeros(edges, np.int32), PAParams(fixed_new_nodes=10, growth_rate=0.0), planned_epochs=1)
+    assert host.fake_pool_idle() > 40 * edges
+    return eng
+
+
+def test_an_export_gives_its_memory_back(host):
+    """Attribute rows of 6M papers take over 500 MB of temporaries, of which the load had left 144 MB reserved: at
+    most 256 MB are."""
+    n = 6_000_000
+    with _engine(n=n) as eng:
+        free, idle = host.fake_free_bytes(), host.fake_pool_idle()
+        rows = dict(ids=np.arange(n), draws=np.zeros((n, 4)), ints=np.zeros((n, 4), np.int32),
+                    generators=np.full((n, 4), -1, np.int64))
+        for _ in range(2):
+            assert _attributes(host, eng, rows) == pg.PG_OK
+            assert host.fake_free_bytes() >= free - ((256 << 20) - idle)
+
+
+def _attributes(host, eng, rows):
+    r = pg._AttrRows()
+    for k, v in rows.items():
+        setattr(r, k, v.ctypes.data)
+    r.num_nodes, r.num_seed = len(rows["ids"]), 0
+    size = C.c_int64()
+    return host.pg_format_attributes(eng._ctx, 0, C.byref(r), None, 0, C.byref(size))
+
+
+def test_idle_temporaries_count_as_free(host):
+    """51 MB of weight table, where an eighth of 350 MB free is too little and of 350 MB and the pool's idle
+    memory enough; and the allocation finds its room in the pool's."""
+    host.fake_ball(16_000)
+    with _pool_idle(host, 6_000_000), GrowthEngine(seed=1) as eng:
+        eng.load_trace(_trace(200_000, 100))
+        held = host.fake_free_bytes() - (350 << 20)
+        host.fake_hold(held)
+        host.fake_clear_launches()
+        eng.loglik(_points(64))
+        assert host.fake_launches(b"k_lik_table2") == 1
+        host.fake_hold(-held)
+
+
+def test_an_allocation_takes_back_idle_temporaries(host):
+    def load(eng, n=200_000):
+        eng.load_graph(np.zeros(n, np.int32), np.ones(n, np.float32), np.zeros(0, np.int32), np.zeros(0, np.int32),
+                       PAParams(fixed_new_nodes=10, growth_rate=0.0), planned_epochs=1)
+
+    with _pool_idle(host), GrowthEngine(seed=1) as eng:
+        with GrowthEngine(seed=1) as other:
+            free = host.fake_free_bytes()
+            load(other)
+            arena = free - host.fake_free_bytes()
+        held = host.fake_free_bytes() - (arena - (10 << 20))
+        host.fake_hold(held)
+        load(eng)
+        assert eng.counts() == (200_000, 0)
         host.fake_hold(-held)
