@@ -15,6 +15,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "pg_core.cuh"
 
 namespace pg {
@@ -500,13 +502,23 @@ __device__ __forceinline__ int advance_replica(const Replica* rep, int R, int r,
 // until the kernel before it (and so all before that) has finished and its writes are visible.  Without
 // the launch attribute the two instructions do nothing.  A kernel reached this way reads nothing through
 // the read-only path (__ldg, const __restrict__), whose loads could be moved ahead of the wait.
-// A launch of more than kDependentThreads threads, over half of what the SMs hold, goes without: it gains
+// A launch of more than 1,280 threads per SM, over half of what the SMs hold, goes without: it gains
 // little against its own length, and its waiting CTAs would keep the SMs from the side stream's kernels
 // (256 replicas x 10 epochs: 78.2 ms with the rule, 80.0 with every launch a dependent, 77.8 with none; ten
 // ER epochs of 10,000 nodes 2.80, 2.74 and 2.86 ms).  A checkpoint's restore and one epoch of 400 agents:
 // 214 us with none, 179 with the rule.
 #if defined(__CUDACC__)
-constexpr int64_t kDependentThreads = 152 * 1280;
+constexpr int64_t kDependentThreadsPerSm = 1280;
+// the current device's limit, its SMs counted once
+inline int64_t dependent_threads() {
+    static std::atomic<int> sms[64];
+    int d = -1;
+    if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= 64) return 0;
+    int n = sms[d].load(std::memory_order_relaxed);
+    if (n == 0 && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d) == cudaSuccess)
+        sms[d].store(n, std::memory_order_relaxed);
+    return n * kDependentThreadsPerSm;
+}
 __device__ __forceinline__ void pdl_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -522,7 +534,7 @@ inline void launch_dependent(void (*kernel)(P...), int64_t grid, int block, size
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = grid * block <= kDependentThreads ? 1 : 0;
+    cfg.numAttrs = grid * block <= dependent_threads() ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, (P)args...);
 }
 #endif

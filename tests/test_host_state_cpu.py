@@ -4,6 +4,7 @@ library keeps does to later calls.  The kernels do nothing but keep an epoch's c
 itself), so results of the sampling are not looked at here."""
 import ctypes as C
 import subprocess
+import sys
 from pathlib import Path
 
 import numpy as np
@@ -14,9 +15,8 @@ from paragraph_gb300 import PG_ERR_CAPACITY, PG_ERR_STATE, PG_WEIGHTS_REFCOMPAT,
 from paragraph_gb300.build import PKG, ROOT, build_library, nvcc
 
 
-@pytest.fixture(scope="module")
-def fake(built, tmp_path_factory):
-    d = tmp_path_factory.mktemp("fake")
+def build_fake(d):
+    """The library on the fake runtime, built in directory d."""
     cuda = Path(nvcc()).resolve().parents[1] / "include"
     if not list((PKG / "_build").glob("*.o")):
         build_library(force=True)
@@ -37,6 +37,11 @@ def fake(built, tmp_path_factory):
     lib.fake_page_locked.restype = C.c_void_p
     lib.fake_page_locked_free.argtypes = [C.c_void_p]
     return lib
+
+
+@pytest.fixture(scope="module")
+def fake(built, tmp_path_factory):
+    return build_fake(tmp_path_factory.mktemp("fake"))
 
 
 @pytest.fixture
@@ -314,3 +319,32 @@ def test_an_allocation_takes_back_idle_temporaries(host):
         load(eng)
         assert eng.counts() == (200_000, 0)
         host.fake_hold(-held)
+
+
+# ---------------------------------------------------------------- dependent launches
+@pytest.mark.parametrize("sms", [152, 76, 20])
+def test_dependent_launches_follow_the_device(built, tmp_path, sms):
+    """Launches of more than 1,280 threads per SM of the device are plain ones, whatever its number of SMs.  The
+    number is asked for once per process: a process each."""
+    code = f"""
+import sys, ctypes as C
+sys.path[:0] = [{str(ROOT)!r}, {str(ROOT / 'tests')!r}]
+import paragraph_gb300 as pg, test_host_state_cpu as t
+lib = pg._lib = t.build_fake(t.Path({str(tmp_path)!r}))
+lib.fake_reset(64 << 30, {sms})
+for new in (10, 300, 900, 1200, 4000, 7000):
+    with t._engine(new=new, epochs=1) as eng:
+        eng.run_epochs(1, use_graph=False)
+most, least = C.c_int64(), C.c_int64()
+for k in (b"k_agent_setup", b"k_bwd_place", b"k_agents<"):
+    lib.fake_dependent_range(k, C.byref(most), C.byref(least))
+    print(k.decode(), most.value, least.value)
+"""
+    out = subprocess.run([sys.executable, "-c", code], check=True, capture_output=True, text=True).stdout
+    limit = sms * 1280
+    seen = [tuple(map(int, line.split()[1:])) for line in out.splitlines()]
+    assert len(seen) == 3
+    assert all(0 < most <= limit for most, _ in seen), out
+    assert all(least == 0 or least > limit for _, least in seen), out
+    if sms < 152:
+        assert any(least for _, least in seen), out
