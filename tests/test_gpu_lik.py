@@ -272,3 +272,20 @@ def test_weights_at_the_ends_of_the_range(gpu, fitness, exact):
         eng.load_trace(tr)
         for b in (1, 8, 40):
             assert np.abs(eng.loglik(pts[:b]) + math.log(100.0)).max() <= 2e-5
+
+
+@pytest.mark.parametrize("points", [3, 20])
+def test_weight_table_in_parts_with_balls_in_chunks(gpu, points):
+    """Epoch groups of the weight table and chunks of balls that do not end at the same agents: the per-agent
+    arithmetic is that of balls kept for all agents, so the results are bitwise equal."""
+    g = W.plain_pa_seed(1_100_000, 10, seed=23)
+    prm = W.calibration_params()
+    prm.growth_rate, prm.fixed_new_nodes = 0.0, 2500
+    tr = W.grow_trace(g, prm, 4, seed=7)
+    pts = W.theta_batch(points, seed=9)
+    with GrowthEngine(seed=1) as a, GrowthEngine(seed=1) as b:
+        a.load_trace(tr)
+        b.set_tuning(lik_chunk_agents=1700)
+        b.load_trace(tr)
+        np.testing.assert_array_equal(a.loglik(pts), b.loglik(pts))
+        np.testing.assert_array_equal(a.loglik_grad(pts), b.loglik_grad(pts))

@@ -190,3 +190,32 @@ def test_refcompat_stream_splits_and_fallbacks_bit_exact(gpu, case):
             for k in ("rows_expanded", "elems_streamed", "draws"):
                 assert st[k] == so[k], k
         _compare(eng, og)
+
+
+def test_refcompat_more_long_streams_than_the_lists_hold(gpu):
+    """More papers with long 2-hop streams than the CTA-wide pass lists, and more parts of them than it has items
+    for: the papers past the list keep the one-warp path and streams past the items stay whole."""
+    n = 3000
+    base = W.rc_seed(n, 4, seed=21)
+    rng = np.random.default_rng(22)
+    hubs = rng.choice(n, 5, replace=False)
+    src = [base.src] + [rng.choice(n, 2600, replace=False).astype(np.int32) for _ in hubs]
+    dst = [base.dst] + [np.full(2600, h, np.int32) for h in hubs]
+    g = W.SeedGraph(base.pub, base.fitness, np.concatenate(src), np.concatenate(dst))
+    rec = 0.8 ** np.arange(40, dtype=np.float64)
+    rc = RCParams(growth_rate=5.8, same_year=0.1)
+    eng, og = _run_both(g, rc, np.array([2, 5, 9], np.int32), rec / rec.sum(), 1)
+    with eng:
+        deg, stream = _row_stats(og)
+        eng.grow_epoch()
+        og.rc_epoch()
+        gens = og.rc_agents()[:, 4].astype(np.int64)
+        long = (deg[gens] >= _BIG_GD) | (stream[gens] >= _BIG_STREAM)
+        parts = -(-stream[gens][long] // _engine_constant("kRcPart")) - 1
+        assert long.sum() > _engine_constant("kRcBigCap") and parts.sum() > _engine_constant("kRcParts")
+        np.testing.assert_array_equal(eng.arrivals(), og.arrivals())
+        np.testing.assert_array_equal(eng.rc_agents(), og.rc_agents())
+        st, so = eng.stats(), og.stats()
+        for k in ("rows_expanded", "elems_streamed", "draws"):
+            assert st[k] == so[k], k
+        _compare(eng, og)
