@@ -2655,10 +2655,15 @@ LikBalls make_balls(const LikState& L, int64_t a0) {
 }
 
 // Epochs per weight table (LikBatch::wt) of rows of BE points, with the table allocated; 0: no table.
-// At 64 points a row costs its 256-byte write, about what five ball elements save (3 epochs of 200k
-// nodes, forward and adjoint, direct against table: 700 us / 883 us at 0.9 ball elements per row,
-// 762 / 965 at 1.9; at 172 per row 46.3 / 15.4 ms).  Up to 32 points the table was faster wherever
-// measured (8 points: 350 / 263 us at 0.15 elements per row, 456 / 300 at 1.9).
+// Above 32 points a row costs its write of up to 256 bytes, which a large trace's table sends to DRAM.  Forward
+// and adjoint of 3 epochs of 200k nodes at 64 points, direct / table: 762 / 966 us at 0.3 ball elements per row,
+// 821 / 1,028 at 3.1, 996 / 1,027 at 4.2, 1,051 / 1,039 at 6.5, 1,242 / 1,082 at 9.2, 2,616 / 1,504 at 31; of 20k
+// and 50k nodes, whose tables stay in L2, the table is as fast at 0.1 per row and 1.1 to 1.2 times as fast from
+// 1 on.  Four per row is between the two.  (In the exact arithmetic a weight costs more and the table was 1.7
+// to 3.7 times as fast at every ratio; the line is the default arithmetic's.)  Up to 32 points the table was
+// faster wherever measured, 5,000 to 200k nodes, 0.05 to 31 elements per row, 8 to 32 points (at 32 points and
+// 200k nodes 806 / 610 us at 0.05, 1,074 / 804 at 0.2, 1,202 / 924 at 3.1): below an eighth the pass is the
+// epoch sums alone.
 int lik_table_epochs(pg_ctx* c, int BE) {
     LikState& L = c->lik;
     int64_t rows = 0;

@@ -41,8 +41,9 @@
 //                     sums: D_i = Z_a - sum_{l<i} W_{c_l}, log-likelihood sum x_i - log D_i, and in
 //                     the adjoint g_i - (dZ_a - dP_i) / D_i.  The adjoint rebuilds the table and
 //                     reads only the forward's per-agent Z_a.
-//   k_lik_eval        the same with every weight evaluated where it is summed, for traces whose balls
-//                     have fewer elements than the epochs have nodes, and where a table has no room.
+//   k_lik_eval        the same with every weight evaluated where it is summed, for traces with few ball
+//                     elements for their table rows (the line depends on the points: run_lik), and where
+//                     a table has no room.
 //   k_lik_sum         agents -> totals per point (fixed order).
 #include "pg_lik.cuh"
 #include "pg_sums.cuh"

@@ -92,8 +92,9 @@ struct LikBalls {
     // of walking the rows again (agent a's bitmap of pass i at bmap + a bmap_stride + i bitmap_words)
     uint32_t* bmap;
     int64_t bmap_stride;
-    // optional: each epoch's agents in descending ball size (by powers of two), the order the agent
-    // pass takes them in; null: as numbered
+    // optional: the agents in the order the agent pass takes them in, those of every group of epochs whose
+    // weight tables are held together by descending ball size (by powers of two).  It permutes the agents
+    // within such a group only, so a pass that uses it covers whole groups; null: as numbered
     const int32_t* order;
 };
 

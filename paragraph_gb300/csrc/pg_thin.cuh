@@ -150,9 +150,10 @@ __device__ __forceinline__ uint32_t hslot_of(int32_t v, int bits) {
 // random words) where the set's bucket takes 16 bytes (about 11); what passes it is looked up in the
 // set.  The agent kernel is bound by instruction issue and by the latency of its short chains at 16
 // warps per SM, and the scan is its largest part (1,535 of a warp's cycles per 512 entries with it).
-// PA at scale, 30 epochs: 37.7 ms of agent kernels without the filter, 33.1 with 256 words, 31.9 with
-// 1,024, and 31.7 with hits taken in any order; 256 replicas x 10 epochs: 67.1, 61.7, 60.1 and 56.5 ms.
-// 512 words and stage buffers of 768 entries instead of 1,024 and 512 took the run from 34.9 to 34.7 ms.
+// Agent kernels of PA at scale, 30 epochs: 37.7 ms without the filter, 33.1 with 256 words (what the general
+// instance and the 1,024-slot shape have), 31.9 with 1,024, 31.7 with hits taken in any order as well; of 256
+// replicas x 10 epochs 67.1, 61.7, 60.1 and 56.5 ms.  The lean instance has 512 words and spends the rest on
+// stage buffers of 768 entries instead of 512: the PA run 34.9 to 34.7 ms.
 template <int BITS>
 __device__ __forceinline__ bool filter_may_have(const uint32_t* F, uint32_t h) {
     const uint32_t w = F[h >> (32 - BITS)];
@@ -670,7 +671,7 @@ __device__ bool process_agent_thin(const Arena& A, int64_t a, int k, ThinSmem<KC
             for (int i0 = 0; i0 < nq; i0 += 32 * kTestU) {
                 // Bit u of `pass`: entry i0 + 32 u + lane may be in Z.  What is past the filter is rare and
                 // stays in a rolled loop: unrolled, its code no longer fits the instruction cache beside
-                // the rest (27 % slower at 8 entries per lane).  A row keeps its smallest hit, so the order
+                // the rest (39 % slower at 8 entries per lane).  A row keeps its smallest hit, so the order
                 // in which hits are taken does not matter.
                 unsigned pass = 0u;
 #pragma unroll
