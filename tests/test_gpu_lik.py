@@ -289,3 +289,20 @@ def test_weight_table_in_parts_with_balls_in_chunks(gpu, points):
         b.load_trace(tr)
         np.testing.assert_array_equal(a.loglik(pts), b.loglik(pts))
         np.testing.assert_array_equal(a.loglik_grad(pts), b.loglik_grad(pts))
+
+
+@pytest.mark.parametrize("exact", [False, True])
+def test_longest_list_drawn_above_half(gpu, exact):
+    """256 citations, all but the first from the half of Z that is left, beside others of a short list: the bound of
+    test_drawn_weight_above_half_in_64_bits, with logarithms below 15."""
+    nodes, cites = 300, 256
+    beta = 2.0 ** np.arange(10, 21)
+    pts = np.stack([np.ones(11), np.full(11, 5.0), np.ones(11), beta], axis=1)
+    pts = np.concatenate([pts] * 4)[:40]
+    with GrowthEngine(seed=1) as eng:
+        eng.set_lik_exact_exp2(exact)
+        eng.load_trace(_unit_weight_trace(nodes, cites))
+        ll = np.concatenate([eng.loglik(pts), eng.loglik(pts[:1])])
+    b = np.concatenate([pts[:, 3], pts[:1, 3]])
+    want = np.log(b) - np.log(nodes - 1 + b) - math.fsum(math.log(nodes - i) for i in range(1, cites))
+    assert np.abs(ll - want).max() <= cites * (8e-15 + 2.0**-53 * 15 * cites)
