@@ -204,11 +204,13 @@ void dfree(DBuf<T>& b) {
 // Temporaries of a load (raw edges, sort scratch, offset-form CSR) and of a text export come from a
 // stream-ordered pool owned by the library: allocating and freeing them does not synchronise the device,
 // and a later call reuses the memory instead of mapping it again.  The pool holds at most what the
-// largest load needed (about 40 bytes per raw edge); an export (60 bytes per edge) leaves it at kPoolKeep or at
-// what it held before.  What it holds idle counts as free memory where a decision depends on that
+// largest load needed (about 40 bytes per raw edge); an export (its text, and 8 or 104 bytes per node) leaves it at
+// kPoolKeep or at what it held before.  What it holds idle counts as free memory where a decision depends on that
 // (device_room), is given up when an allocation finds no room (dalloc), and is all given back when the
 // device's last context is destroyed.
-constexpr size_t kPoolKeep = 256ull << 20;  // 4M edges' text; beyond, the copy to the host dwarfs the mapping
+// 19M edges' text.  Beyond, a call maps the rest anew, little beside its copy to the host: 19.5M edges, 37.4 ms
+// against 37.1 with everything kept.
+constexpr size_t kPoolKeep = 256ull << 20;
 struct TempPool {
     cudaMemPool_t pool = nullptr;
     int contexts = 0;
